@@ -50,32 +50,120 @@ constexpr uint64_t kEmuHidden = 0x0010000000000000ull;
 __device__ __forceinline__ uint64_t emu_bits(double x) { return (uint64_t)__double_as_longlong(x); }
 __device__ __forceinline__ double emu_double(uint64_t b) { return __longlong_as_double((long long)b); }
 
-// RN(x y), on 32-bit words: the 106-bit product of the significands from
-// four 32 x 32 -> 64-bit products, its leading 53 bits taken by funnel shifts
-__device__ __forceinline__ double emu_mul(double x, double y) {
+// ---- words and carries. The device forms are PTX (a carry chain, a left
+// funnel shift, the approximate FP32 seeds); the host forms serve the
+// host-compiled check of the same arithmetic.
+__device__ __forceinline__ uint32_t emu_hi(double x) { return (uint32_t)(emu_bits(x) >> 32); }
+__device__ __forceinline__ uint32_t emu_lo(double x) { return (uint32_t)emu_bits(x); }
+
+// the high word of (hi:lo) << s, s in 0 .. 31
+__device__ __forceinline__ uint32_t emu_fsl(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, s);
+#else
+    return (uint32_t)(((((uint64_t)hi << 32) | lo) << (s & 31u)) >> 32);
+#endif
+}
+
+__device__ __forceinline__ float emu_rcp_seed(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.0f / x;
+#endif
+}
+
+__device__ __forceinline__ float emu_rsqrt_seed(float x) {
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return rsqrtf(x);
+#endif
+}
+
+// The double (hi:lo) rounded up when the bits below it, (r1:r0), exceed half
+// a unit, or equal it and lo is odd: the carry out of (r1 : r0 | odd) +
+// (2^63 - 1) is exactly that decision, and runs on into the exponent when the
+// significand overflows.
+__device__ __forceinline__ double emu_round_pack(uint32_t hi, uint32_t lo, uint32_t r1, uint32_t r0) {
+    r0 |= lo & 1u;
+#ifdef __CUDA_ARCH__
+    uint32_t ol, oh;
+    asm("{\n\t.reg .u32 t;\n\t"
+        "add.cc.u32 t, %2, 0xffffffff;\n\t"
+        "addc.cc.u32 t, %3, 0x7fffffff;\n\t"
+        "addc.cc.u32 %0, %4, 0;\n\t"
+        "addc.u32 %1, %5, 0;\n\t}"
+        : "=r"(ol), "=r"(oh)
+        : "r"(r0), "r"(r1), "r"(lo), "r"(hi));
+    return emu_double(((uint64_t)oh << 32) | ol);
+#else
+    const uint64_t r = ((uint64_t)r1 << 32) | r0;
+    return emu_double((((uint64_t)hi << 32) | lo) + (r > 0x8000000000000000ull ? 1ull : 0ull));
+#endif
+}
+
+// ---- the operations without their range checks: operands normal (not zero,
+// subnormal, infinite or NaN) and the result's exponent in the normal range,
+// both the caller's to ensure.
+
+// RN(x y): the 106-bit product of the significands from four 32 x 32 ->
+// 64-bit products, its leading 53 bits and the two words below them by funnel
+// shifts. 40 cycles per warp and sub-partition in a probe of independent
+// chains, against 75 for the hardware's DMUL and 61 for the form this
+// replaced (the round and sticky bits extracted and compared). Two variants
+// that moved the alignment and the normalisation to the multiply pipe
+// (multiplications by powers of two) took 53 to 55: the 64-bit addends they
+// zero-extend cost register moves.
+__device__ __forceinline__ double emu_mul_n(double x, double y) {
+    const uint32_t xh = emu_hi(x), a0 = emu_lo(x), yh = emu_hi(y), b0 = emu_lo(y);
+    const uint32_t a1 = (xh & 0xfffffu) | 0x100000u, b1 = (yh & 0xfffffu) | 0x100000u;
+    const uint64_t t0 = (uint64_t)a0 * b0;
+    const uint64_t m = (uint64_t)a0 * b1 + (uint64_t)a1 * b0 + (t0 >> 32);  // < 2^55
+    const uint64_t u = (uint64_t)a1 * b1 + (m >> 32);
+    const uint32_t w0 = (uint32_t)t0, w1 = (uint32_t)m, w2 = (uint32_t)u, w3 = (uint32_t)(u >> 32);
+    const uint32_t top = w3 >> 9, sh = 20u + top;  // product >= 2: the significand is its bits from 53 on, else from 52
+    // sign and exponent: the sum's carry out of the sign bits is their XOR;
+    // the hidden bit (and a rounding carry) add one
+    const uint32_t eh = (xh & 0xfff00000u) + (yh & 0xfff00000u) + ((top << 20) - (1024u << 20));
+    return emu_round_pack(__funnelshift_r(w2, w3, sh) + eh, __funnelshift_r(w1, w2, sh), __funnelshift_r(w0, w1, sh),
+                          __funnelshift_r(0u, w0, sh));
+}
+
+// Whether |x| lies in [2^-L, 2^L): one multiply-add and one compare, the sign
+// shifted out. False for zeros, infinities and NaNs.
+template <uint32_t L>
+__device__ __forceinline__ bool emu_within(double x) {
+    return emu_hi(x) * 2u - ((1023u - L) << 21) < (2u * L) << 21;
+}
+
+// RN(x + y) for x, y > 0 whose exponents differ by less than 32: the smaller
+// significand shifted right, its lost bits kept whole in one word below.
+__device__ __forceinline__ double emu_addp_n(double x, double y) {
     const uint64_t a = emu_bits(x), b = emu_bits(y);
-    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
-    const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-    const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
-    const uint64_t t0 = (uint64_t)al * bl, t1 = (uint64_t)mah * bl, t2 = (uint64_t)al * mbh;
-    const uint64_t t3 = (uint64_t)mah * mbh;  // < 2^42
-    const uint64_t mid = t1 + t2 + (t0 >> 32);  // < 2^55
-    const uint64_t upper = t3 + (mid >> 32);  // P = upper 2^64 + (uint32)mid 2^32 + (uint32)t0
-    const uint32_t w0 = (uint32_t)t0, w1 = (uint32_t)mid, w2 = (uint32_t)upper, w3 = (uint32_t)(upper >> 32);
-    const uint32_t top = (w3 >> 9) & 1u;  // P >= 2^105: the significand is P >> 53, else P >> 52
-    const uint32_t sh = 20u + top;
-    const uint32_t mlo = __funnelshift_r(w1, w2, sh), mhi = __funnelshift_r(w2, w3, sh);
-    const uint32_t rb = (w1 >> (sh - 1u)) & 1u;  // the round bit; below it the sticky bits
-    const uint32_t sticky = (w1 & ((1u << (sh - 1u)) - 1u)) | w0;
-    const uint32_t up = rb & ((sticky != 0u ? 1u : 0u) | (mlo & 1u));
-    const int e = (int)(ea + eb) - 1023 + (int)top;  // biased exponent before rounding
-    // (e - 1) << 20 plus the significand's hidden bit gives exponent field e;
-    // a rounding carry moves it to e + 1 (2047: the correctly rounded infinity)
-    const uint32_t rhi = ((ah ^ bh) & 0x80000000u) | (((uint32_t)(e - 1) << 20) + mhi);
-    uint64_t r = (((uint64_t)rhi << 32) | mlo) + up;
-    const bool ok = ea - 1u < 0x7feu && eb - 1u < 0x7feu && (uint32_t)(e - 1) < 2046u;
-    if (!ok) r = emu_bits(emu_native_mul(x, y));
-    return emu_double(r);
+    const uint64_t g = a > b ? a : b, l = a > b ? b : a;
+    const uint32_t gh = (uint32_t)(g >> 32), lh = (uint32_t)(l >> 32), l0 = (uint32_t)l;
+    const uint32_t d = (gh >> 20) - (lh >> 20);
+    const uint32_t l1 = (lh & 0xfffffu) | 0x100000u;
+    const uint64_t sh = ((uint64_t)(l1 >> d) << 32) | __funnelshift_r(l0, l1, d);
+    const uint32_t w1 = __funnelshift_r(0u, l0, d);
+    const uint64_t S = ((((uint64_t)((gh & 0xfffffu) | 0x100000u)) << 32) | (uint32_t)g) + sh;  // [2^52, 2^54)
+    const uint32_t Sh = (uint32_t)(S >> 32), Sl = (uint32_t)S;
+    const uint32_t s = Sh >> 21;
+    const uint32_t eh = (gh & 0xfff00000u) - 0x100000u + (s << 20);
+    return emu_round_pack((Sh >> s) + eh, __funnelshift_r(Sl, Sh, s), __funnelshift_r(w1, Sl, s), w1 & s);
+}
+
+// RN(x y): the unchecked product, or the hardware's when an operand lies
+// outside [2^-500, 2^500) (zeros, subnormals, infinities and NaNs included)
+__device__ __forceinline__ double emu_mul(double x, double y) {
+    double r = emu_mul_n(x, y);
+    if (!(emu_within<500>(x) && emu_within<500>(y))) r = emu_native_mul(x, y);
+    return r;
 }
 
 // RN(1 - x) for x in [1/2, 1], where the difference is exact (Sterbenz):
@@ -164,139 +252,115 @@ __device__ __forceinline__ double emu_addsub(double x, double y) {
     return emu_double(r);
 }
 
-// S^2 for S < 2^54 as two 64-bit words
-__device__ __forceinline__ void emu_sq_wide(uint64_t S, uint64_t &hi, uint64_t &lo) {
-    const uint32_t sh = (uint32_t)(S >> 32), sl = (uint32_t)S;
-    const uint64_t ll = (uint64_t)sl * sl, mid = ((uint64_t)sl * sh) << 1, hh = (uint64_t)sh * sh;
-    lo = ll + (mid << 32);
-    hi = hh + (mid >> 32) + (lo < ll ? 1ull : 0ull);
+// RN(sqrt(x)), x > 0 normal. V = the significand times 2^62 (times 2 for an
+// odd exponent), in [2^62, 2^64). S0 = 24 bits of sqrt from the FP32
+// reciprocal square root y0; two Newton corrections S += (V - S^2) y0 / 2
+// bring the error to 2^-44 and 2^-66 relative, each residual exact in 64-bit
+// modular arithmetic (it is far smaller than its operands) and read as a
+// 32-bit window; so S2 = sqrt(V) 2^31 to within one unit of its 63 bits. The
+// ten bits below the result's last decide the rounding unless they lie within
+// that error of one half (1 in 256); then the exact sign of x - (midpoint)^2
+// does (a square root is never a midpoint itself). Newton's iteration with a
+// final exact remainder test, e.g. R. Brent and P. Zimmermann, "Modern
+// Computer Arithmetic", 2010, section 1.5.1. 70 cycles in the probe (174 for
+// the form before, which tested every result; 85 for this one testing always).
+__device__ __forceinline__ double emu_sqrt_n(double x) {
+    const uint32_t xh = emu_hi(x), xl = emu_lo(x);
+    const uint32_t even = (xh >> 20) & 1u;  // biased exponent odd: the unbiased one is even
+    const uint32_t a1 = emu_fsl(xl, xh, 11) | 0x80000000u, a0 = xl << 11;
+    const uint32_t v1 = a1 >> even, v0 = __funnelshift_r(a0, a1, even);
+    const float uf = __uint2float_rn(v1) * 0x1p-30f;  // V 2^-62 in [1, 4]
+    const float y0 = emu_rsqrt_seed(uf);
+    const uint32_t s0 = __float2uint_rn(uf * y0 * 0x1p23f);  // sqrt 2^23
+    const uint64_t V = ((uint64_t)v1 << 32) | v0;
+    // |V - s0^2 2^16| < 2^43
+    const int64_t r0 = (int64_t)(V - (((uint64_t)s0 * s0) << 16));
+    const int32_t c1 = __float2int_rn((float)(int32_t)(r0 >> 14) * y0 * 0x1p-3f);  // r0 y0 / 2 in units of 2^-46: * 2^-62 2^46 / 2
+    const uint64_t S1 = ((uint64_t)s0 << 23) + (uint64_t)(int64_t)c1;  // sqrt 2^46
+    const int64_t r1 = (int64_t)((V << 30) - S1 * S1);  // units of 2^-92, |r1| < 2^52
+    const int32_t c2 = __float2int_rn((float)(int32_t)(r1 >> 22) * y0 * 0x1p-9f);  // r1 y0 / 2 in units of 2^-62
+    const uint64_t S2 = (S1 << 16) + (uint64_t)(int64_t)c2;  // sqrt 2^62, within one unit
+    uint64_t R = (S2 + 512ull) >> 10;  // [2^52, 2^53]
+    if ((((uint32_t)S2 + 514u) & 1023u) < 4u) {
+        R = (S2 + 510ull) >> 10;  // the candidate below the midpoint m / 2
+        const uint64_t m = 2ull * R + 1ull;
+        // sign of V 2^44 - m^2 (units of 2^-106), from the low 64 bits: |.| < 2^62
+        if ((int64_t)((V << 44) - m * m) > 0) R += 1ull;
+    }
+    // exponent field of the result: (e - 1023 - odd) / 2 + 1023
+    const uint32_t er = ((xh >> 20) + 1023u - (even ^ 1u)) >> 1;
+    return emu_double(((uint64_t)(er - 1u) << 52) + R);
 }
 
-// RN(sqrt(x)). With x = M0 2^p (M0 the significand, shifted left once when
-// p is odd) the result's significand is RN(sqrt(M)) for the integer
-// M = M0 2^52 in [2^104, 2^106): S0 from the FP32 reciprocal square root
-// y0 ~ 1/sqrt(M0 2^-52) (about 21 good bits), two Newton corrections
-// S += (M - S^2) y0 / (2 sqrt(M)) evaluated on 32-bit windows of the exact
-// 128-bit residual (the error falls from ~2^32 to ~2^12 to below 0.51), then
-// the exact remainder r = M - S^2 makes S the floor (0 <= r <= 2S) and
-// decides the rounding: up iff r > S (sqrt(M) > S + 1/2; never a tie for an
-// integer M). The method is Newton's iteration for the square root with an
-// exact integer remainder test, e.g. R. Brent and P. Zimmermann, "Modern
-// Computer Arithmetic", 2010, section 1.5.1.
+// RN(sqrt(x)), any x
 __device__ __forceinline__ double emu_sqrt(double x) {
-    const uint64_t a = emu_bits(x);
-    const uint32_t ah = (uint32_t)(a >> 32);
-    const uint32_t e = ah >> 20;  // with the sign bit: > 2046 for negative x
-    const uint32_t odd = ~e & 1u;  // the unbiased exponent e - 1075 is odd
-    const uint64_t M0 = ((a & kEmuFrac) | kEmuHidden) << odd;  // [2^52, 2^54)
-    const uint64_t Mhi = M0 >> 12, Mlo = M0 << 52;  // M = M0 2^52
-    const float uf = __uint2float_rn((uint32_t)(M0 >> 30)) * 0x1p-22f;  // M0 2^-52 in [1, 4), 24 bits
-    const float y0 = rsqrtf(uf);
-    uint64_t S = (uint64_t)__float2uint_rn(uf * y0 * 0x1p23f) << 29;  // ~ sqrt(M)
-    uint64_t hi, lo;
-    // first correction: |M - S^2| < 2^86, read as bits 56 .. 87
-    emu_sq_wide(S, hi, lo);
-    {
-        const uint64_t rlo = Mlo - lo, rhi = Mhi - hi - (Mlo < lo ? 1ull : 0ull);
-        const int32_t w = (int32_t)__funnelshift_r((uint32_t)(rlo >> 32), (uint32_t)rhi, 24);
-        // S += r y0 / 2^53 = w y0 2^3, rounded in units of 2^8
-        S += (uint64_t)((int64_t)__float2int_rn((float)w * y0 * 0x1p-5f) * 256);
-    }
-    // second correction: |M - S^2| < 2^66, read as bits 36 .. 67
-    emu_sq_wide(S, hi, lo);
-    {
-        const uint64_t rlo = Mlo - lo, rhi = Mhi - hi - (Mlo < lo ? 1ull : 0ull);
-        const int32_t w = (int32_t)__funnelshift_r((uint32_t)(rlo >> 32), (uint32_t)rhi, 4);
-        S += (uint64_t)(int64_t)__float2int_rn((float)w * y0 * 0x1p-17f);
-    }
-    // the exact remainder (|r| < 2^56: the low word suffices), floor, rounding
-    int64_t r = (int64_t)(Mlo - S * S);
-    if (r < 0) {
-        S -= 1ull;
-        r += (int64_t)(2ull * S + 1ull);
-    }
-    if (r > (int64_t)(2ull * S)) {
-        r -= (int64_t)(2ull * S + 1ull);
-        S += 1ull;
-    }
-    const uint64_t Sr = S + (r > (int64_t)S ? 1ull : 0ull);  // [2^52, 2^53]
-    const int32_t er = ((int32_t)e - 1023 - (int32_t)odd) / 2 + 1023;  // exponent field of the result
-    uint64_t res = ((uint64_t)(uint32_t)(er - 1) << 52) + Sr;
-    const bool ok = e - 1u < 0x7feu;  // positive and normal
-    if (!ok) res = emu_bits(emu_native_sqrt(x));
-    return emu_double(res);
+    const uint32_t e = emu_hi(x) >> 20;  // with the sign bit: > 2046 for negative x
+    double r = emu_sqrt_n(x);
+    if (!(e - 1u < 0x7feu)) r = emu_native_sqrt(x);
+    return r;
 }
 
 // A divisor b prepared for several quotients: its significand mb and
-// inv ~ 2^115 / mb to within a few units (FP32 seed, two Newton corrections
-// inv += inv (2^115 - mb inv) / 2^115 on 32-bit windows of the exact
-// residual; the relative error falls from ~2^-21 to ~2^-42 to ~2^-61).
+// inv = 2^115 / mb to within one unit (inv in [2^62, 2^63]). FP32 seed v0 (24
+// bits), two Newton corrections v += v (1 - b v) to 2^-44 and 2^-66 relative;
+// each residual is small against 2^64, so its low 64 bits are all of it.
 struct EmuDivisor {
     uint64_t mb, inv;
     uint32_t bh;  // high word of b: sign and exponent
 };
 
 __device__ __forceinline__ EmuDivisor emu_divisor(double b) {
-    const uint64_t bb = emu_bits(b);
     EmuDivisor D;
-    D.bh = (uint32_t)(bb >> 32);
-    D.mb = (bb & kEmuFrac) | kEmuHidden;
-    const float rf = __frcp_rn(__uint2float_rn((uint32_t)(D.mb >> 29)));  // ~ 2^29 / mb
-    uint64_t inv = (uint64_t)__float2uint_rn(rf * 0x1p46f) << 40;  // ~ 2^115 / mb
-    uint64_t hi = __umul64hi(D.mb, inv), lo = D.mb * inv;
-    {
-        // E = 2^115 - mb inv, |E| < 2^95: bits 64 .. 95; inv += inv E / 2^115
-        // = w rf 2^35, rounded in units of 2^16
-        const int32_t w = (int32_t)((1ull << 51) - hi - (lo != 0ull ? 1ull : 0ull));
-        inv += (uint64_t)((int64_t)__float2int_rn((float)w * rf * 0x1p19f) * 65536);
-    }
-    hi = __umul64hi(D.mb, inv);
-    lo = D.mb * inv;
-    {
-        // |E| < 2^75: bits 44 .. 75; inv += w rf 2^15
-        const uint64_t elo = 0ull - lo, ehi = (1ull << 51) - hi - (lo != 0ull ? 1ull : 0ull);
-        const int32_t w = (int32_t)__funnelshift_r((uint32_t)(elo >> 32), (uint32_t)ehi, 12);
-        inv += (uint64_t)(int64_t)__float2int_rn((float)w * rf * 0x1p15f);
-    }
-    D.inv = inv;
+    const uint32_t bl = emu_lo(b);
+    D.bh = emu_hi(b);
+    const uint32_t b1 = (D.bh & 0xfffffu) | 0x100000u;
+    D.mb = ((uint64_t)b1 << 32) | bl;
+    const float bf = __uint_as_float((emu_fsl(bl, D.bh, 3) & 0x7fffffu) | 0x3f800000u);  // [1, 2), truncated
+    const float rf = emu_rcp_seed(bf);
+    const uint32_t v0 = __float2uint_rn(rf * 0x1p24f);  // 2^76 / mb, 2^23 .. 2^24
+    // 2^76 - mb v0, |.| < 2^55
+    const int64_t e0 = (int64_t)(0ull - ((uint64_t)bl * v0 + ((uint64_t)(b1 * v0) << 32)));
+    const int32_t c1 = __float2int_rn((float)(int32_t)(e0 >> 25) * rf * 0x1p-4f);  // e0 v0 / 2^76 in units of 2^-23
+    const uint64_t v1 = ((uint64_t)v0 << 23) + (uint64_t)(int64_t)c1;  // 2^99 / mb
+    // 2^99 - mb v1, |.| < 2^57
+    const int64_t e1 = (int64_t)(0ull - D.mb * v1);
+    const int32_t c2 = __float2int_rn((float)(int32_t)(e1 >> 27) * rf * 0x1p-9f);
+    D.inv = (v1 << 16) + (uint64_t)(int64_t)c2;  // 2^115 / mb
     return D;
 }
 
-// RN(x / y) with D = emu_divisor(y). The significand quotient
-// Q = floor(ma 2^(52+s) / mb) (s = 1 when ma < mb, so Q is in [2^52, 2^53))
-// comes from ma inv to within one unit; the exact remainder
-// R = ma 2^(52+s) - Q mb makes Q the floor (0 <= R < mb) and rounds: up iff
-// 2R > mb (a quotient of two 53-bit significands is never a midpoint).
-// Long division by a scaled reciprocal with remainder correction, e.g.
-// R. Brent and P. Zimmermann, "Modern Computer Arithmetic", 2010, 1.4.1.
+// RN(x / y) with D = emu_divisor(y). X = ma inv is ma / mb 2^115 to within
+// 2^53 (inv's unit times ma), so its leading 53 bits Q (a quotient >= 1: bits
+// 63 on, else bits 62 on) are the quotient's floor, or one beside it when the
+// quotient lies within 2^-9 units of a whole number; in every case the exact
+// sign of x - (Q + 1/2) y, from the low 64 bits of ma 2^k - (2Q + 1) mb, says
+// whether Q or Q + 1 is nearest (a quotient of two 53-bit significands is
+// never a midpoint). Division by a scaled reciprocal with an exact remainder
+// test, e.g. R. Brent and P. Zimmermann, "Modern Computer Arithmetic", 2010,
+// 1.4.1. The test is taken always: rounding on the bits below Q and testing
+// only the ambiguous ones took 80 cycles in a probe, this form 55.
+__device__ __forceinline__ double emu_div_n(double x, const EmuDivisor &D) {
+    const uint32_t xh = emu_hi(x), a0 = emu_lo(x);
+    const uint32_t a1 = (xh & 0xfffffu) | 0x100000u;
+    const uint32_t i1 = (uint32_t)(D.inv >> 32), i0 = (uint32_t)D.inv;
+    const uint64_t m = (uint64_t)a0 * i1 + (uint64_t)a1 * i0 + (((uint64_t)a0 * i0) >> 32);  // < 2^64
+    const uint64_t u = (uint64_t)a1 * i1 + (m >> 32);  // X >> 64, [2^50, 2^52)
+    const uint32_t w1 = (uint32_t)m, w2 = (uint32_t)u, w3 = (uint32_t)(u >> 32);
+    const uint32_t big = w3 >> 19, s = 2u - big;
+    uint64_t Q = ((uint64_t)emu_fsl(w2, w3, s) << 32) | emu_fsl(w1, w2, s);
+    // ma 2^(54 - big): its low word is zero
+    const int64_t rem = (int64_t)(((uint64_t)(a0 << (22u - big)) << 32) - (2ull * Q + 1ull) * D.mb);
+    Q += rem > 0 ? 1ull : 0ull;
+    const uint32_t eh = (xh & 0xfff00000u) - (D.bh & 0xfff00000u) + ((1021u + big) << 20);
+    return emu_double(((uint64_t)eh << 32) + Q);
+}
+
+// RN(x / y): the unchecked quotient, or the hardware's when an operand lies
+// outside [2^-500, 2^500)
 __device__ __forceinline__ double emu_div(double x, const EmuDivisor &D, double y) {
-    const uint64_t a = emu_bits(x);
-    const uint32_t ah = (uint32_t)(a >> 32);
-    const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (D.bh >> 20) & 0x7ffu;
-    const uint64_t ma = (a & kEmuFrac) | kEmuHidden;
-    const uint32_t s = ma < D.mb ? 1u : 0u;
-    uint64_t Q = __umul64hi(ma << 11, D.inv) >> (10u - s);
-    int64_t R = (int64_t)((ma << (52u + s)) - Q * D.mb);
-    if (R < 0) {
-        Q -= 1ull;
-        R += (int64_t)D.mb;
-    }
-    if (R >= (int64_t)D.mb) {
-        Q += 1ull;
-        R -= (int64_t)D.mb;
-    }
-    const uint64_t up = (uint64_t)(2 * R) > D.mb ? 1ull : 0ull;
-    const int e = (int)ea - (int)eb + 1023 - (int)s;  // biased exponent before rounding
-    const uint64_t sign = (uint64_t)((ah ^ D.bh) & 0x80000000u) << 32;
-    uint64_t r = sign | ((((uint64_t)(e - 1)) << 52) + Q + up);
-    const bool bn = eb - 1u < 0x7feu;
-    bool ok = bn && ea - 1u < 0x7feu && (uint32_t)(e - 1) < 2046u;
-    if (bn && (a & ~kEmuSign) == 0ull) {  // +-0 / b
-        r = sign;
-        ok = true;
-    }
-    if (!ok) r = emu_bits(emu_native_div(x, y));
-    return emu_double(r);
+    double r = emu_div_n(x, D);
+    if (!(emu_within<500>(x) && emu_within<500>(y))) r = emu_native_div(x, y);
+    return r;
 }
 
 __device__ __forceinline__ double emu_add(double x, double y) { return emu_addsub<false>(x, y); }
