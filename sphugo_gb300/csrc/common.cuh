@@ -116,6 +116,12 @@ struct Ctx {
 // slot range, so a static per-slot index answers with one load.
 __device__ __forceinline__ int sim_of(const Ctx &c, int64_t i) { return c.simidx ? __ldg(c.simidx + i) : 0; }
 
+__device__ __forceinline__ uint32_t lanemask_lt() {
+    uint32_t m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+
 __device__ __forceinline__ uint32_t part1by1(uint32_t x) {
     x &= 0x0000ffffu;
     x = (x | (x << 8)) & 0x00ff00ffu;
@@ -225,6 +231,7 @@ void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &
 // tiles computed the settled queries' densities, only the deferred are done
 void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int mode,
                     const KnnTune *tune);
+void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D);
 void force_init_attrs(int k);
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
                   const Derived &D, int mode, bool integrate);

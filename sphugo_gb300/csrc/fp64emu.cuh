@@ -56,6 +56,9 @@ __device__ __forceinline__ double emu_double(uint64_t b) { return __longlong_as_
 __device__ __forceinline__ uint32_t emu_hi(double x) { return (uint32_t)(emu_bits(x) >> 32); }
 __device__ __forceinline__ uint32_t emu_lo(double x) { return (uint32_t)emu_bits(x); }
 
+// -x (the compiler negates a double with an FP64 instruction)
+__device__ __forceinline__ double emu_neg(double x) { return emu_double(emu_bits(x) ^ kEmuSign); }
+
 // the high word of (hi:lo) << s, s in 0 .. 31
 __device__ __forceinline__ uint32_t emu_fsl(uint32_t lo, uint32_t hi, uint32_t s) {
 #ifdef __CUDA_ARCH__
@@ -166,17 +169,37 @@ __device__ __forceinline__ double emu_mul(double x, double y) {
     return r;
 }
 
-// RN(1 - x) for x in [1/2, 1], where the difference is exact (Sterbenz):
-// 1 - x = (2^53 - m) 2^-53 for the significand m of x in [1/2, 1), shifted to
-// put its leading bit at bit 52. Other x take the hardware subtraction.
+// u as a float, truncated
+__device__ __forceinline__ float emu_u2f_rz(uint32_t u) {
+#ifdef __CUDA_ARCH__
+    return __uint2float_rz(u);
+#else
+    const int lz = u ? __builtin_clz(u) : 0;
+    return (float)(lz < 8 ? u & ~((1u << (8 - lz)) - 1u) : u);
+#endif
+}
+
+// 1 - x for x in [1/2, 1), where the difference is exact (Sterbenz):
+// 1 - x = t 2^-53 with t = 2^53 - m for the significand m of x, shifted to put
+// its leading bit at bit 52. The leading bit comes from the exponent of t's
+// top 32 bits as a float (a conversion issues four times as often as a count
+// of leading zeros: 20 cycles in the probe against 57); x closer to 1 than
+// 2^-32 takes the hardware subtraction.
+__device__ __forceinline__ double emu_one_minus_n(double x) {
+    const uint64_t t = (1ull << 53) - ((emu_bits(x) & kEmuFrac) | kEmuHidden);  // (0, 2^52]
+    const uint32_t tl = (uint32_t)t, th = (uint32_t)(t >> 32);
+    const uint32_t top = emu_fsl(tl, th, 11);  // t >> 21
+    const uint32_t lz = 158u - (__float_as_uint(emu_u2f_rz(top)) >> 23);  // 0 .. 31
+    double r = emu_double(((uint64_t)(emu_fsl(tl, th, lz) + ((1021u - lz) << 20)) << 32) | (tl << (lz & 31u)));
+    if (top == 0u) r = emu_native_sub(1.0, x);
+    return r;
+}
+
+// RN(1 - x): the unchecked difference, or the hardware's for x outside [1/2, 1)
 __device__ __forceinline__ double emu_one_minus(double x) {
-    const uint64_t a = emu_bits(x);
-    const uint64_t t = (1ull << 53) - ((a & kEmuFrac) | kEmuHidden);  // in (0, 2^52]
-    const int lz = __clzll((long long)t) - 11;  // 0 .. 52
-    uint64_t r = (((uint64_t)(1021 - lz)) << 52) + (t << lz);
-    if (a == 0x3FF0000000000000ull) r = 0ull;  // 1 - 1 = +0
-    else if ((a >> 52) != 1022ull) r = emu_bits(emu_native_sub(1.0, x));
-    return emu_double(r);
+    double r = emu_one_minus_n(x);
+    if (emu_hi(x) >> 20 != 1022u) r = emu_native_sub(1.0, x);
+    return r;
 }
 
 // The float pair of v: hi = RN_float(v) and lo = RN_float(v - hi) (v - hi is

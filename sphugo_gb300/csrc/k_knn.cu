@@ -955,57 +955,7 @@ __global__ void __launch_bounds__(256, 4) k_density(KnnArgs a) {
         const double gamma = S.gamma;
         const double up = B.up[q];
         double h, rho, cs, cterm;
-        if (MODE == MODE_EXACT64) {
-            // sim/nearest-neighbour.go:64-66 square roots, sim/sph.go:306-323 sum farthest first
-            double2 *dist = a.D.dist + q * k;
-            const double2 P = B.pos[q];
-            const int32_t *nb = a.D.nbr + q * k;
-            const double dk2 = nbr_d2(S, B, P, (uint32_t)nb[k - 1]);
-            if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
-            h = emu_sqrt(dk2);
-            const EmuDivisor dh = emu_divisor(h);  // shared by the k quotients d/h
-            // NNDists and q = NNDists/h; q grows with e (the list is sorted), so
-            // the entries with q < 0.5 are a prefix of length s
-            int s_lo = 0;
-            for_each_nbr_desc(nb, k, [&](int e, uint32_t code) {
-                const double d = e == k - 1 ? h : emu_sqrt(nbr_d2(S, B, P, code));
-                // RN(d / h); in [0, 1] because d <= h
-                const double x = emu_div(d, dh, h);
-                s_lo += __double_as_longlong(x) < __double_as_longlong(0.5);  // x < 0.5 (x >= 0)
-                dist[e] = make_double2(d, x);
-            });
-            // kernel sums farthest first (sim/sph.go:311-316), each branch of the
-            // Monahan kernel in its own loop (no divergent branch per term); the
-            // force's dF(q) replaces q in the list
-            double acc = 0.0;
-            if (S.kernel == SPH_KERNEL_WENDLAND) {
-                for (int e = k - 1; e >= 0; e--) {
-                    const double x = dist[e].y;
-                    acc = __dadd_rn(acc, kf_exact(SPH_KERNEL_WENDLAND, x));
-                    dist[e].y = kdf_exact(SPH_KERNEL_WENDLAND, x);
-                }
-            } else {
-                for (int e = k - 1; e >= s_lo; e--) {  // q >= 0.5
-                    const double x = dist[e].y;
-                    const double a1 = emu_one_minus(x);  // x in [1/2, 1]: exact
-                    const double a2 = emu_mul(a1, a1);
-                    acc = __dadd_rn(acc, div3_rn(emu_mul(a2, a1)));
-                    dist[e].y = -a2;
-                }
-                for (int e = s_lo - 1; e >= 0; e--) {  // q < 0.5
-                    const double x = dist[e].y;
-                    const double qq = emu_mul(x, x);
-                    acc = __dadd_rn(acc, __dadd_rn(__dsub_rn(emu_mul(qq, x), qq), 1.0 / 6.0));
-                    dist[e].y = __dsub_rn(emu_mul(emu_mul(3.0, x), x), emu_mul(2.0, x));
-                }
-            }
-            const double hh = __dmul_rn(h, h);
-            rho = emu_div(__dmul_rn(__dmul_rn(S.fpref, S.mass), acc), emu_divisor(hh), hh);
-            if (!(rho >= 0.0 && rho < 1.0e308)) fl |= FLAG_Q_RANGE;  // a NaN or infinite distance
-            cs = emu_sqrt(__dmul_rn(__dmul_rn(gamma, __dsub_rn(gamma, 1.0)), up));
-            const double grho = __dmul_rn(gamma, rho);
-            cterm = emu_div(__dmul_rn(cs, cs), emu_divisor(grho), grho);
-        } else if (MODE == MODE_FAST64) {
+        if (MODE == MODE_FAST64) {
             double2 *dist = a.D.dist + q * k;
             const double2 P = B.pos[q];
             const int32_t *nb = a.D.nbr + q * k;
@@ -1264,7 +1214,7 @@ void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Deriv
     a.B = B;
     a.D = D;
     a.use_defer = tune && D.defer && knn_fuses_density(c.k, mode, *tune) ? 1 : 0;
-    if (mode == MODE_EXACT64) run_density<MODE_EXACT64>(a, L);
+    if (mode == MODE_EXACT64) launch_density_fp64(c, L, B, D);
     else if (mode == MODE_FAST64) run_density<MODE_FAST64>(a, L);
     else run_density<MODE_MIXED>(a, L);
 }

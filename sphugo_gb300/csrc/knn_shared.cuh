@@ -25,12 +25,6 @@ constexpr float kEpsRel = 9.5367431640625e-7f;  // 2^-20 (about 8x the bound)
 
 __device__ __forceinline__ float eps_of(float d2, float abs_term) { return kEpsRel * d2 + abs_term; }
 
-__device__ __forceinline__ uint32_t lanemask_lt() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 // Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their
 // applications", 1968) of NS keys in registers, ascending: the network for the
 // next power of two with every comparator that touches a position >= NS left
@@ -98,19 +92,6 @@ __device__ __forceinline__ void rerank_lanes(const KnnArgs &a, bool mine, int64_
     if (lane == 0) base = atomicAdd(a.D.ndefer + 1, __popc(bal));
     base = __shfl_sync(0xffffffffu, base, 0);
     if (mine) a.D.defer[a.c.n - 1 - (base + __popc(bal & lanemask_lt()))] = (int32_t)q;
-}
-
-// the reference's squared distance to the neighbour image a list code names
-__device__ __forceinline__ double nbr_d2(const SimDev &S, const PArrays &B, double2 P, uint32_t code) {
-    const double2 Q = B.pos[code >> kCodeShift];
-    if ((code & 15u) == 4u) {
-        // no offset: p + 0 = p (and -0 + 0 = +0 squares to the same value)
-        const double dx = __dsub_rn(P.x, Q.x), dy = __dsub_rn(P.y, Q.y);
-        return __dadd_rn(emu_mul(dx, dx), emu_mul(dy, dy));
-    }
-    double ox, oy;
-    img_shift(S, code & 15u, ox, oy);
-    return dist_sq_ref(P.x, P.y, ox, oy, Q.x, Q.y);
 }
 
 // block-tile search (k_knn_block.cu): false when no block kernel serves the

@@ -190,4 +190,17 @@ __device__ __forceinline__ void img_shift(const SimDev &S, uint32_t img, double 
     oy = ib ? (ib > 0 ? S.dimg[1] : -S.dimg[1]) : 0.0;
 }
 
+// the reference's squared distance to the neighbour image a list code names
+__device__ __forceinline__ double nbr_d2(const SimDev &S, const PArrays &B, double2 P, uint32_t code) {
+    const double2 Q = B.pos[code >> kCodeShift];
+    if ((code & 15u) == 4u) {
+        // no offset: p + 0 = p (and -0 + 0 = +0 squares to the same value)
+        const double dx = __dsub_rn(P.x, Q.x), dy = __dsub_rn(P.y, Q.y);
+        return __dadd_rn(emu_mul(dx, dx), emu_mul(dy, dy));
+    }
+    double ox, oy;
+    img_shift(S, code & 15u, ox, oy);
+    return dist_sq_ref(P.x, P.y, ox, oy, Q.x, Q.y);
+}
+
 }  // namespace sphgpu
