@@ -255,7 +255,8 @@ SimDev make_simdev(const sph_params &p, int64_t off, int64_t n, int64_t cell_off
     S.dth = p.dth;
     S.accel[0] = p.accel[0];
     S.accel[1] = p.accel[1];
-    for (int i = 0; i < 4; i++) S.refl[i] = p.refl[i];
+    // a NaN bound reflects nothing, as an infinite one (the force compares bounds as integers)
+    for (int i = 0; i < 4; i++) S.refl[i] = std::isnan(p.refl[i]) ? (i & 1 ? HUGE_VAL : -HUGE_VAL) : p.refl[i];
     S.alpha = p.alpha;
     S.beta = p.beta;
     S.etasq = p.etasq;
@@ -297,11 +298,12 @@ void enqueue_eval(sph_handle *h, int pred, bool integrate, bool events = false) 
     mark(2);
     launch_permute(c, L, h->A, h->B, h->T, pred, true);  // velocity records: every form's force reads them
     mark(3);
-    launch_knn(c, L, h->B, h->D, h->T, h->mode, h->tune);
+    const int mode = kernel_mode(h->mode);
+    launch_knn(c, L, h->B, h->D, h->T, mode, h->tune);
     mark(4);
-    launch_density(c, L, h->B, h->D, h->mode, &h->tune);
+    launch_density(c, L, h->B, h->D, mode, &h->tune);
     mark(5);
-    launch_force(c, L, h->B, h->A, h->D, h->mode, integrate);
+    launch_force(c, L, h->B, h->A, h->D, mode, integrate);
     mark(6);
 }
 
@@ -448,14 +450,14 @@ int create_impl(const sph_params *params, const int64_t *counts, int32_t nsims, 
             return bail(fail(SPH_ERR_CUDA, "device initialisation failed"));
     }
     knn_init_attrs();
-    force_init_attrs((int)k);
+    force_init_attrs();
     h->tune.block = 256;
     h->tune.cap = (int)(k + 16);
     h->tune.theta = 0.5f;
     h->tune.hgrow = 1.04f;
-    h->tune.blocks_per_sm = std::max(1, knn_occupancy_blocks(h->tune.block, h->tune.cap, h->mode));
+    h->tune.blocks_per_sm = std::max(1, knn_occupancy_blocks(h->tune.block, h->tune.cap, kernel_mode(h->mode)));
     h->tune.tile = 1;
-    h->tune.tile_blocks_per_sm = std::max(1, knn_tile_occupancy_blocks((int)k, h->mode));
+    h->tune.tile_blocks_per_sm = std::max(1, knn_tile_occupancy_blocks((int)k, kernel_mode(h->mode)));
     h->tune.block_warps = default_block_warps((int)k);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return bail(fail(SPH_ERR_CUDA, cudaGetErrorString(e)));

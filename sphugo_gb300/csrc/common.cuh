@@ -24,8 +24,16 @@ constexpr int kCodeShift = 5;          // bit 4 is a scratch flag inside the kNN
 constexpr uint32_t kCodeFlag = 16u;
 constexpr int64_t kMaxParticles = (int64_t)1 << 27;
 
-// internal precision modes (SPH_PREC_* of the ABI map onto these)
+// precision modes of a handle (SPH_PREC_* of the ABI map onto these)
 enum Mode { MODE_EXACT64 = 0, MODE_FAST64 = 1, MODE_MIXED = 2 };
+
+// The kernels of a mode: the fast form runs the exact form's. Its own
+// kernels (contracted FP64 with per-particle reciprocals) did all their work
+// on the FP64 unit, of which GB300 has two lanes per SM, and took 1.28x the
+// time of the exact ones, which share theirs with the integer pipes (uniform
+// blast N = 1,048,576, k = 32: 3.92 against 3.07 ms a step, and 2.15 with
+// the exact form's present kernels).
+constexpr int kernel_mode(int mode) { return mode == MODE_FAST64 ? MODE_EXACT64 : mode; }
 
 // integration mode of a force evaluation
 enum Pred { PRED_DRIFT = 0, PRED_INIT = 1, PRED_KEEP = 2 };
@@ -84,8 +92,8 @@ struct Derived {
     double4 *der;   // FP64 modes: (c, rho, h, c^2/(gamma rho))
     float4 *derf;   // mixed:      (c, rho, h, c^2/(gamma rho))
     int32_t *nbr;   // n*k neighbour codes, slot 0 = nearest
-    double2 *dist;  // FP64 modes: n*k squared distance from the search, then
-                    // (NNDists, NNDists/h) [bit-exact form] or (NNDists, 1/NNDists) [fast form]
+    double2 *dist;  // FP64 modes, from the density pass: n*k
+                    // (NNDists, dF(NNDists/h))
     float *d2f;     // mixed: n*k FP32 squared distances
     int32_t *defer;  // queries the group-tile search leaves to the per-query search (n)
     int32_t *ndefer; // their count; ndefer[1]: queries to re-rank, stored from the end of defer
@@ -232,7 +240,7 @@ void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &
 void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int mode,
                     const KnnTune *tune);
 void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D);
-void force_init_attrs(int k);
+void force_init_attrs();
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
                   const Derived &D, int mode, bool integrate);
 void launch_error_norms(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, double *anorm,

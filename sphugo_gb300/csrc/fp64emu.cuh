@@ -144,6 +144,8 @@ __device__ __forceinline__ bool emu_within(double x) {
     return emu_hi(x) * 2u - ((1023u - L) << 21) < (2u * L) << 21;
 }
 
+__device__ __forceinline__ bool emu_is_zero(double x) { return ((emu_hi(x) * 2u) | emu_lo(x)) == 0u; }
+
 // RN(x + y) for x, y > 0 whose exponents differ by less than 32: the smaller
 // significand shifted right, its lost bits kept whole in one word below.
 __device__ __forceinline__ double emu_addp_n(double x, double y) {
@@ -388,16 +390,5 @@ __device__ __forceinline__ double emu_div(double x, const EmuDivisor &D, double 
 
 __device__ __forceinline__ double emu_add(double x, double y) { return emu_addsub<false>(x, y); }
 __device__ __forceinline__ double emu_sub(double x, double y) { return emu_addsub<true>(x, y); }
-
-// Out-of-line copies, one body per translation unit, for kernels whose loops
-// would outgrow the instruction cache with every operation inlined (the FP64
-// force kernel: inlined, ncu counted 4.5 cycles of "no instruction" stall per
-// issued instruction; out of line, the kernel ran 1.3x faster). Kernels with
-// short loops (the density) keep the inlined forms.
-static __device__ __noinline__ double emu_mul_ol(double x, double y) { return emu_mul(x, y); }
-static __device__ __noinline__ double emu_sqrt_ol(double x) { return emu_sqrt(x); }
-static __device__ __noinline__ EmuDivisor emu_divisor_ol(double b) { return emu_divisor(b); }
-// (the divisor by value: by reference it went through the stack, 5 % of the force's time)
-static __device__ __noinline__ double emu_div_ol(double x, EmuDivisor D, double y) { return emu_div(x, D, y); }
 
 }  // namespace sphgpu

@@ -1,14 +1,21 @@
 // k_force.cu -- pressure + artificial-viscosity acceleration and du/dt
 // (sim/sph.go:327-401 AccelerationAndEDot2D) fused with the rest of the
 // leapfrog step (sim/sph.go:121-193: kick, drift, periodic wrap,
-// reflections). One thread per particle walks its k neighbours from the
-// farthest to the nearest, as the reference's loop does, gathering the
-// neighbours' predicted velocity, sound speed, density and smoothing length.
-#include "physics.cuh"
+// reflections). The mixed form: one thread per particle walks its k
+// neighbours from the farthest to the nearest. The FP64 form: the pairs dealt
+// over the lanes, their terms added in that order.
+#include "pair_tile.cuh"
 
 #include <algorithm>
 
 namespace sphgpu {
+
+// Resident blocks of the FP64 force per SM (96 registers, 38 KB): 1160 us at
+// N = 1,048,576; 4 blocks 1198, 6 (80 registers) slower still.
+constexpr int kForceBlocks = 5;
+// Tiles up to this width sum with three lanes per particle: 31 us at N = 10,000
+// against 40 with one.
+constexpr int kSplitWidth = 10;
 
 struct ForceArgs {
     Ctx c;
@@ -18,26 +25,40 @@ struct ForceArgs {
     int integrate;
 };
 
-// sim/sph.go:121-193 with two roundings per multiply-add.
+// x < y for x, y not NaN, on the integer pipes (an FP64 compare costs the FP64
+// unit as much as an addition): the order of the bits read as integers, the
+// negative ones mirrored (-0 onto 0).
+__device__ __forceinline__ int64_t order_key(double x) {
+    const int64_t b = (int64_t)emu_bits(x);
+    return b < 0 ? (int64_t)(kEmuSign - (uint64_t)b) : b;
+}
+__device__ __forceinline__ bool less(double x, double y) { return order_key(x) < order_key(y); }
+__device__ __forceinline__ bool is_nan(double x) { return (emu_bits(x) & ~kEmuSign) > 0x7ff0000000000000ull; }
+__device__ __forceinline__ bool is_finite(double x) { return (emu_hi(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+// sim/sph.go:121-193 with two roundings per multiply-add: five additions on
+// the FP64 unit, the products and compares on the integer pipes (the bounds
+// are never NaN; a NaN position compares false)
 __device__ __forceinline__ void integrate_one(const SimDev &S, double2 &pos, double2 &vel, double &u,
                                               double ax, double ay, double udot) {
     const double dth = S.dth;
-    const double dt2 = __dmul_rn(2.0, dth);
-    vel.x = __dadd_rn(vel.x, __dmul_rn(ax, dt2));
-    vel.y = __dadd_rn(vel.y, __dmul_rn(ay, dt2));
-    u = __dadd_rn(u, __dmul_rn(__dmul_rn(udot, 2.0), dth));
-    pos.x = __dadd_rn(pos.x, __dmul_rn(vel.x, dth));
-    pos.y = __dadd_rn(pos.y, __dmul_rn(vel.y, dth));
+    const double dt2 = emu_mul(2.0, dth);  // exact, as is 2 udot: (2 udot) dth = udot (2 dth)
+    vel.x = __dadd_rn(vel.x, emu_mul(ax, dt2));
+    vel.y = __dadd_rn(vel.y, emu_mul(ay, dt2));
+    u = __dadd_rn(u, emu_mul(udot, dt2));
+    pos.x = __dadd_rn(pos.x, emu_mul(vel.x, dth));
+    pos.y = __dadd_rn(pos.y, emu_mul(vel.y, dth));
+    const bool fx = !is_nan(pos.x), fy = !is_nan(pos.y);
     // periodic wrap: an if/continue chain, at most one axis per step
-    if (pos.x < S.per_lo[0]) pos.x = __dadd_rn(pos.x, __dsub_rn(S.per_hi[0], S.per_lo[0]));
-    else if (pos.x > S.per_hi[0]) pos.x = __dsub_rn(pos.x, __dsub_rn(S.per_hi[0], S.per_lo[0]));
-    else if (pos.y < S.per_lo[1]) pos.y = __dadd_rn(pos.y, __dsub_rn(S.per_hi[1], S.per_lo[1]));
-    else if (pos.y > S.per_hi[1]) pos.y = __dsub_rn(pos.y, __dsub_rn(S.per_hi[1], S.per_lo[1]));
+    if (fx && less(pos.x, S.per_lo[0])) pos.x = __dadd_rn(pos.x, __dsub_rn(S.per_hi[0], S.per_lo[0]));
+    else if (fx && less(S.per_hi[0], pos.x)) pos.x = __dsub_rn(pos.x, __dsub_rn(S.per_hi[0], S.per_lo[0]));
+    else if (fy && less(pos.y, S.per_lo[1])) pos.y = __dadd_rn(pos.y, __dsub_rn(S.per_hi[1], S.per_lo[1]));
+    else if (fy && less(S.per_hi[1], pos.y)) pos.y = __dsub_rn(pos.y, __dsub_rn(S.per_hi[1], S.per_lo[1]));
     // reflections: Pos -= Pos - bound; Vel = -Vel
-    if (pos.x < S.refl[0]) { pos.x = __dsub_rn(pos.x, __dsub_rn(pos.x, S.refl[0])); vel.x = -vel.x; }
-    if (pos.x > S.refl[1]) { pos.x = __dsub_rn(pos.x, __dsub_rn(pos.x, S.refl[1])); vel.x = -vel.x; }
-    if (pos.y < S.refl[2]) { pos.y = __dsub_rn(pos.y, __dsub_rn(pos.y, S.refl[2])); vel.y = -vel.y; }
-    if (pos.y > S.refl[3]) { pos.y = __dsub_rn(pos.y, __dsub_rn(pos.y, S.refl[3])); vel.y = -vel.y; }
+    if (fx && less(pos.x, S.refl[0])) { pos.x = __dsub_rn(pos.x, __dsub_rn(pos.x, S.refl[0])); vel.x = emu_neg(vel.x); }
+    if (fx && less(S.refl[1], pos.x)) { pos.x = __dsub_rn(pos.x, __dsub_rn(pos.x, S.refl[1])); vel.x = emu_neg(vel.x); }
+    if (fy && less(pos.y, S.refl[2])) { pos.y = __dsub_rn(pos.y, __dsub_rn(pos.y, S.refl[2])); vel.y = emu_neg(vel.y); }
+    if (fy && less(S.refl[3], pos.y)) { pos.y = __dsub_rn(pos.y, __dsub_rn(pos.y, S.refl[3])); vel.y = emu_neg(vel.y); }
 }
 
 // The mixed form (the FP64 forms run k_force_fp64 below).
@@ -99,7 +120,7 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
             ayo = (double)(ay.value_f() * ff) + S.accel[1];
             edot = (double)(caf * ed.value_f() * S.fmass);
         }
-        if (!isfinite(axo) || !isfinite(ayo) || !isfinite(edot)) fl |= FLAG_Q_RANGE;
+        if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
         double2 pos = P, vel = B.vel[q];
         double u = B.u[q];
         if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
@@ -115,33 +136,6 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
     }
     if (fl) atomicOr(a.c.flags, fl);
 }
-
-// ---------------------------------------------------------------- FP64 form,
-// viscosity compacted. One warp per 32 consecutive particles, one lane per
-// particle, in three phases:
-//   1. each lane flags its approaching neighbour pairs (v_AB . r_AB < 0);
-//   2. the warp computes the viscosity term Pi of every flagged pair of its
-//      32 particles with all lanes busy (the pairs dealt out in turn) and
-//      keeps them in shared memory;
-//   3. each lane sums its k terms farthest first (sim/sph.go:343-392), taking
-//      Pi from shared memory for the flagged pairs.
-// Phase 3 is the reference's loop with Pi looked up instead of computed in a
-// branch that a warp runs whenever any of its lanes needs it; every operation
-// and its order are unchanged, so the results stay bit-exact.
-constexpr int kForceWarps = 4;
-
-// per-warp shared memory: Pi doubles of one chunk (at most 32 entries per
-// particle), masks, counts; rounded up to 16 bytes so that every warp's Pi
-// array starts 8-byte (in fact 16-byte) aligned
-__host__ __device__ constexpr size_t force_exact_warp_bytes(int k) {
-    return ((size_t)(k < 32 ? k : 32) * 256 + 4 * 32 * 4 + 33 * 4 + 15) & ~(size_t)15;
-}
-constexpr bool force_exact_layout_aligned() {
-    for (int k = 1; k <= 128; k++)
-        if (force_exact_warp_bytes(k) % 16 != 0 || ((size_t)k * 256) % 8 != 0) return false;
-    return true;
-}
-static_assert(force_exact_layout_aligned(), "per-warp shared-memory regions must stay 16-byte aligned");
 
 // r_AB = (q - offset) - p and v_AB . r_AB for neighbour code `code` of a
 // particle at P with predicted velocity vpi (sim/sph.go:355-367)
@@ -160,199 +154,254 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
         rabx = __dsub_rn(__dsub_rn(Q.x, ox), P.x);
         raby = __dsub_rn(__dsub_rn(Q.y, oy), P.y);
     }
-    dot = __dadd_rn(emu_mul_ol(vabx, rabx), emu_mul_ol(vaby, raby));
+    dot = __dadd_rn(__dmul_rn(vabx, rabx), __dmul_rn(vaby, raby));
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kForceWarps * 32) k_force_fp64(ForceArgs a) {
-    static_assert(MODE == MODE_EXACT64 || MODE == MODE_FAST64, "FP64 forms only");
+// ---------------------------------------------------------------- FP64 form.
+// A warp takes a tile of W particles (pair_tile.cuh) and, chunk by chunk of
+// their lists, farthest first:
+//   A. a lane per (particle, entry) pair computes r_AB and v_AB . r_AB, and
+//      lists the approaching pairs (v_AB . r_AB < 0) and the others;
+//   B. in the listed order, the approaching ones' viscosity terms Pi with all
+//      lanes at work (in list order a warp would run them whenever one of its
+//      lanes needs them: two divisions, and about half of the pairs), and
+//      every pair's terms;
+//   C. the ordered sums (sim/sph.go:343-392, farthest first), a lane per
+//      particle, or, for tiles of few particles, per particle and component.
+// Sums and differences run on the FP64 unit (75 cycles a warp instruction),
+// products and quotients on the integer pipes, unchecked behind range tests
+// (fp64emu.cuh); pairs that fail one (zero components, values outside 2^+-150,
+// infinities and NaNs) take the hardware's arithmetic out of line. Every
+// operation and its order are the reference's, so the results stay bit-exact.
+//
+// Bound (ncu, uniform blast N = 1,048,576, k = 32): FP64 pipe 67 %, ALU 52 %,
+// issue 60 % busy; moving work either way between the two pipes (the sums
+// cA + cB, hA + hB, rhoA + rhoB on the integer pipe, the dot product or r^2 on
+// the FP64 unit) changed nothing or cost up to 5 %. The loads are issued a
+// round early: 1335 -> 1231 us; one loop for both kinds of pairs instead of
+// one each: 1231 -> 1160.
+//
+// Against one warp per 32 particles, a lane each, with the approaching pairs
+// compacted per warp (force stage, us): N = 1000 112 -> 16, 10,000 154 -> 31,
+// 100,000 297 -> 148, 1,048,576 1750 -> 1160, clustered 4,194,304
+// 6800 -> 4520, stress 2,000,003 (k = 64) 6370 -> 4210.
+struct ForceRow {
+    double x, y, vx, vy;      // position and predicted velocity
+    double c, rho, h, cterm;  // sound speed, density, smoothing length, c^2 / (gamma rho)
+};
+
+struct ForceWarp {
+    double x[kPairSlots], y[kPairSlots];  // r_AB, then the acceleration terms
+    double e[kPairSlots];                 // v_AB . r_AB, then the du/dt terms
+    ForceRow row[32];
+    uint16_t list[kPairSlots];            // approaching pairs from the front, the others from the back
+};
+
+struct Vec2D {
+    double x, y;
+};
+
+// v_AB . r_AB with hardware arithmetic
+__device__ __noinline__ double force_dot_slow(double rx, double ry, double vx, double vy) {
+    return __dadd_rn(__dmul_rn(vx, rx), __dmul_rn(vy, ry));
+}
+
+// Pi (sim/sph.go:370-390) with hardware arithmetic, from the sums cA + cB, ...
+__device__ __noinline__ double force_pi_slow(double rx, double ry, double dot, double c2, double rho2, double h2,
+                                             double alpha, double beta, double etasq) {
+    const double cab = __dmul_rn(0.5, c2), rhoab = __dmul_rn(0.5, rho2), hab = __dmul_rn(0.5, h2);
+    const double r2 = __dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry));
+    const double mu = __ddiv_rn(__dmul_rn(dot, hab), __dadd_rn(r2, etasq));
+    return __ddiv_rn(__dadd_rn(__dmul_rn(__dmul_rn(-alpha, cab), mu), __dmul_rn(__dmul_rn(beta, mu), mu)), rhoab);
+}
+
+struct ForceTerms {
+    double x, y, e;
+};
+
+// a pair's terms with hardware arithmetic
+__device__ __noinline__ ForceTerms force_terms_slow(double rx, double ry, double dot, double sum3, double drk, double d) {
+    return ForceTerms{__ddiv_rn(__dmul_rn(__dmul_rn(rx, sum3), drk), d), __ddiv_rn(__dmul_rn(__dmul_rn(ry, sum3), drk), d),
+                      __dmul_rn(dot, drk)};
+}
+
+__device__ __forceinline__ double emu_halve(double x) { return emu_double(emu_bits(x) - (1ull << 52)); }
+
+__global__ void __launch_bounds__(kPairWarps * 32, kForceBlocks) k_force_fp64(ForceArgs a, int W) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int k = a.c.k;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nw = (k + 31) >> 5;  // mask words per particle (k <= 128)
-    // per warp: Pi[min(k, 32)][32] doubles, approach masks [4][32], inclusive pair counts [33]
-    unsigned char *wb = smem_raw + (size_t)w * force_exact_warp_bytes(k);
-    double *spi = (double *)wb;
-    uint32_t *smask = (uint32_t *)(wb + (size_t)(k < 32 ? k : 32) * 256);
-    int32_t *sinc = (int32_t *)(smask + 4 * 32);
+    ForceWarp &sm = reinterpret_cast<ForceWarp *>(smem_raw)[w];
     const PArrays &B = a.B;
     const Derived &D = a.D;
+    const PairChunks ch(k, W);
     unsigned fl = 0;
-    const int64_t n = a.c.n;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kForceWarps + w) * 32; q0 < n;
-         q0 += (int64_t)gridDim.x * kForceWarps * 32) {
-        const int64_t q = q0 + lane;
-        const bool valid = q < n;
-        const SimDev &S = a.c.sims[valid ? sim_of(a.c, q) : 0];
-        double2 P = make_double2(0.0, 0.0), vpi = P;
-        double4 di = make_double4(0.0, 0.0, 0.0, 0.0);
-        const int32_t *nb = D.nbr + q * k;
-        // ---- 1. approaching pairs: the sign of v_AB . r_AB from the float-pair
-        // records, with an error bound; the reference's FP64 dot product only
-        // where the bound cannot decide (e.g. equal velocities)
-        if (valid) {
-            P = B.pos[q];
-            vpi = B.vp[q];
-            di = D.der[q];
-            const float4 pr = B.rec[q], vi = B.vrec[q];
-            const float dXh = S.fimg_h[0], dXl = S.fimg_l[0], dYh = S.fimg_h[1], dYl = S.fimg_l[1];
-            const float lbig = 2.f * fmaxf(S.flmax, S.fmag);
-            uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;  // approach bits of entries 0-31, 32-63, ...
-            for_each_nbr_desc(nb, k, [&](int e, uint32_t code) {
-                {
-                    const uint32_t j = code >> kCodeShift;
-                    const int ia = (int)((code & 15u) / 3u) - 1, ib = (int)((code & 15u) % 3u) - 1;
-                    const float4 r = B.rec[j], vj = B.vrec[j];
-                    const float rx = ((r.x - (ia > 0 ? dXh : 0.f)) - (ia < 0 ? pr.x - dXh : pr.x)) +
-                                     (r.z - (pr.z + (ia > 0 ? dXl : ia < 0 ? -dXl : 0.f)));
-                    const float ry = ((r.y - (ib > 0 ? dYh : 0.f)) - (ib < 0 ? pr.y - dYh : pr.y)) +
-                                     (r.w - (pr.w + (ib > 0 ? dYl : ib < 0 ? -dYl : 0.f)));
-                    const float vx = (vj.x - vi.x) + (vj.z - vi.z), vy = (vj.y - vi.y) + (vj.w - vi.w);
-                    const float px = vx * rx, py = vy * ry;
-                    const float dotf = px + py;
-                    // |dotf - reference dot| bound: float-pair residues (2^-48 relative
-                    // to |p|, |v|), FP32 differences, products and sum (2^-23 each)
-                    const float vmag = fabsf(vj.x) + fabsf(vi.x) + fabsf(vj.y) + fabsf(vi.y);
-                    const float eb = 9.5367431640625e-7f * (fabsf(px) + fabsf(py)) +
-                                     9.094947017729282e-13f * (lbig * (fabsf(vx) + fabsf(vy)) + vmag * (fabsf(rx) + fabsf(ry)));
-                    bool approach;
-                    if (dotf < -eb) approach = true;
-                    else if (dotf > eb) approach = false;
-                    else {
-                        double rabx, raby, dot;
-                        pair_geom(S, B, code, P, vpi, rabx, raby, dot);
+    for (int64_t q0 = ((int64_t)blockIdx.x * kPairWarps + w) * W; q0 < a.c.n; q0 += (int64_t)gridDim.x * kPairWarps * W) {
+        const int np = (int)min((int64_t)W, a.c.n - q0);
+        const int32_t *nb = D.nbr + q0 * k;
+        const double2 *dist = D.dist + q0 * k;
+        if (lane < np) {
+            const int64_t q = q0 + lane;
+            const double2 P = B.pos[q], V = B.vp[q];
+            ForceRow &R = sm.row[lane];
+            R.x = P.x; R.y = P.y; R.vx = V.x; R.vy = V.y;
+            const double4 d = D.der[q];
+            R.c = d.x; R.rho = d.y; R.h = d.z; R.cterm = d.w;
+        }
+        __syncwarp();
+        double ax = 0.0, ay = 0.0, ed = 0.0;  // (three lanes per particle: ax alone, lane 3 p + component)
+        for (int c = 0, e_lo = k; c < ch.n; c++) {
+            const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
+            e_lo -= ce;
+            // ---- A
+            int nlist = 0, nrest = 0;
+            // a round's loads are issued a round (the neighbour's data) or two (its
+            // code) before their use
+            auto entry = [&](int i) {
+                const int p = pair_row(i, magic);
+                return p * k + e_lo + (i - p * ce);
+            };
+            uint32_t code1 = lane < npair ? (uint32_t)nb[entry(lane)] : 0u;
+            uint32_t code2 = lane + 32 < npair ? (uint32_t)nb[entry(lane + 32)] : 0u;
+            double2 V1 = B.vp[code1 >> kCodeShift], Q1 = B.pos[code1 >> kCodeShift];
+            for (int i0 = 0; i0 < npair; i0 += 32) {
+                const int i = i0 + lane;
+                bool approach = false;
+                const uint32_t code = code1;
+                const double2 V = V1, Q = Q1;
+                code1 = code2;
+                V1 = B.vp[code1 >> kCodeShift];
+                Q1 = B.pos[code1 >> kCodeShift];
+                code2 = i + 64 < npair ? (uint32_t)nb[entry(i + 64)] : 0u;
+                if (i < npair) {
+                    const int p = pair_row(i, magic), slot = i + p * (st - ce);
+                    const ForceRow &R = sm.row[p];
+                    const double vx = __dsub_rn(V.x, R.vx), vy = __dsub_rn(V.y, R.vy);
+                    double qx = Q.x, qy = Q.y;
+                    if ((code & 15u) != 4u) {
+                        double ox, oy;
+                        img_shift(a.c.sims[sim_of(a.c, q0 + p)], code & 15u, ox, oy);
+                        qx = __dsub_rn(qx, ox);
+                        qy = __dsub_rn(qy, oy);
+                    }
+                    const double rx = __dsub_rn(qx, R.x), ry = __dsub_rn(qy, R.y);
+                    double dot;
+                    if (emu_within<150>(rx) && emu_within<150>(ry) && emu_within<150>(vx) && emu_within<150>(vy)) {
+                        dot = __dadd_rn(emu_mul_n(vx, rx), emu_mul_n(vy, ry));  // 0, or 2^-353 at least (no subnormal)
+                        approach = emu_hi(dot) > 0x80000000u;
+                    } else {
+                        dot = force_dot_slow(rx, ry, vx, vy);
                         approach = dot < 0.0;
                     }
-                    if (approach) {
-                        const uint32_t bit = 1u << (e & 31);
-                        if (e < 32) m0 |= bit;
-                        else if (e < 64) m1 |= bit;
-                        else if (e < 96) m2 |= bit;
-                        else m3 |= bit;
+                    sm.x[slot] = rx;
+                    sm.y[slot] = ry;
+                    sm.e[slot] = dot;
+                }
+                const uint32_t bal = __ballot_sync(0xffffffffu, approach);
+                const int before = __popc(bal & lanemask_lt());
+                if (i < npair) sm.list[approach ? nlist + before : npair - 1 - (nrest + lane - before)] = (uint16_t)i;
+                nlist += __popc(bal);
+                nrest = min(i0 + 32, npair) - nlist;
+            }
+            __syncwarp();
+            // ---- B, the approaching pairs first: one round at most holds both kinds
+            int at = lane < npair ? entry(sm.list[lane]) : 0;
+            double2 dd1 = dist[at];  // (NNDists, dF)
+            const double4 *der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);  // (c, rho, h, c^2 / (gamma rho))
+            double c1 = 0.0, rho1 = 0.0, h1 = 0.0, ct1 = der1->w;
+            if (lane < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
+            for (int n = lane; n < npair; n += 32) {
+                const double2 dd = dd1;
+                const double cj = c1, rhoj = rho1, hj = h1, ctj = ct1;
+                if (n + 32 < npair) {
+                    at = entry(sm.list[n + 32]);
+                    dd1 = dist[at];
+                    der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);
+                    ct1 = der1->w;
+                    if (n + 32 < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
+                }
+                const int i = sm.list[n], p = pair_row(i, magic), slot = i + p * (st - ce);
+                const ForceRow &R = sm.row[p];
+                const double rx = sm.x[slot], ry = sm.y[slot], dot = sm.e[slot];
+                const bool in_r = emu_within<150>(rx) && emu_within<150>(ry);
+                double sum = R.cterm;  // Pi + cA (0 + cA = cA)
+                if (n < nlist) {
+                    const SimDev &S = a.c.sims[sim_of(a.c, q0 + p)];
+                    const double alpha = S.alpha, beta = S.beta;
+                    const double c2 = __dadd_rn(R.c, cj), rho2 = __dadd_rn(R.rho, rhoj), h2 = __dadd_rn(R.h, hj);
+                    bool ok = in_r && emu_within<400>(dot) && emu_within<150>(c2) && emu_within<150>(rho2) &&
+                              emu_within<150>(h2) && emu_within<150>(alpha) && emu_within<150>(beta);
+                    double pi = 0.0;
+                    if (ok) {
+                        const double den = __dadd_rn(__dadd_rn(emu_mul_n(rx, rx), emu_mul_n(ry, ry)), S.etasq);
+                        const double mu = emu_div_n(emu_mul_n(dot, emu_halve(h2)), emu_divisor(den));
+                        const double num = __dadd_rn(emu_mul_n(emu_mul_n(emu_neg(alpha), emu_halve(c2)), mu),
+                                                     emu_mul_n(emu_mul_n(beta, mu), mu));
+                        pi = emu_div_n(num, emu_divisor(emu_halve(rho2)));
+                        ok = emu_within<300>(den) && emu_within<300>(mu) && emu_within<800>(num);
                     }
+                    if (!ok) pi = force_pi_slow(rx, ry, dot, c2, rho2, h2, alpha, beta, S.etasq);
+                    sum = __dadd_rn(pi, sum);
                 }
-            });
-            const uint32_t mw[4] = {m0, m1, m2, m3};
-#pragma unroll
-            for (int wd = 0; wd < 4; wd++) {
-                if (wd < nw) {
-                    smask[wd * 32 + lane] = mw[wd];
-                }
-            }
-        } else {
-            for (int wd = 0; wd < nw; wd++) smask[wd * 32 + lane] = 0u;
-        }
-        // ---- 2 and 3 one chunk of 32 neighbour entries at a time (the chunk
-        // of mask word c: entries 32 c .. 32 c + 31), farthest chunk first, so
-        // the Pi table holds 32 entries per particle whatever k is; the sums run
-        // through the chunks in the reference's order (sim/sph.go:343,
-        // farthest first)
-        const double ca = di.w;
-        const double2 *dist = D.dist + q * k;
-        double ax = 0.0, ay = 0.0, ed = 0.0;
-        for (int c = nw - 1; c >= 0; c--) {
-            const int e_lo = 32 * c, e_hi = min(k, e_lo + 32);
-            const uint32_t mine = smask[c * 32 + lane];
-            int inc = __popc(mine);
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            sinc[lane] = inc;
-            const int total = __shfl_sync(0xffffffffu, inc, 31);
-            __syncwarp();
-            // ---- 2. Pi of every flagged pair of the chunk
-            for (int i = lane; i < total; i += 32) {
-                int p = 0;  // owner: the first lane whose inclusive count exceeds i
-#pragma unroll
-                for (int b = 16; b > 0; b >>= 1)
-                    if (sinc[p + b - 1] <= i) p += b;
-                const int r = i - (p ? sinc[p - 1] : 0);  // r-th flagged pair of particle p in the chunk
-                uint32_t m = smask[c * 32 + p];
-                for (int t = 0; t < r; t++) m &= m - 1;
-                const int eo = __ffs(m) - 1;  // entry e_lo + eo
-                const int64_t qp = q0 + p;
-                const SimDev &Sp = a.c.sims[sim_of(a.c, qp)];
-                const double2 Pp = B.pos[qp], vpp = B.vp[qp];
-                const double4 dp = D.der[qp];
-                const uint32_t code = (uint32_t)D.nbr[qp * k + e_lo + eo];
-                double rabx, raby, dot;
-                pair_geom(Sp, B, code, Pp, vpp, rabx, raby, dot);
-                const double4 dj = D.der[code >> kCodeShift];
-                if (MODE == MODE_EXACT64) {
-                    const double cab = __dmul_rn(0.5, __dadd_rn(dp.x, dj.x));
-                    const double rhoab = __dmul_rn(0.5, __dadd_rn(dp.y, dj.y));
-                    const double hab = __dmul_rn(0.5, __dadd_rn(dp.z, dj.z));
-                    const double r2 = __dadd_rn(__dmul_rn(rabx, rabx), __dmul_rn(raby, raby));
-                    const double den = __dadd_rn(r2, Sp.etasq);
-                    const double mu = emu_div_ol(emu_mul_ol(dot, hab), emu_divisor_ol(den), den);
-                    spi[eo * 32 + p] = emu_div_ol(__dadd_rn(emu_mul_ol(emu_mul_ol(-Sp.alpha, cab), mu),
-                                                            emu_mul_ol(emu_mul_ol(Sp.beta, mu), mu)),
-                                                  emu_divisor_ol(rhoab), rhoab);
+                // the terms r_AB (Pi + cA + cB) dF / NNDists and v_AB . r_AB dF
+                sum = __dadd_rn(sum, ctj);
+                const double d = dd.x, drk = dd.y;
+                // a zero dF (always so for the farthest neighbour) makes zero terms, whose
+                // signs do not matter to the sums, which are never -0
+                const bool dz = emu_is_zero(drk), dot0 = emu_is_zero(dot);
+                ForceTerms t;
+                if (in_r && emu_within<150>(sum) && emu_within<150>(d) && (dz || emu_within<150>(drk)) &&
+                    (emu_within<400>(dot) || dot0)) {
+                    const EmuDivisor dv = emu_divisor(d);  // shared by both quotients
+                    t.x = emu_div_n(emu_mul_n(emu_mul_n(rx, sum), drk), dv);
+                    t.y = emu_div_n(emu_mul_n(emu_mul_n(ry, sum), drk), dv);
+                    t.e = emu_mul_n(dot, drk);
+                    if (dz) t.x = t.y = 0.0;
+                    if (dz || dot0) t.e = 0.0;
                 } else {
-                    const double cab = 0.5 * (dp.x + dj.x), rhoab = 0.5 * (dp.y + dj.y), hab = 0.5 * (dp.z + dj.z);
-                    const double mu = dot * hab / (rabx * rabx + raby * raby + Sp.etasq);
-                    spi[eo * 32 + p] = mu * (Sp.beta * mu - Sp.alpha * cab) / rhoab;
+                    t = force_terms_slow(rx, ry, dot, sum, drk, d);
                 }
+                sm.x[slot] = t.x;
+                sm.y[slot] = t.y;
+                sm.e[slot] = t.e;
             }
             __syncwarp();
-            // ---- 3. the chunk's terms of the reference's ordered sums
-            if (valid) {
-                if (MODE == MODE_EXACT64) {
-                    for_each_nbr_desc_range(nb, e_lo, e_hi, k, [&](int e, uint32_t code) {
-                        const double d = dist[e].x;
-                        const double drk = dist[e].y;  // dF(NNDists[i]/maxR), evaluated by the density pass
-                        double rabx, raby, dot;
-                        pair_geom(S, B, code, P, vpi, rabx, raby, dot);
-                        const bool visc = (mine >> (e - e_lo)) & 1u;
-                        const double piab = visc ? spi[(e - e_lo) * 32 + lane] : 0.0;
-                        const double cb = D.der[code >> kCodeShift].w;
-                        const double sum3 = __dadd_rn(__dadd_rn(piab, ca), cb);
-                        // both quotients by NNDists[i] share one prepared divisor
-                        const EmuDivisor dd = emu_divisor_ol(d);
-                        ax = __dadd_rn(ax, emu_div_ol(emu_mul_ol(emu_mul_ol(rabx, sum3), drk), dd, d));
-                        ay = __dadd_rn(ay, emu_div_ol(emu_mul_ol(emu_mul_ol(raby, sum3), drk), dd, d));
-                        ed = __dadd_rn(ed, emu_mul_ol(dot, drk));
-                    });
-                } else {
-                    // the fast form keeps (dF, dF / NNDists) per neighbour
-                    for_each_nbr_desc_range(nb, e_lo, e_hi, k, [&](int e, uint32_t code) {
-                        const double2 dd = dist[e];
-                        const uint32_t j = code >> kCodeShift;
-                        const double2 vpj = B.vp[j], Q = B.pos[j];
-                        double ox = 0.0, oy = 0.0;
-                        if ((code & 15u) != 4u) img_shift(S, code & 15u, ox, oy);
-                        const double rabx = (Q.x - ox) - P.x, raby = (Q.y - oy) - P.y;
-                        const double dot = (vpj.x - vpi.x) * rabx + (vpj.y - vpi.y) * raby;
-                        const bool visc = (mine >> (e - e_lo)) & 1u;
-                        const double piab = visc ? spi[(e - e_lo) * 32 + lane] : 0.0;
-                        const double w = (piab + ca + D.der[j].w) * dd.y;
-                        ax += rabx * w;
-                        ay += raby * w;
-                        ed += dot * dd.x;
-                    });
+            // ---- C
+            if (W <= kSplitWidth) {
+                if (lane < 3 * np) {
+                    const int p = lane / 3, comp = lane - 3 * p;
+                    const double *t = (comp == 0 ? sm.x : comp == 1 ? sm.y : sm.e) + p * st;
+                    for (int e = ce - 1; e >= 0; e--) ax = __dadd_rn(ax, t[e]);
+                }
+            } else if (lane < np) {
+                const int t = lane * st;
+                for (int e = ce - 1; e >= 0; e--) {
+                    ax = __dadd_rn(ax, sm.x[t + e]);
+                    ay = __dadd_rn(ay, sm.y[t + e]);
+                    ed = __dadd_rn(ed, sm.e[t + e]);
                 }
             }
             __syncwarp();
         }
-        if (valid) {
-            const double hi = di.z;
-            double axo, ayo, edot;
-            if (MODE == MODE_EXACT64) {
-                const double f = __ddiv_rn(__dmul_rn(S.mass, S.dfpref), __dmul_rn(__dmul_rn(hi, hi), hi));
-                axo = __dadd_rn(__dmul_rn(ax, f), S.accel[0]);
-                ayo = __dadd_rn(__dmul_rn(ay, f), S.accel[1]);
-                edot = __dmul_rn(__dmul_rn(ca, ed), S.mass);
-            } else {
-                const double inv_h = 1.0 / hi;
-                const double f = S.mass * S.dfpref * (inv_h * inv_h * inv_h);
-                axo = ax * f + S.accel[0];
-                ayo = ay * f + S.accel[1];
-                edot = ca * ed * S.mass;
-            }
-            if (!isfinite(axo) || !isfinite(ayo) || !isfinite(edot)) fl |= FLAG_Q_RANGE;
-            double2 pos = P, vel = B.vel[q];
+        if (W <= kSplitWidth) {
+            const double s = ax;
+            const int l3 = min(3 * lane, 29);
+            ax = __shfl_sync(0xffffffffu, s, l3);
+            ay = __shfl_sync(0xffffffffu, s, l3 + 1);
+            ed = __shfl_sync(0xffffffffu, s, l3 + 2);
+        }
+        if (lane < np) {
+            const int64_t q = q0 + lane;
+            const ForceRow &R = sm.row[lane];
+            const SimDev &S = a.c.sims[sim_of(a.c, q)];
+            const double hi = R.h;
+            const double h3 = emu_mul(emu_mul(hi, hi), hi);
+            const double f = emu_div(emu_mul(S.mass, S.dfpref), emu_divisor(h3), h3);
+            const double axo = __dadd_rn(emu_mul(ax, f), S.accel[0]);
+            const double ayo = __dadd_rn(emu_mul(ay, f), S.accel[1]);
+            const double edot = emu_mul(emu_mul(R.cterm, ed), S.mass);
+            if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
+            double2 pos = make_double2(R.x, R.y), vel = B.vel[q];
             double u = B.u[q];
             if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
             a.A.pos[q] = pos;
@@ -361,8 +410,8 @@ __global__ void __launch_bounds__(kForceWarps * 32) k_force_fp64(ForceArgs a) {
             a.A.acc[q] = make_double2(axo, ayo);
             a.A.udot[q] = edot;
             a.A.id[q] = B.id[q];
-            a.A.hprev[q] = (float)D.h[q];
-            a.A.vp[q] = vpi;
+            a.A.hprev[q] = (float)hi;
+            a.A.vp[q] = make_double2(R.vx, R.vy);
             a.A.up[q] = B.up[q];
         }
         __syncwarp();
@@ -370,20 +419,16 @@ __global__ void __launch_bounds__(kForceWarps * 32) k_force_fp64(ForceArgs a) {
     if (fl) atomicOr(a.c.flags, fl);
 }
 
-static size_t force_exact_smem(int k) { return (size_t)kForceWarps * force_exact_warp_bytes(k); }
-
-static int g_force_exact_blocks[129];  // resident blocks per SM by k (filled before any capture)
+constexpr size_t kForceSmem = kPairWarps * sizeof(ForceWarp);
+static int g_force_blocks;  // resident blocks per SM (set before any capture)
 
 // Sets the shared-memory limit of the FP64 force kernel and records its
-// occupancy for k; must run before any stream capture.
-void force_init_attrs(int k) {
-    cudaFuncSetAttribute(k_force_fp64<MODE_EXACT64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_exact_smem(128));
-    cudaFuncSetAttribute(k_force_fp64<MODE_FAST64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_exact_smem(128));
-    if (k >= 1 && k <= 128 && !g_force_exact_blocks[k]) {
-        int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64<MODE_EXACT64>, kForceWarps * 32, force_exact_smem(k));
-        g_force_exact_blocks[k] = std::max(nb, 1);
-    }
+// occupancy; must run before any stream capture.
+void force_init_attrs() {
+    cudaFuncSetAttribute(k_force_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForceSmem);
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64, kPairWarps * 32, kForceSmem);
+    g_force_blocks = std::max(nb, 1);
 }
 
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
@@ -394,19 +439,18 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
     a.A = A;
     a.D = D;
     a.integrate = integrate ? 1 : 0;
-    const int block = 128;
-    int64_t need = (c.n + block - 1) / block;
-    int grid = (int)(need < (int64_t)L.sms * 16 ? need : (int64_t)L.sms * 16);
-    if (grid < 1) grid = 1;
-    if (mode == MODE_EXACT64 || mode == MODE_FAST64) {
-        const int64_t tiles = (c.n + 31) / 32;
-        const int64_t eneed = (tiles + kForceWarps - 1) / kForceWarps;
-        const int nb = c.k >= 1 && c.k <= 128 ? std::max(g_force_exact_blocks[c.k], 1) : 1;
-        const int eg = (int)std::max<int64_t>(1, std::min<int64_t>(eneed, (int64_t)L.sms * nb));
-        if (mode == MODE_EXACT64) k_force_fp64<MODE_EXACT64><<<eg, kForceWarps * 32, force_exact_smem(c.k), L.stream>>>(a);
-        else k_force_fp64<MODE_FAST64><<<eg, kForceWarps * 32, force_exact_smem(c.k), L.stream>>>(a);
+    if (mode != MODE_MIXED) {
+        const int nb = std::max(g_force_blocks, 1);
+        const int W = pair_width(c.n, (int64_t)L.sms * nb * kPairWarps);
+        const int64_t tiles = (c.n + W - 1) / W;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((tiles + kPairWarps - 1) / kPairWarps, (int64_t)L.sms * nb));
+        k_force_fp64<<<grid, kPairWarps * 32, kForceSmem, L.stream>>>(a, W);
+        return;
     }
-    else k_force<MODE_MIXED><<<grid, block, 0, L.stream>>>(a);
+    const int block = 128;
+    const int64_t need = (c.n + block - 1) / block;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)L.sms * 16));
+    k_force<MODE_MIXED><<<grid, block, 0, L.stream>>>(a);
 }
 
 // ------------------------------------------------------------ error norms

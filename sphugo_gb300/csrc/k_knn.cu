@@ -22,8 +22,8 @@
 //   5. every order the FP32 values cannot decide (entries within 2 eps of each
 //      other) is settled with the reference's FP64 squared distance, ties
 //      broken by (particle id, image code); the FP64 forms settle all of them.
-// k_density, one thread per particle: smoothing length h = sqrt of the k-th
-// FP64 squared distance, density (sim/sph.go:306-323),
+// k_density_mixed, one thread per particle: the mixed form's smoothing length
+// (sqrt of the k-th FP64 squared distance), density (sim/sph.go:306-323),
 // c = sqrt(gamma (gamma-1) u_pred) and c^2/(gamma rho).
 // The neighbour set and its order are identical in every arithmetic form.
 #include "knn_shared.cuh"
@@ -937,104 +937,47 @@ __global__ void __launch_bounds__(kTileWarps * 32, (MODE == MODE_MIXED || NR > 2
 }
 
 // ---------------------------------------------------------------- density
-// five resident blocks (48 registers): the FP64 forms' first loop waits on the
-// neighbour gathers, and more resident warps hide them (2.06 -> 2.02 ms at N = 1M)
-template <int MODE>
-__global__ void __launch_bounds__(256, 4) k_density(KnnArgs a) {
+// The mixed form's density (the FP64 forms': k_density.cu), one thread per
+// particle: all of them, or (use_defer) only the queries the block tiles left
+// to the per-query search, since the tiles computed the others' densities.
+__global__ void __launch_bounds__(256, 4) k_density_mixed(KnnArgs a) {
     const int k = a.c.k;
     const PArrays &B = a.B;
     unsigned fl = 0;
-    // all particles, or (use_defer) only the queries the block tiles left to
-    // the per-query search: the tiles computed the others' densities
     const int64_t nq = a.use_defer ? (int64_t)*a.D.ndefer : a.c.n;
     for (int64_t qi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; qi < nq;
          qi += (int64_t)gridDim.x * blockDim.x) {
         const int64_t q = a.use_defer ? (int64_t)a.D.defer[qi] : qi;
-        const int s = sim_of(a.c, q);
-        const SimDev &S = a.c.sims[s];
-        const double gamma = S.gamma;
-        const double up = B.up[q];
-        double h, rho, cs, cterm;
-        if (MODE == MODE_FAST64) {
-            double2 *dist = a.D.dist + q * k;
-            const double2 P = B.pos[q];
-            const int32_t *nb = a.D.nbr + q * k;
-            const double dk2 = nbr_d2(S, B, P, (uint32_t)nb[k - 1]);
-            if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
-            h = emu_sqrt(dk2);
-            const double inv_h = 1.0 / h;
-            // q and 1/NNDists first; then the kernel sums and dF in branch-split
-            // loops (q grows with e), leaving (dF, dF / NNDists) for the force
-            int s_lo = 0;
-            for_each_nbr_desc(nb, k, [&](int e, uint32_t code) {
-                const double d2 = e == k - 1 ? dk2 : nbr_d2(S, B, P, code);
-                const double y = rsqrt(d2);
-                const double x = fmin(d2 * y * inv_h, 1.0);
-                s_lo += x < 0.5;
-                dist[e] = make_double2(x, y);
-            });
-            double acc = 0.0;
-            if (S.kernel == SPH_KERNEL_WENDLAND) {
-                for (int e = k - 1; e >= 0; e--) {
-                    const double2 xy = dist[e];
-                    acc += kf_fast(SPH_KERNEL_WENDLAND, xy.x);
-                    const double drk = kdf_fast(SPH_KERNEL_WENDLAND, xy.x);
-                    dist[e] = make_double2(drk, drk * xy.y);
-                }
-            } else {
-                for (int e = k - 1; e >= s_lo; e--) {
-                    const double2 xy = dist[e];
-                    const double a1 = 1.0 - xy.x, a2 = a1 * a1;
-                    acc += a2 * a1 * (1.0 / 3.0);
-                    dist[e] = make_double2(-a2, -a2 * xy.y);
-                }
-                for (int e = s_lo - 1; e >= 0; e--) {
-                    const double2 xy = dist[e];
-                    acc += (xy.x - 1.0) * xy.x * xy.x + (1.0 / 6.0);
-                    const double drk = (3.0 * xy.x - 2.0) * xy.x;
-                    dist[e] = make_double2(drk, drk * xy.y);
-                }
+        const SimDev &S = a.c.sims[sim_of(a.c, q)];
+        // FP64 only where it decides: the k-th neighbour's squared distance and h
+        const double dk2 = nbr_d2(S, B, B.pos[q], (uint32_t)a.D.nbr[q * k + k - 1]);
+        if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
+        const double h = emu_sqrt(dk2);
+        // everything after h in FP32 (prefactors from FP32 copies)
+        const float hf = __double2float_rn(h);
+        const float inv_hf = 1.f / hf;
+        const float *d2f = a.D.d2f + q * k;
+        KahanF acc;
+        auto term = [&](float v) { acc.add(kf_f32(S.kernel, fminf(sqrtf(v) * inv_hf, 1.f))); };
+        if ((k & 3) == 0) {  // farthest first, four values per load
+            const float4 *d4 = reinterpret_cast<const float4 *>(d2f);
+            for (int b = (k >> 2) - 1; b >= 0; b--) {
+                const float4 v = d4[b];
+                term(v.w);
+                term(v.z);
+                term(v.y);
+                term(v.x);
             }
-            rho = S.fpref * S.mass * acc * (inv_h * inv_h);
-            if (!(rho >= 0.0 && rho < 1.0e308)) fl |= FLAG_Q_RANGE;
-            cs = sqrt(gamma * (gamma - 1.0) * up);
-            cterm = cs * cs / (gamma * rho);
         } else {
-            // FP64 only where it decides: the k-th neighbour's squared distance and h
-            const double dk2 = nbr_d2(S, B, B.pos[q], (uint32_t)a.D.nbr[q * k + k - 1]);
-            if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
-            h = emu_sqrt(dk2);
-            // everything after h in FP32 (prefactors from FP32 copies)
-            const float hf = __double2float_rn(h);
-            const float inv_hf = 1.f / hf;
-            const float *d2f = a.D.d2f + q * k;
-            KahanF acc;
-            auto term = [&](float v) { acc.add(kf_f32(S.kernel, fminf(sqrtf(v) * inv_hf, 1.f))); };
-            if ((k & 3) == 0) {  // farthest first, four values per load
-                const float4 *d4 = reinterpret_cast<const float4 *>(d2f);
-                for (int b = (k >> 2) - 1; b >= 0; b--) {
-                    const float4 v = d4[b];
-                    term(v.w);
-                    term(v.z);
-                    term(v.y);
-                    term(v.x);
-                }
-            } else {
-                for (int e = k - 1; e >= 0; e--) term(d2f[e]);
-            }
-            const float rhof = S.ffm * (inv_hf * inv_hf) * acc.value_f();
-            const float csf = sqrtf(S.fgg1 * __double2float_rn(up));
-            const float ctf = csf * csf / (S.fgamma * rhof);
-            a.D.rho[q] = rhof;
-            a.D.c[q] = csf;
-            a.D.h[q] = h;
-            a.D.derf[q] = make_float4(csf, rhof, hf, ctf);
-            continue;
+            for (int e = k - 1; e >= 0; e--) term(d2f[e]);
         }
-        a.D.rho[q] = rho;
-        a.D.c[q] = cs;
+        const float rhof = S.ffm * (inv_hf * inv_hf) * acc.value_f();
+        const float csf = sqrtf(S.fgg1 * __double2float_rn(B.up[q]));
+        const float ctf = csf * csf / (S.fgamma * rhof);
+        a.D.rho[q] = rhof;
+        a.D.c[q] = csf;
         a.D.h[q] = h;
-        a.D.der[q] = make_double4(cs, rho, h, cterm);
+        a.D.derf[q] = make_float4(csf, rhof, hf, ctf);
     }
     if (fl) atomicOr(a.c.flags, fl);
 }
@@ -1066,7 +1009,6 @@ static void knn_attrs_mode() {
 // before any stream capture.
 void knn_init_attrs() {
     knn_attrs_mode<MODE_EXACT64>();
-    knn_attrs_mode<MODE_FAST64>();
     knn_attrs_mode<MODE_MIXED>();
     knn_block_init_attrs();
 }
@@ -1090,7 +1032,6 @@ int knn_occupancy_blocks(int, int cap, int mode) {
     const int nr = list_regs(std::max(1, cap - 16));
     auto pick = [&](auto f1, auto f2, auto f4, auto f8) { return nr == 1 ? f1(0) : nr == 2 ? f2(0) : nr == 4 ? f4(0) : f8(0); };
     if (mode == MODE_EXACT64) return pick(occ<MODE_EXACT64, 1>, occ<MODE_EXACT64, 2>, occ<MODE_EXACT64, 4>, occ<MODE_EXACT64, 8>);
-    if (mode == MODE_FAST64) return pick(occ<MODE_FAST64, 1>, occ<MODE_FAST64, 2>, occ<MODE_FAST64, 4>, occ<MODE_FAST64, 8>);
     return pick(occ<MODE_MIXED, 1>, occ<MODE_MIXED, 2>, occ<MODE_MIXED, 4>, occ<MODE_MIXED, 8>);
 }
 
@@ -1099,8 +1040,6 @@ int knn_tile_occupancy_blocks(int k, int mode) {
     auto pick = [&](auto f1, auto f2, auto f4, auto f8) { return nr == 1 ? f1(0) : nr == 2 ? f2(0) : nr == 4 ? f4(0) : f8(0); };
     if (mode == MODE_EXACT64)
         return pick(occ_tile<MODE_EXACT64, 1>, occ_tile<MODE_EXACT64, 2>, occ_tile<MODE_EXACT64, 4>, occ_tile<MODE_EXACT64, 8>);
-    if (mode == MODE_FAST64)
-        return pick(occ_tile<MODE_FAST64, 1>, occ_tile<MODE_FAST64, 2>, occ_tile<MODE_FAST64, 4>, occ_tile<MODE_FAST64, 8>);
     return pick(occ_tile<MODE_MIXED, 1>, occ_tile<MODE_MIXED, 2>, occ_tile<MODE_MIXED, 4>, occ_tile<MODE_MIXED, 8>);
 }
 
@@ -1184,13 +1123,6 @@ static void run_knn(const KnnArgs &args, const Launch &L, const KnnTune &tune) {
     else launch_knn_nr<MODE, 8>(args, L, tune);
 }
 
-template <int MODE>
-static void run_density(const KnnArgs &args, const Launch &L) {
-    const int64_t dneed = (args.c.n + 255) / 256;
-    const int dgrid = (int)std::max<int64_t>(1, std::min<int64_t>(dneed, (int64_t)L.sms * 8));
-    k_density<MODE><<<dgrid, 256, 0, L.stream>>>(args);
-}
-
 void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D,
                 const Tables &T, int mode, const KnnTune &tune) {
     KnnArgs a;
@@ -1203,20 +1135,23 @@ void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &
     a.use_defer = 0;
     a.fuse_density = knn_fuses_density(c.k, mode, tune) ? 1 : 0;
     if (mode == MODE_EXACT64) run_knn<MODE_EXACT64>(a, L, tune);
-    else if (mode == MODE_FAST64) run_knn<MODE_FAST64>(a, L, tune);
     else run_knn<MODE_MIXED>(a, L, tune);
 }
 
 void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int mode,
                     const KnnTune *tune) {
+    if (mode != MODE_MIXED) {
+        launch_density_fp64(c, L, B, D);
+        return;
+    }
     KnnArgs a{};
     a.c = c;
     a.B = B;
     a.D = D;
     a.use_defer = tune && D.defer && knn_fuses_density(c.k, mode, *tune) ? 1 : 0;
-    if (mode == MODE_EXACT64) launch_density_fp64(c, L, B, D);
-    else if (mode == MODE_FAST64) run_density<MODE_FAST64>(a, L);
-    else run_density<MODE_MIXED>(a, L);
+    const int64_t dneed = (c.n + 255) / 256;
+    const int dgrid = (int)std::max<int64_t>(1, std::min<int64_t>(dneed, (int64_t)L.sms * 8));
+    k_density_mixed<<<dgrid, 256, 0, L.stream>>>(a);
 }
 
 }  // namespace sphgpu

@@ -648,7 +648,6 @@ static void block_attrs_mode() {
 // records its occupancy; must run before any stream capture.
 void knn_block_init_attrs() {
     block_attrs_mode<MODE_EXACT64>();
-    block_attrs_mode<MODE_FAST64>();
     block_attrs_mode<MODE_MIXED>();
 }
 
@@ -680,7 +679,6 @@ static bool block_mode(const KnnArgs &args, const Launch &L, int nr, int warps) 
 // false when no block kernel serves this list shape (the warp tiles do).
 bool launch_knn_block(const KnnArgs &args, const Launch &L, int mode, int nr, int warps) {
     if (mode == MODE_EXACT64) return block_mode<MODE_EXACT64>(args, L, nr, warps);
-    if (mode == MODE_FAST64) return block_mode<MODE_FAST64>(args, L, nr, warps);
     return block_mode<MODE_MIXED>(args, L, nr, warps);
 }
 

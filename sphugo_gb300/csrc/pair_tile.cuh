@@ -4,17 +4,16 @@
 // The reference sums each particle's neighbour terms in list order, farthest
 // first, with a rounding per addition, so the additions of one particle are a
 // chain; the terms themselves are independent and hold nearly all the work.
-// A warp takes a tile of W particles and, chunk by chunk of at most 32 / W * 8
-// entries (farthest chunk first), computes the W x chunk terms with one lane
-// per (particle, entry) pair, leaves them in shared memory, and then a lane per
+// A warp takes a tile of W particles and, chunk by chunk of their lists
+// (farthest chunk first), computes the W x chunk terms with one lane per
+// (particle, entry) pair, leaves them in shared memory, and then a lane per
 // particle adds its terms in order.
 //
-// W = 32 when there are enough particles to fill the GPU (the ordered sums
-// then use all lanes, as one thread per particle would); fewer particles take
-// a smaller W, down to one particle per warp: the terms of a particle's list
-// run side by side in the lanes, where one thread per particle computed them
-// one after the other in a few resident warps (N = 10,000: 313 warps on 608
-// sub-partitions).
+// W follows the particle count: the warps the GPU holds at once take equal
+// shares, of 32 particles at most. With few particles that is one or a few per
+// warp: the terms of a particle's list run side by side in the lanes, where
+// one thread per particle computed them one after the other in a few resident
+// warps (N = 10,000: 313 warps on 608 sub-partitions).
 #pragma once
 #include "physics.cuh"
 
@@ -23,20 +22,31 @@ namespace sphgpu {
 constexpr int kPairWarps = 4;    // warps per block (each works alone)
 constexpr int kPairSlots = 288;  // terms a warp's tile holds: W (chunk | 1) at most
 
-// Entries per chunk at tile width W.
-__host__ __device__ constexpr int pair_chunk(int W) { return W >= 32 ? 8 : W >= 16 ? 16 : 32; }
 // A row of ce terms is kept at an odd stride (in doubles), so that the lanes
 // of the ordered sums, one row each, meet every bank pair once.
 __host__ __device__ constexpr int pair_stride(int ce) { return ce | 1; }
-static_assert(32 * pair_stride(8) <= kPairSlots && 16 * pair_stride(16) <= kPairSlots && 8 * pair_stride(32) <= kPairSlots,
-              "a tile's terms fit its slots at every width");
+// Entries per chunk at tile width W: the most, up to 32, whose rows fit.
+__host__ __device__ constexpr int pair_chunk(int W) {
+    const int t = kPairSlots / W, c = t & 1 ? t : t - 1;
+    return c < 32 ? c : 32;
+}
+constexpr bool pair_rows_fit() {
+    for (int W = 1; W <= 32; W++)
+        for (int ce = 1; ce <= pair_chunk(W); ce++)
+            if (W * pair_stride(ce) > kPairSlots) return false;
+    return true;
+}
+static_assert(pair_rows_fit(), "a tile's terms fit its slots at every width");
 
-// The smallest power of two that covers n particles with the warps the GPU
-// holds at once, at most 32.
+// Particles per tile for n particles on the warps the GPU holds at once: equal
+// shares in one pass; or in two when full tiles would leave less than an
+// eighth of a pass over (force stage at N = 100,000, 1.03 passes: 148 us at 17
+// particles, 168 at 32); else full tiles, whose lanes are all at work in the
+// ordered sums (density stage at N = 200,001, 1.28 passes: 157 us at 32, 171
+// at 21).
 inline int pair_width(int64_t n, int64_t resident_warps) {
-    int W = 1;
-    while (W < 32 && (int64_t)W * resident_warps < n) W *= 2;
-    return W;
+    const int64_t passes = n <= 32 * resident_warps ? 1 : n <= 36 * resident_warps ? 2 : 0;
+    return passes ? (int)((n + resident_warps * passes - 1) / (resident_warps * passes)) : 32;
 }
 
 // Chunk c = 0, 1, ... of a list of k entries, farthest first: entries

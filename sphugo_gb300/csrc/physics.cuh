@@ -1,10 +1,9 @@
-// physics.cuh -- SPH kernel functions in the three arithmetic forms.
+// physics.cuh -- SPH kernel functions in FP64 and FP32.
 //
-// EXACT64 keeps the reference's operation order with every product and sum
-// rounded separately (no contraction), so its results equal a -ffp-contract=off
-// restatement of sim/sph.go bit for bit. FAST64 lets the compiler contract
-// into FMA and replaces per-neighbour divisions by per-particle reciprocals
-// (agreement within ~1e-14 relative). The float forms serve the mixed path.
+// The FP64 functions keep the reference's operation order with every product
+// and sum rounded separately (no contraction), so their results equal a
+// -ffp-contract=off restatement of sim/sph.go bit for bit. The float functions
+// serve the mixed form.
 #pragma once
 
 #include "common.cuh"
@@ -61,26 +60,6 @@ __device__ __forceinline__ double kdf_exact(int kernel, double q) {
     if (q < 0.5) return __dsub_rn(__dmul_rn(__dmul_rn(3.0, q), q), __dmul_rn(2.0, q));
     double a = __dsub_rn(1.0, q);
     return __dmul_rn(-a, a);
-}
-
-// contractible FP64 forms
-__device__ __forceinline__ double kf_fast(int kernel, double q) {
-    if (kernel == SPH_KERNEL_WENDLAND) {
-        double a = 1.0 - q, a2 = a * a;
-        return a2 * a2 * (1.0 + 4.0 * q);
-    }
-    if (q < 0.5) return (q - 1.0) * q * q + (1.0 / 6.0);
-    double a = 1.0 - q;
-    return a * a * a * (1.0 / 3.0);
-}
-__device__ __forceinline__ double kdf_fast(int kernel, double q) {
-    if (kernel == SPH_KERNEL_WENDLAND) {
-        double a = 1.0 - q;
-        return -10.0 * q * a * a * a;
-    }
-    if (q < 0.5) return (3.0 * q - 2.0) * q;
-    double a = 1.0 - q;
-    return -(a * a);
 }
 
 // FP32 forms (mixed path)

@@ -63,6 +63,7 @@ def test_operands_left_to_the_hardware(gpu, oracle, n):
     z = np.zeros(n)
     for vx, vy, dt in [(z, z, 1e-4),                                        # at rest
                        (np.full(n, 0.25), r.normal(0, 1e-170, n), 1e-4),    # equal, and tiny, velocities
+                       (r.normal(0, 1e-306, n), r.normal(0, 1e-306, n), 1e-300),  # products below the normal range
                        (1e37 * np.sign(np.sin(7 * x)), z, 1e-100)]:         # huge ones
         check(oracle, ics.periodic_config(n, 32, dt), (x, y, vx, vy, np.ones(n)))
     x, y, vx, vy, u = flow(n, 5)
