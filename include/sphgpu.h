@@ -189,8 +189,9 @@ int32_t sph_kernels_per_step(sph_handle *h);
 /* Neighbour search path (no reference counterpart): tiles of candidate
  * records in shared memory scanned by one thread per query, the queries they
  * cannot settle finished by the per-query search. 1 (default) = the default
- * tile shape for k (block tiles of 8 warps = 256 consecutive particles for
- * k <= 37, of 4 warps for k <= 80, else one tile per warp); 4 or 8 = block
+ * for k and the particle count (block tiles of 8 warps = 256 consecutive
+ * particles for k <= 37, of 4 warps for k <= 80, else one tile per warp; in
+ * the FP64 forms the per-query search up to 16,384 particles); 4 or 8 = block
  * tiles of that many warps; 2 = one tile per warp (32 particles); 0 =
  * per-query search for every particle. The neighbour sets and every FP64
  * result are identical on every path; the mixed form's FP32 sums may differ

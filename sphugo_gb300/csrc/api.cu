@@ -52,6 +52,16 @@ int default_block_warps(int k) {
     return need <= 64 ? 8 : need <= 128 ? 4 : 0;
 }
 
+// Whether the default search is the per-query one. With few particles the
+// block tiles are few (40 of 256 queries at N = 10,000, on 152 SMs), and a
+// tile's chain of steps is longer than a warp per query, of which all are
+// resident at once. FP64 forms, kNN stage: N = 1000 26 us with tiles, 12
+// without, 3000 33 and 14, 10,000 34 and 23, 30,000 38 and 45. The mixed form
+// keeps the tiles at every size: its sums follow the order of the lists they
+// leave, and a changed default would move its results in the last bits.
+constexpr int64_t kPerQueryMaxN = 16384;
+bool default_per_query(int64_t n, int mode) { return mode != MODE_MIXED && n <= kPerQueryMaxN; }
+
 int auto_level(int64_t n) {
     // about one to four particles per finest cell
     double l = std::floor(0.5 * std::log2(std::max<double>((double)n, 2.0) / 2.0) + 0.5);
@@ -85,6 +95,7 @@ struct sph_handle {
     Derived D{};
     Tables T{};
     KnnTune tune{};
+    bool search_default = true;  // the search path follows k and n (not set by the caller, the tuner or a checkpoint)
     bool any_open = false, uploaded = false, evaluated = false;
     std::vector<int> base_level;  // per simulation; explicit grid_level or automatic
     std::vector<bool> auto_lvl;   // true when the level is the automatic one (the tuner may shift it)
@@ -456,7 +467,7 @@ int create_impl(const sph_params *params, const int64_t *counts, int32_t nsims, 
     h->tune.theta = 0.5f;
     h->tune.hgrow = 1.04f;
     h->tune.blocks_per_sm = std::max(1, knn_occupancy_blocks(h->tune.block, h->tune.cap, kernel_mode(h->mode)));
-    h->tune.tile = 1;
+    h->tune.tile = default_per_query(n, h->mode) ? 0 : 1;
     h->tune.tile_blocks_per_sm = std::max(1, knn_tile_occupancy_blocks((int)k, kernel_mode(h->mode)));
     h->tune.block_warps = default_block_warps((int)k);
     cudaError_t e = cudaDeviceSynchronize();
@@ -751,6 +762,7 @@ int sph_append(sph_handle *h, int64_t count, const double *x, const double *y, c
     CUDA_TRY(cudaMemcpyAsync(h->d_offs, h->offs.data(), 2 * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     draw_keys_append(h, n0, count, z);
+    if (h->search_default) h->tune.tile = default_per_query(n1, h->mode) ? 0 : 1;
     destroy_graphs(h);
     return SPH_OK;
 }
@@ -1063,7 +1075,8 @@ int sph_set_search(sph_handle *h, int32_t tiles) {
     const int bdef = default_block_warps(h->k);
     if ((tiles == 4 || tiles == 8) && tiles > bdef)
         return fail(SPH_ERR_ARG, "no block tiles of that many warps for this k");
-    const int tile = tiles ? 1 : 0;
+    h->search_default = tiles == 1;
+    const int tile = tiles == 1 ? (default_per_query(h->n, h->mode) ? 0 : 1) : tiles ? 1 : 0;
     const int block = tiles == 1 ? bdef : tiles == 2 ? 0 : tiles == 0 ? h->tune.block_warps : tiles;
     if (h->tune.tile != tile || h->tune.block_warps != block) {
         h->tune.tile = tile;
@@ -1186,6 +1199,7 @@ int sph_autotune(sph_handle *h, int32_t use_cache, char *report, int32_t report_
         tune_cache_put(key, best);
     }
     h->tune = base;
+    h->search_default = false;
     h->tune.theta = best.theta;
     h->tune.hgrow = best.hgrow;
     h->tune.tile = best.tile;
@@ -1342,6 +1356,7 @@ int sph_load(sph_handle *h, const char *path) {
     }
     if ((rc = check_checkpoint(h, hd, bufs))) return rc;
     if (hd.level_delta != h->level_delta && (rc = apply_levels(h, hd.level_delta))) return rc;
+    h->search_default = false;  // the saved run's search
     if (hd.theta != h->tune.theta || hd.hgrow != h->tune.hgrow || hd.tile != h->tune.tile ||
         hd.block_warps != h->tune.block_warps) {
         h->tune.theta = hd.theta;
