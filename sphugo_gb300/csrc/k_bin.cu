@@ -27,24 +27,91 @@ void launch_prep(const Ctx &c, const Launch &L, bool) {
 }
 
 // ------------------------------------------------------------------ bbox
-// Bounding box of the predicted positions, for simulations with an open axis.
-__global__ void k_bbox(Ctx c, PArrays A, int pred) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < c.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        int s = sim_of(c, i);
-        const SimDev &S = c.sims[s];
-        if (S.periodic[0] && S.periodic[1]) continue;
-        double2 p, vp;
-        double up;
-        predict(S, pred, A.pos[i], A.vel[i], A.acc[i], A.u[i], A.udot[i], A.vp[i], A.up[i], p, vp, up);
-        SimDev &W = c.sims_rw[s];
-        if (!S.periodic[0]) { atomicMin(&W.bbox[0], dkey(p.x)); atomicMax(&W.bbox[1], dkey(p.x)); }
-        if (!S.periodic[1]) { atomicMin(&W.bbox[2], dkey(p.y)); atomicMax(&W.bbox[3], dkey(p.y)); }
+// Bounding box of the predicted positions, for simulations with an open axis,
+// as ordered 64-bit keys. A block takes one contiguous range of slots, so
+// nearly every block (and nearly every warp of the others) lies in a single
+// simulation; its threads reduce their keys first and one of them does the
+// four atomics. With four atomics per particle, all on the same words, the
+// kernel took 760 us at N = 300,000 (170 at 65,537).
+__device__ __forceinline__ unsigned long long key_min(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
+__device__ __forceinline__ unsigned long long key_max(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+
+struct BoxKeys {
+    unsigned long long k[4];  // min x, max x, min y, max y
+    __device__ __forceinline__ void clear() { k[0] = k[2] = ~0ull; k[1] = k[3] = 0ull; }
+    __device__ __forceinline__ void add(double2 p) {
+        const unsigned long long x = dkey(p.x), y = dkey(p.y);
+        k[0] = key_min(k[0], x);
+        k[1] = key_max(k[1], x);
+        k[2] = key_min(k[2], y);
+        k[3] = key_max(k[3], y);
+    }
+    __device__ __forceinline__ void reduce_warp() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, k[i], o);
+                k[i] = i & 1 ? key_max(k[i], v) : key_min(k[i], v);
+            }
+        }
+    }
+    __device__ __forceinline__ void flush(const SimDev &S, SimDev &W) const {
+        if (!S.periodic[0]) { atomicMin(&W.bbox[0], k[0]); atomicMax(&W.bbox[1], k[1]); }
+        if (!S.periodic[1]) { atomicMin(&W.bbox[2], k[2]); atomicMax(&W.bbox[3], k[3]); }
+    }
+};
+
+__global__ void __launch_bounds__(256) k_bbox(Ctx c, PArrays A, int pred) {
+    __shared__ BoxKeys part[8];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t per = (c.n + gridDim.x - 1) / gridDim.x;
+    const int64_t i0 = blockIdx.x * per, i1 = min(c.n, i0 + per);
+    if (i0 >= i1) return;
+    const int s0 = sim_of(c, i0);
+    const bool one = s0 == sim_of(c, i1 - 1);  // slots are ordered by simulation
+    BoxKeys b;
+    b.clear();
+    for (int64_t base = i0; base < i1; base += blockDim.x) {
+        const int64_t i = base + threadIdx.x;
+        if (!one) b.clear();
+        int s = s0;
+        if (i < i1) {
+            s = sim_of(c, i);
+            double2 p = A.pos[i];
+            if (pred == PRED_DRIFT) {  // predict()'s position
+                const double2 v = A.vel[i];
+                const double dth = c.sims[s].dth;
+                p.x = __dadd_rn(p.x, emu_mul(v.x, dth));
+                p.y = __dadd_rn(p.y, emu_mul(v.y, dth));
+            }
+            b.add(p);
+        }
+        if (!one) {
+            const uint32_t live = __ballot_sync(0xffffffffu, i < i1);
+            const int first = __shfl_sync(0xffffffffu, s, 0);
+            if (__all_sync(0xffffffffu, i >= i1 || s == first)) {
+                b.reduce_warp();
+                if (live && lane == 0) b.flush(c.sims[first], c.sims_rw[first]);
+            } else if (i < i1) {
+                b.flush(c.sims[s], c.sims_rw[s]);
+            }
+        }
+    }
+    if (!one) return;
+    b.reduce_warp();
+    if (lane == 0) part[w] = b;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int j = 1; j < (int)(blockDim.x >> 5); j++)
+            for (int i = 0; i < 4; i++) b.k[i] = i & 1 ? key_max(b.k[i], part[j].k[i]) : key_min(b.k[i], part[j].k[i]);
+        b.flush(c.sims[s0], c.sims_rw[s0]);
     }
 }
 
 void launch_bbox(const Ctx &c, const Launch &L, const PArrays &A, int pred) {
-    k_bbox<<<L.sms * 4, 256, 0, L.stream>>>(c, A, pred);
+    const int64_t need = (c.n + 255) / 256;
+    k_bbox<<<(int)(need < (int64_t)L.sms * 4 ? need : (int64_t)L.sms * 4), 256, 0, L.stream>>>(c, A, pred);
 }
 
 // Grid of open axes from the bounding box (one thread per sim).
