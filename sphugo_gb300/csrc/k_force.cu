@@ -12,6 +12,12 @@ namespace sphgpu {
 
 // Resident blocks of the FP64 force per SM (96 registers, 38 KB): 1160 us at
 // N = 1,048,576; 4 blocks 1198, 6 (80 registers) slower still.
+// Particles up to which the mixed force deals its pairs over the lanes (force
+// stage with and without: N = 1000 12 and 18 us, 10,000 17 and 20, 20,000 20
+// and 20, 100,000 39 and 29: a thread per particle then fills the GPU, and
+// the factors' way through shared memory costs issue slots).
+constexpr int64_t kMixedPairsMaxN = 16384;
+constexpr int kMixedBlocks = 5;  // resident blocks per SM (31 KB each)
 constexpr int kForceBlocks = 5;
 // Tiles up to this width sum with three lanes per particle: 31 us at N = 10,000
 // against 40 with one.
@@ -61,10 +67,11 @@ __device__ __forceinline__ void integrate_one(const SimDev &S, double2 &pos, dou
     if (fy && less(S.refl[3], pos.y)) { pos.y = __dsub_rn(pos.y, __dsub_rn(pos.y, S.refl[3])); vel.y = emu_neg(vel.y); }
 }
 
-// The mixed form (the FP64 forms run k_force_fp64 below).
-template <int MODE>
-__global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
-    static_assert(MODE == MODE_MIXED, "the FP64 forms run k_force_fp64");
+// The mixed form, one thread per particle. Bound by its neighbour gathers (ncu,
+// uniform blast N = 1,048,576: L1 data path 69 % busy, 9 cycles of waiting on
+// loads per issued instruction); 80 registers: at the 10 or 12 resident blocks
+// that fewer would allow it ran 271 and 328 us against 217.
+__global__ void __launch_bounds__(128, 6) k_force_mixed(ForceArgs a) {
     const int k = a.c.k;
     const PArrays &B = a.B;
     const Derived &D = a.D;
@@ -130,9 +137,132 @@ __global__ void __launch_bounds__(256, 4) k_force(ForceArgs a) {
         a.A.acc[q] = make_double2(axo, ayo);
         a.A.udot[q] = edot;
         a.A.id[q] = B.id[q];
-        a.A.hprev[q] = (float)D.h[q];
+        a.A.hprev[q] = a.D.derf[q].z;  // the smoothing length rounded to FP32
         a.A.vp[q] = B.vp[q];
         a.A.up[q] = B.up[q];
+    }
+    if (fl) atomicOr(a.c.flags, fl);
+}
+
+// The mixed form for few particles: the same arithmetic with the pairs
+// dealt over the lanes (pair_tile.cuh). Each pair leaves its factors in shared
+// memory, and a lane per particle runs the compensated sums over them,
+// farthest first, a term's product fused with the compensation's subtraction
+// as in the loop above, so that both kernels return the same bits.
+struct MixedRow {
+    float4 rec, vrec;  // position and predicted velocity as float pairs
+    float inv_h, cterm, h, c, rho;
+    int32_t sim;
+};
+
+struct MixedWarp {
+    float rx[kPairSlots], ry[kPairSlots], w[kPairSlots], dot[kPairSlots], drk[kPairSlots];
+    MixedRow row[32];
+};
+
+// Kahan's sum with the next term a product: y = x f - c in one rounding
+__device__ __forceinline__ void kahan_fma(KahanF &s, float x, float f) {
+    const float y = __fmaf_rn(x, f, -s.c);
+    const float t = __fadd_rn(s.s, y);
+    s.c = __fsub_rn(__fsub_rn(t, s.s), y);
+    s.s = t;
+}
+
+__global__ void __launch_bounds__(kPairWarps * 32, kMixedBlocks) k_force_mixed_pairs(ForceArgs a, int W) {
+    __shared__ MixedWarp smem[kPairWarps];
+    const int k = a.c.k;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    MixedWarp &sm = smem[w];
+    const PArrays &B = a.B;
+    const Derived &D = a.D;
+    const PairChunks ch(k, W);
+    unsigned fl = 0;
+    for (int64_t q0 = ((int64_t)blockIdx.x * kPairWarps + w) * W; q0 < a.c.n; q0 += (int64_t)gridDim.x * kPairWarps * W) {
+        const int np = (int)min((int64_t)W, a.c.n - q0);
+        const int32_t *nb = D.nbr + q0 * k;
+        if (lane < np) {
+            const int64_t q = q0 + lane;
+            const float4 di = D.derf[q];
+            MixedRow &R = sm.row[lane];
+            R.rec = B.rec[q];
+            R.vrec = B.vrec[q];
+            R.c = di.x; R.rho = di.y; R.h = di.z; R.cterm = di.w;
+            R.inv_h = 1.f / di.z;
+            R.sim = sim_of(a.c, q);
+        }
+        __syncwarp();
+        KahanF ax, ay, ed;
+        for (int c = 0, e_lo = k; c < ch.n; c++) {
+            const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
+            e_lo -= ce;
+            for (int i = lane; i < npair; i += 32) {
+                const int p = pair_row(i, magic), at = p * k + e_lo + (i - p * ce), slot = i + p * (st - ce);
+                const MixedRow &R = sm.row[p];
+                const SimDev &S = a.c.sims[R.sim];
+                const uint32_t code = (uint32_t)nb[at], j = code >> kCodeShift;
+                const float4 rj = __ldg(&B.rec[j]), vj = __ldg(&B.vrec[j]), dj = __ldg(&D.derf[j]);
+                const float4 vi = R.vrec;
+                float rabx, raby;  // r_AB = (q - offset) - p from float pairs
+                float_pair_rel(S, R.rec, rj, code & 15u, rabx, raby);
+                const float d2 = __fmaf_rn(rabx, rabx, raby * raby);
+                const float invd = rsqrtf(d2);
+                const float qq = fminf(d2 * invd * R.inv_h, 1.f);
+                const float drk = kdf_f32(S.kernel, qq);
+                const float vabx = (vj.x - vi.x) + (vj.z - vi.z);
+                const float vaby = (vj.y - vi.y) + (vj.w - vi.w);
+                const float dot = vabx * rabx + vaby * raby;
+                float piab = 0.f;
+                if (dot < 0.f) {
+                    const float cab = 0.5f * (R.c + dj.x);
+                    const float rhoab = 0.5f * (R.rho + dj.y);
+                    const float hab = 0.5f * (R.h + dj.z);
+                    // two-instruction quotients (<= 2 ulp; both denominators are
+                    // normal: d2 + eta^2 >= eta^2, rho_AB > 0)
+                    const float mu = __fdividef(dot * hab, d2 + S.fetasq);
+                    piab = __fdividef(mu * (S.fbeta * mu - S.falpha * cab), rhoab);
+                }
+                sm.rx[slot] = rabx;
+                sm.ry[slot] = raby;
+                sm.w[slot] = (piab + R.cterm + dj.w) * drk * invd;
+                sm.dot[slot] = dot;
+                sm.drk[slot] = drk;
+            }
+            __syncwarp();
+            if (lane < np) {
+                for (int e = ce - 1; e >= 0; e--) {
+                    const int t = lane * st + e;
+                    const float wt = sm.w[t];
+                    kahan_fma(ax, sm.rx[t], wt);
+                    kahan_fma(ay, sm.ry[t], wt);
+                    kahan_fma(ed, sm.dot[t], sm.drk[t]);
+                }
+            }
+            __syncwarp();
+        }
+        if (lane < np) {
+            const int64_t q = q0 + lane;
+            const MixedRow &R = sm.row[lane];
+            const SimDev &S = a.c.sims[R.sim];
+            const float inv_hf = R.inv_h;
+            const float ff = S.fdfm * (inv_hf * inv_hf * inv_hf);
+            const double axo = (double)(ax.value_f() * ff) + S.accel[0];
+            const double ayo = (double)(ay.value_f() * ff) + S.accel[1];
+            const double edot = (double)(R.cterm * ed.value_f() * S.fmass);
+            if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
+            double2 pos = B.pos[q], vel = B.vel[q];
+            double u = B.u[q];
+            if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
+            a.A.pos[q] = pos;
+            a.A.vel[q] = vel;
+            a.A.u[q] = u;
+            a.A.acc[q] = make_double2(axo, ayo);
+            a.A.udot[q] = edot;
+            a.A.id[q] = B.id[q];
+            a.A.hprev[q] = R.h;  // the smoothing length rounded to FP32
+            a.A.vp[q] = B.vp[q];
+            a.A.up[q] = B.up[q];
+        }
+        __syncwarp();
     }
     if (fl) atomicOr(a.c.flags, fl);
 }
@@ -447,10 +577,15 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
         k_force_fp64<<<grid, kPairWarps * 32, kForceSmem, L.stream>>>(a, W);
         return;
     }
-    const int block = 128;
-    const int64_t need = (c.n + block - 1) / block;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)L.sms * 16));
-    k_force<MODE_MIXED><<<grid, block, 0, L.stream>>>(a);
+    if (c.n <= kMixedPairsMaxN) {
+        const int W = pair_width(c.n, (int64_t)L.sms * kMixedBlocks * kPairWarps);
+        const int64_t tiles = (c.n + W - 1) / W;
+        const int grid = (int)std::max<int64_t>(1, (tiles + kPairWarps - 1) / kPairWarps);
+        k_force_mixed_pairs<<<grid, kPairWarps * 32, 0, L.stream>>>(a, W);
+        return;
+    }
+    const int64_t need = (c.n + 127) / 128;
+    k_force_mixed<<<(int)std::min<int64_t>(need, (int64_t)L.sms * 16), 128, 0, L.stream>>>(a);
 }
 
 // ------------------------------------------------------------ error norms

@@ -72,3 +72,24 @@ def test_operands_left_to_the_hardware(gpu, oracle, n):
         conf.ViscosityAlpha, conf.ViscosityBeta = alpha, beta
         check(oracle, conf, (x, y, vx, vy, u))
     check(oracle, ics.periodic_config(n, 32, 1e-4), (x, y, vx, vy, np.where(r.random(n) < 0.5, 0.0, u)))  # c = 0
+
+
+@pytest.mark.parametrize("n,k,kernel", [(333, 32, "Monahan"), (3001, 21, "Wendtland"), (16384, 32, "Monahan"), (2500, 9, "Monahan"),
+                                        (5000, 65, "Monahan"), (1200, 128, "Monahan")])
+def test_mixed_force_same_bits_pair_by_pair(gpu, n, k, kernel):
+    """The mixed force deals its pairs over the lanes up to 16,384 particles
+    and runs one thread per particle beyond: a simulation alone, and as a member
+    of a larger ensemble, gives the same bits (per-query search in both, whose
+    list order does not depend on the other members)."""
+    conf, big = ics.periodic_config(n, k, 1e-4, "Mixed"), ics.periodic_config(20_000, k, 1e-4, "Mixed")
+    conf.Kernel = kernel
+    arrs = flow(n, 21)
+    one, many = S.Simulation(conf, *arrs), S.Ensemble([big, conf], [flow(20_000, 22), arrs])
+    for s in (one, many):
+        s.SetSearch(False)
+        s.Step(3)
+    a, b, da, db = one.state(), many.state(), one.derived(), many.derived()
+    for key in a:
+        assert np.array_equal(a[key], b[key][20_000:]), key
+    for key in da:
+        assert np.array_equal(da[key], db[key][20_000:]), key
