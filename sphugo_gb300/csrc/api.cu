@@ -4,7 +4,7 @@
 // A handle mirrors the reference's Simulation (sim/sph.go:14-21): its mutex
 // plays the role of Simulation.IsBusy, it owns the particle state (kept
 // resident in HBM) and counts steps. Each force evaluation is the kernel
-// chain prep -> [bbox -> grid] -> bin -> scan -> permute -> knn -> force,
+// chain [bbox] -> bin -> scan -> permute -> knn -> density -> force,
 // captured once into a CUDA graph per integration mode and replayed.
 #include <algorithm>
 #include <cfloat>
@@ -174,7 +174,7 @@ int alloc_parrays(sph_handle *h, PArrays &P, bool mixed, int64_t n) {
     rc |= dalloc(h, &P.id, n);
     rc |= dalloc(h, &P.hprev, n);
     rc |= dalloc(h, &P.rec, n);
-    rc |= dalloc(h, &P.vrec, n);  // predicted velocities as float pairs (mixed sums, FP64 force's sign test)
+    if (mixed) rc |= dalloc(h, &P.vrec, n);  // predicted velocities as float pairs
     return rc ? SPH_ERR_NOMEM : SPH_OK;
 }
 
@@ -273,7 +273,7 @@ SimDev make_simdev(const sph_params &p, int64_t off, int64_t n, int64_t cell_off
     S.etasq = p.etasq;
     S.fpref = p.kernel == SPH_KERNEL_WENDLAND ? kWendFPref : kMonahanPref;
     S.dfpref = p.kernel == SPH_KERNEL_WENDLAND ? kWendDFPref : kMonahanPref;
-    S.overshoot = 0.f;
+    reset_reductions(S);
     S.tol = (float)(std::max(S.L[0], S.L[1]) * 4.0e-7);
     simdev_floats(S);
     return S;
@@ -297,17 +297,12 @@ void enqueue_eval(sph_handle *h, int pred, bool integrate, bool events = false) 
         if (events) cudaEventRecordWithFlags(h->ev[i], h->stream, cudaEventRecordExternal);
     };
     mark(0);
-    launch_prep(c, L, h->any_open);
-    if (h->any_open) {
-        launch_bbox(c, L, h->A, pred);
-        launch_grid(c, L);
-    }
+    if (h->any_open) launch_bbox(c, L, h->A, pred);
     launch_bin(c, L, h->A, h->T, pred);
     mark(1);
     launch_scan(c, L, h->T);
-    launch_stable(c, L, h->T);
     mark(2);
-    launch_permute(c, L, h->A, h->B, h->T, pred, true);  // velocity records: every form's force reads them
+    launch_permute(c, L, h->A, h->B, h->T, pred, h->mode == MODE_MIXED);  // velocity records: the mixed force reads them
     mark(3);
     const int mode = kernel_mode(h->mode);
     launch_knn(c, L, h->B, h->D, h->T, mode, h->tune);
@@ -435,7 +430,7 @@ int create_impl(const sph_params *params, const int64_t *counts, int32_t nsims, 
     rc |= dalloc(h, &h->d_sims, nsims);
     rc |= dalloc(h, &h->d_offs, nsims + 1);
     if (nsims > 1) rc |= dalloc(h, &h->d_simidx, total);
-    rc |= dalloc(h, &h->d_flags, 1);
+    rc |= dalloc(h, &h->d_flags, 2);
     if (rc) return bail(SPH_ERR_NOMEM);
     if (alloc_particles(h, n)) return bail(SPH_ERR_NOMEM);
     rc |= dalloc(h, &h->D.ndefer, 2);
@@ -448,7 +443,7 @@ int create_impl(const sph_params *params, const int64_t *counts, int32_t nsims, 
         cudaMemset(h->D.nbr, 0, n * k * sizeof(int32_t)) != cudaSuccess ||
         cudaMemset(h->B.id, 0, n * sizeof(int32_t)) != cudaSuccess ||
         cudaMemset(h->A.id, 0, n * sizeof(int32_t)) != cudaSuccess ||
-        cudaMemset(h->d_flags, 0, sizeof(unsigned)) != cudaSuccess ||
+        cudaMemset(h->d_flags, 0, 2 * sizeof(unsigned)) != cudaSuccess ||
         cudaMemset(h->A.hprev, 0, n * sizeof(float)) != cudaSuccess ||
         cudaMemcpy(h->d_sims, h->hsims.data(), nsims * sizeof(SimDev), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(h->d_offs, h->offs.data(), (nsims + 1) * sizeof(int64_t), cudaMemcpyHostToDevice) != cudaSuccess)

@@ -100,7 +100,7 @@ struct Derived {
 };
 
 struct Tables {
-    int32_t *key, *rank;   // per particle (rank becomes the destination slot)
+    int32_t *key, *rank;   // per particle: cell, and arrival order inside it
     int32_t *tmp;          // per particle: source indices grouped by cell
     int32_t *count;        // per cell (zero between binnings)
     int32_t *start;        // per cell + 1
@@ -116,7 +116,7 @@ struct Ctx {
     int nsims;
     int64_t n;
     int k;
-    unsigned *flags;
+    unsigned *flags;       // error word; flags[1]: tickets of k_bbox (zero between launches)
 };
 
 // ---------------------------------------------------------------- helpers
@@ -207,20 +207,30 @@ __device__ __forceinline__ void predict(const SimDev &S, int mode, double2 pos, 
     }
 }
 
+// The per-binning reductions of a simulation, as the next binning expects them.
+__host__ __device__ inline void reset_reductions(SimDev &S) {
+    S.overshoot = 0.f;
+    S.bbox[0] = S.bbox[2] = ~0ull;
+    S.bbox[1] = S.bbox[3] = 0ull;
+}
+
+// By the density kernels: the search is the last to read the reductions.
+__device__ __forceinline__ void reset_for_next_binning(const Ctx &c) {
+    if (blockIdx.x == 0)
+        for (int s = threadIdx.x; s < c.nsims; s += blockDim.x) reset_reductions(c.sims_rw[s]);
+}
+
 // ------------------------------------------------------------- launchers
 struct Launch {
     int sms;
     cudaStream_t stream;
 };
 
-void launch_prep(const Ctx &c, const Launch &L, bool any_open);
-void launch_bbox(const Ctx &c, const Launch &L, const PArrays &A, int pred);
-void launch_grid(const Ctx &c, const Launch &L);
+void launch_bbox(const Ctx &c, const Launch &L, const PArrays &A, int pred);  // and the grids of open axes
 void launch_bin(const Ctx &c, const Launch &L, const PArrays &A, const Tables &T, int pred);
 void launch_scan(const Ctx &c, const Launch &L, const Tables &T);
-void launch_stable(const Ctx &c, const Launch &L, const Tables &T);
 void launch_permute(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
-                    const Tables &T, int pred, bool mixed);
+                    const Tables &T, int pred, bool velrec);
 
 struct KnnTune {
     int block;      // threads per block

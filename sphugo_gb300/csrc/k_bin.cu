@@ -6,25 +6,23 @@
 // particle's rank inside its cell), an exclusive scan of the histogram into
 // cell starts, and a permute of the state into cell order. Every coarser
 // level's cell is a contiguous range of the same table, which is what the
-// neighbour search walks. All four passes are HBM streams.
+// neighbour search walks. With many particles the passes are HBM streams; with
+// few, each is a launch of about 2 us, so they are few: keys, scan (with the
+// grouping by cell while one block can do both), permute.
 #include "common.cuh"
+
+#include <algorithm>
 
 namespace sphgpu {
 
-// ------------------------------------------------------------------ prep
-// Per-simulation reset of the per-binning reductions (one thread per sim).
-__global__ void k_prep(Ctx c) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= c.nsims) return;
-    SimDev &S = c.sims_rw[s];
-    S.overshoot = 0.f;
-    S.bbox[0] = ~0ull; S.bbox[1] = 0ull;
-    S.bbox[2] = ~0ull; S.bbox[3] = 0ull;
-}
-
-void launch_prep(const Ctx &c, const Launch &L, bool) {
-    k_prep<<<(c.nsims + 127) / 128, 128, 0, L.stream>>>(c);
-}
+// Blocks for a pass over n particles: small ones for few particles, so that
+// they spread over the SMs.
+struct Pass {
+    int grid, block;
+    Pass(const Launch &L, int64_t n) : block(n <= 32768 ? 64 : 256) {
+        grid = (int)std::min<int64_t>((n + block - 1) / block, (int64_t)L.sms * 8);
+    }
+};
 
 // ------------------------------------------------------------------ bbox
 // Bounding box of the predicted positions, for simulations with an open axis,
@@ -62,14 +60,47 @@ struct BoxKeys {
     }
 };
 
+// Grid of open axes from the bounding box.
+__device__ void grid_one(SimDev &S) {
+    const int G = 1 << S.level;
+    for (int ax = 0; ax < 2; ax++) {
+        if (S.periodic[ax]) continue;
+        double mn = dkey_inv(__ldcg(&S.bbox[2 * ax])), mx = dkey_inv(__ldcg(&S.bbox[2 * ax + 1]));
+        if (!(mn <= mx)) { mn = 0; mx = 1; }
+        double w = mx - mn;
+        if (!(w > 0)) w = 1e-300 + fabs(mn) * 1e-12 + 1e-12;
+        double L = w * (1.0 + 1e-9) + 1e-300;
+        S.lo[ax] = mn;
+        S.L[ax] = L;
+        S.s[ax] = L / G;
+        S.inv_s[ax] = G / L;
+    }
+    double Lm = fmax(S.L[0], S.L[1]);
+    S.tol = (float)(Lm * 4.0e-7);
+    simdev_floats(S);
+}
+
+// The last block to finish turns the boxes into grids; it takes the ticket back
+// to zero for the next launch.
+__device__ __forceinline__ void last_block_grids(const Ctx &c) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(c.flags + 1, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int s = threadIdx.x; s < c.nsims; s += blockDim.x) grid_one(c.sims_rw[s]);
+    if (threadIdx.x == 0) c.flags[1] = 0u;
+}
+
 __global__ void __launch_bounds__(256) k_bbox(Ctx c, PArrays A, int pred) {
     __shared__ BoxKeys part[8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t per = (c.n + gridDim.x - 1) / gridDim.x;
-    const int64_t i0 = blockIdx.x * per, i1 = min(c.n, i0 + per);
-    if (i0 >= i1) return;
-    const int s0 = sim_of(c, i0);
-    const bool one = s0 == sim_of(c, i1 - 1);  // slots are ordered by simulation
+    const int64_t i0 = min(c.n, blockIdx.x * per), i1 = min(c.n, i0 + per);
+    const int s0 = sim_of(c, min(i0, c.n - 1));
+    const bool one = i0 >= i1 || s0 == sim_of(c, i1 - 1);  // slots are ordered by simulation
     BoxKeys b;
     b.clear();
     for (int64_t base = i0; base < i1; base += blockDim.x) {
@@ -98,47 +129,21 @@ __global__ void __launch_bounds__(256) k_bbox(Ctx c, PArrays A, int pred) {
             }
         }
     }
-    if (!one) return;
-    b.reduce_warp();
-    if (lane == 0) part[w] = b;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int j = 1; j < (int)(blockDim.x >> 5); j++)
-            for (int i = 0; i < 4; i++) b.k[i] = i & 1 ? key_max(b.k[i], part[j].k[i]) : key_min(b.k[i], part[j].k[i]);
-        b.flush(c.sims[s0], c.sims_rw[s0]);
+    if (one) {
+        b.reduce_warp();
+        if (lane == 0) part[w] = b;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int j = 1; j < (int)(blockDim.x >> 5); j++)
+                for (int i = 0; i < 4; i++) b.k[i] = i & 1 ? key_max(b.k[i], part[j].k[i]) : key_min(b.k[i], part[j].k[i]);
+            b.flush(c.sims[s0], c.sims_rw[s0]);
+        }
     }
+    last_block_grids(c);
 }
 
 void launch_bbox(const Ctx &c, const Launch &L, const PArrays &A, int pred) {
-    const int64_t need = (c.n + 255) / 256;
-    k_bbox<<<(int)(need < (int64_t)L.sms * 4 ? need : (int64_t)L.sms * 4), 256, 0, L.stream>>>(c, A, pred);
-}
-
-// Grid of open axes from the bounding box (one thread per sim).
-__global__ void k_grid(Ctx c) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= c.nsims) return;
-    SimDev &S = c.sims_rw[s];
-    int G = 1 << S.level;
-    for (int ax = 0; ax < 2; ax++) {
-        if (S.periodic[ax]) continue;
-        double mn = dkey_inv(S.bbox[2 * ax]), mx = dkey_inv(S.bbox[2 * ax + 1]);
-        if (!(mn <= mx)) { mn = 0; mx = 1; }
-        double w = mx - mn;
-        if (!(w > 0)) w = 1e-300 + fabs(mn) * 1e-12 + 1e-12;
-        double L = w * (1.0 + 1e-9) + 1e-300;
-        S.lo[ax] = mn;
-        S.L[ax] = L;
-        S.s[ax] = L / G;
-        S.inv_s[ax] = G / L;
-    }
-    double Lm = fmax(S.L[0], S.L[1]);
-    S.tol = (float)(Lm * 4.0e-7);
-    simdev_floats(S);
-}
-
-void launch_grid(const Ctx &c, const Launch &L) {
-    k_grid<<<(c.nsims + 127) / 128, 128, 0, L.stream>>>(c);
+    k_bbox<<<(int)std::min<int64_t>((c.n + 255) / 256, (int64_t)L.sms * 4), 256, 0, L.stream>>>(c, A, pred);
 }
 
 // ------------------------------------------------------------------- bin
@@ -179,17 +184,45 @@ __global__ void k_bin(Ctx c, PArrays A, Tables T, int pred) {
 }
 
 void launch_bin(const Ctx &c, const Launch &L, const PArrays &A, const Tables &T, int pred) {
-    k_bin<<<L.sms * 8, 256, 0, L.stream>>>(c, A, T, pred);
+    const Pass p(L, c.n);
+    k_bin<<<p.grid, p.block, 0, L.stream>>>(c, A, T, pred);
+}
+
+// ---------------------------------------------------------- stable order
+// The histogram's atomic ranks order a cell's particles arbitrarily. To make
+// every later order (and so every floating-point sum) reproducible, each
+// particle's slot inside its cell is its rank by index in the previous order
+// among the cell's members: the members are grouped by cell (which also zeroes
+// the touched counts for the next binning), then every particle counts the
+// members of its cell with a smaller index (in the permute). Both are per
+// particle, so their cost does not grow with the cell table (the k = 64 stress
+// workload bins into 4^14 mostly empty cells).
+__device__ __forceinline__ void group_one(const Tables &T, int64_t i) {
+    const int32_t key = T.key[i];
+    T.tmp[T.start[key] + T.rank[i]] = (int32_t)i;
+    T.count[key] = 0;
+}
+
+__global__ void k_group(Ctx c, Tables T) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < c.n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        group_one(T, i);
 }
 
 // ------------------------------------------------------------------ scan
-// Exclusive scan of the cell counts into cell starts (three passes over
-// tiles of kScanTile cells). The counts are zeroed per particle afterwards
-// (k_group), so the passes over the whole cell table only read counts and
+// Exclusive scan of the cell counts into cell starts, over tiles of kScanTile
+// cells: one block for small tables; tile sums and then starts while a block
+// can add up the sums before its own (a few KB from L2); with a pass over the
+// sums between for the largest. The counts are zeroed per particle afterwards
+// (grouping), so the passes over the whole cell table only read counts and
 // write starts.
 constexpr int kScanThreads = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int64_t kScanOneBlockCells = 16384;  // (scan stage at 65,536 cells: 38 us against 12)
+constexpr int kScanDirectTiles = 4096;
+constexpr int64_t kGroupOneBlockN = 4096;  // (16,000 particles: step 97 us against 94 with a launch of its own)
+constexpr int64_t kRankPassN = 524288;  // beyond, the ranks are a pass of their own (step at 200,001: 707 us with, 704 without)
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int *warp_sums, int &total) {
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -264,16 +297,27 @@ __global__ void k_scan_partials(Tables T, int ntiles) {
     if (threadIdx.x == 0) T.start[T.ncells] = carry;
 }
 
+// DIRECT: partial holds the tiles' own sums; else their exclusive scan
+template <bool DIRECT>
 __global__ void k_scan_final(Tables T) {
     __shared__ int ws[32];
     int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int v[kScanItems];
     load_counts(T, base, v);
+    int before = 0;
+    if (DIRECT) {
+        int mine = 0;
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += kScanThreads) mine += T.partial[b];
+        block_exclusive_scan(mine, ws, before);
+    } else {
+        before = T.partial[blockIdx.x];
+    }
     int sum = 0;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) sum += v[j];
     int total;
-    int ex = block_exclusive_scan(sum, ws, total) + T.partial[blockIdx.x];
+    int ex = block_exclusive_scan(sum, ws, total) + before;
+    if (DIRECT && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) T.start[T.ncells] = before + total;
     int st[kScanItems];
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
@@ -290,58 +334,88 @@ __global__ void k_scan_final(Tables T) {
     }
 }
 
-void launch_scan(const Ctx &, const Launch &L, const Tables &T) {
-    int ntiles = (int)((T.ncells + kScanTile - 1) / kScanTile);
-    k_scan_tiles<<<ntiles, kScanThreads, 0, L.stream>>>(T);
-    k_scan_partials<<<1, 1024, 0, L.stream>>>(T, ntiles);
-    k_scan_final<<<ntiles, kScanThreads, 0, L.stream>>>(T);
+// A table of at most kScanOneBlockCells cells by one block, and with it (group)
+// the particles' grouping by cell.
+__global__ void __launch_bounds__(1024) k_scan_one(Ctx c, Tables T, int group) {
+    __shared__ int ws[32];
+    const int nc = (int)T.ncells, per = ((nc + 1023) / 1024 + 3) & ~3;  // whole 16-byte words of counts
+    const int x0 = min((int)threadIdx.x * per, nc), x1 = min(x0 + per, nc);
+    int sum = 0;
+    if ((nc & 3) == 0) {
+        for (int x = x0; x < x1; x += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(T.count + x);
+            sum += v.x + v.y + v.z + v.w;
+        }
+    } else {
+        for (int x = x0; x < x1; x++) sum += T.count[x];
+    }
+    int total;
+    int run = block_exclusive_scan(sum, ws, total);
+    if (threadIdx.x == 0) T.start[nc] = total;
+    if ((nc & 3) == 0) {
+        for (int x = x0; x < x1; x += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(T.count + x);
+            *reinterpret_cast<int4 *>(T.start + x) = make_int4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+            run += v.x + v.y + v.z + v.w;
+        }
+    } else {
+        for (int x = x0; x < x1; x++) {
+            T.start[x] = run;
+            run += T.count[x];
+        }
+    }
+    if (!group) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < (int)c.n; i += 1024) group_one(T, i);
 }
 
-// ---------------------------------------------------------- stable order
-// The histogram's atomic ranks order a cell's particles arbitrarily. To make
-// every later order (and so every floating-point sum) reproducible, each
-// particle's slot inside its cell is its rank by index in the previous order
-// among the cell's members: the members are grouped by cell (k_group, which
-// also zeroes the touched counts for the next binning), then every particle
-// counts the members of its cell with a smaller index (k_rank). Both passes
-// are per particle, so their cost does not grow with the cell table (the
-// k = 64 stress workload bins into 4^14 mostly empty cells).
-__global__ void k_group(Ctx c, Tables T) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < c.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t key = T.key[i];
-        T.tmp[T.start[key] + T.rank[i]] = (int32_t)i;
-        T.count[key] = 0;
-    }
+// A particle's slot: the cell's first plus the members with a smaller index.
+__device__ __forceinline__ int slot_of(const Tables &T, int64_t i) {
+    const int32_t key = T.key[i];
+    const int x0 = T.start[key], x1 = T.start[key + 1];
+    int d = x0;
+    for (int x = x0; x < x1; x++) d += T.tmp[x] < (int32_t)i ? 1 : 0;
+    return d;
 }
 
 __global__ void k_rank(Ctx c, Tables T) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < c.n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t key = T.key[i];
-        const int a = T.start[key], b = T.start[key + 1];
-        int r = a;
-        for (int x = a; x < b; x++) r += T.tmp[x] < (int32_t)i ? 1 : 0;
-        T.rank[i] = r;
-    }
+         i += (int64_t)gridDim.x * blockDim.x)
+        T.rank[i] = slot_of(T, i);
 }
 
-void launch_stable(const Ctx &c, const Launch &L, const Tables &T) {
-    k_group<<<L.sms * 8, 256, 0, L.stream>>>(c, T);
-    k_rank<<<L.sms * 8, 256, 0, L.stream>>>(c, T);
+// starts, the particles grouped by cell, and (many particles) their slots
+void launch_scan(const Ctx &c, const Launch &L, const Tables &T) {
+    const bool one = T.ncells <= kScanOneBlockCells, group = one && c.n <= kGroupOneBlockN;
+    if (one) {
+        k_scan_one<<<1, 1024, 0, L.stream>>>(c, T, group ? 1 : 0);
+    } else {
+        const int ntiles = (int)((T.ncells + kScanTile - 1) / kScanTile);
+        k_scan_tiles<<<ntiles, kScanThreads, 0, L.stream>>>(T);
+        if (ntiles <= kScanDirectTiles) {
+            k_scan_final<true><<<ntiles, kScanThreads, 0, L.stream>>>(T);
+        } else {
+            k_scan_partials<<<1, 1024, 0, L.stream>>>(T, ntiles);
+            k_scan_final<false><<<ntiles, kScanThreads, 0, L.stream>>>(T);
+        }
+    }
+    const Pass p(L, c.n);
+    if (!group) k_group<<<p.grid, p.block, 0, L.stream>>>(c, T);
+    if (c.n > kRankPassN) k_rank<<<p.grid, p.block, 0, L.stream>>>(c, T);
 }
 
 // --------------------------------------------------------------- permute
 // Writes the predicted state into cell order (B), plus the float-pair
 // position record relative to the grid origin used by the FP32 distance
-// filter and the mixed-precision sums, and (vel_records) the predicted
+// filter and the mixed-precision sums, and (velrec) the predicted
 // velocity as float pairs.
-__global__ void k_permute(Ctx c, PArrays A, PArrays B, Tables T, int pred, int mixed) {
+template <bool RANKED>
+__global__ void k_permute(Ctx c, PArrays A, PArrays B, Tables T, int pred, int velrec) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < c.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         int s = sim_of(c, i);
         const SimDev &S = c.sims[s];
-        const int64_t d = T.rank[i];  // destination slot (stable within the cell)
+        const int64_t d = RANKED ? T.rank[i] : slot_of(T, i);
         double2 pos = A.pos[i], vel = A.vel[i];
         double u = A.u[i];
         double2 p, vp;
@@ -358,7 +432,7 @@ __global__ void k_permute(Ctx c, PArrays A, PArrays B, Tables T, int pred, int m
         split_df(__dsub_rn(p.x, S.lo[0]), r.x, r.z);
         split_df(__dsub_rn(p.y, S.lo[1]), r.y, r.w);
         B.rec[d] = r;
-        if (mixed) {
+        if (velrec) {
             float4 v;
             split_df(vp.x, v.x, v.z);
             split_df(vp.y, v.y, v.w);
@@ -368,8 +442,12 @@ __global__ void k_permute(Ctx c, PArrays A, PArrays B, Tables T, int pred, int m
 }
 
 void launch_permute(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
-                    const Tables &T, int pred, bool mixed) {
-    k_permute<<<L.sms * 8, 256, 0, L.stream>>>(c, A, B, T, pred, mixed ? 1 : 0);
+                    const Tables &T, int pred, bool velrec) {
+    const Pass p(L, c.n);
+    // the ranks' loads in front of the drift cost more than a launch once the
+    // arrays outgrow L2 (clustered N = 4,194,304: 165 us against 130 + 21)
+    if (c.n > kRankPassN) k_permute<true><<<p.grid, p.block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
+    else k_permute<false><<<p.grid, p.block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
 }
 
 }  // namespace sphgpu

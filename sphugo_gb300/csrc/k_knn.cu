@@ -941,6 +941,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, (MODE == MODE_MIXED || NR > 2
 // particle: all of them, or (use_defer) only the queries the block tiles left
 // to the per-query search, since the tiles computed the others' densities.
 __global__ void __launch_bounds__(256, 4) k_density_mixed(KnnArgs a) {
+    reset_for_next_binning(a.c);
     const int k = a.c.k;
     const PArrays &B = a.B;
     unsigned fl = 0;

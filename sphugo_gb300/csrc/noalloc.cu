@@ -36,7 +36,7 @@ constexpr size_t kScratchBytes =
     3 * align256(8 * kN) + align256(32 * kN) + align256(4 * kNK) + align256(16 * kNK) +  // D
     3 * align256(4 * kN) + align256(4 * kNoAllocCells) + align256(4 * (kNoAllocCells + 1)) +
     align256(4 * (kNoAllocCells / 4096 + 2)) +                               // T
-    align256(sizeof(SimDev)) + align256(2 * sizeof(int64_t)) + align256(sizeof(unsigned));
+    align256(sizeof(SimDev)) + align256(2 * sizeof(int64_t)) + align256(2 * sizeof(unsigned));
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -83,7 +83,7 @@ __global__ void k_noalloc_init(SimDev S, SimDev *sims, int64_t *offs, unsigned *
     sims[0] = S;
     offs[0] = 0;
     offs[1] = S.n;
-    flags[0] = 0u;
+    flags[0] = flags[1] = 0u;
 }
 
 const double kMonahanPref = 0x1.5d3b3e3583243p+3;  // 6*40/(pi*7), sim/sph.go:266
@@ -165,7 +165,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     T.partial = cv.take<int32_t>(kNoAllocCells / 4096 + 2);
     SimDev *d_sims = cv.take<SimDev>(1);
     int64_t *d_offs = cv.take<int64_t>(2);
-    unsigned *d_flags = cv.take<unsigned>(1);
+    unsigned *d_flags = cv.take<unsigned>(2);
     if ((size_t)(cv.p - ds.ptr) > kScratchBytes)
         return nfail(SPH_ERR_ARG, "sph_density_noalloc: internal scratch layout exceeds the static array");
 
@@ -196,6 +196,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     S.etasq = p->etasq;
     S.fpref = p->kernel == SPH_KERNEL_WENDLAND ? kWendFPref : kMonahanPref;
     S.dfpref = p->kernel == SPH_KERNEL_WENDLAND ? kWendDFPref : kMonahanPref;
+    reset_reductions(S);
     S.tol = (float)(std::max(S.L[0], S.L[1]) * 4.0e-7);
     simdev_floats(S);
     T.ncells = (int64_t)1 << (2 * S.level);
@@ -218,14 +219,9 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
         return nfail(SPH_ERR_CUDA, "sph_density_noalloc: clearing the cell table failed");
     k_noalloc_init<<<1, 1, 0, st>>>(S, d_sims, d_offs, d_flags);
     launch_scatter_state(c, L, A, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false);
-    launch_prep(c, L, any_open);
-    if (any_open) {
-        launch_bbox(c, L, A, PRED_INIT);
-        launch_grid(c, L);
-    }
+    if (any_open) launch_bbox(c, L, A, PRED_INIT);
     launch_bin(c, L, A, T, PRED_INIT);
     launch_scan(c, L, T);
-    launch_stable(c, L, T);
     launch_permute(c, L, A, B, T, PRED_INIT, false);
     launch_knn(c, L, B, D, T, MODE_EXACT64, tune);
     launch_density(c, L, B, D, MODE_EXACT64, nullptr);
