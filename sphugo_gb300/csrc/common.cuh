@@ -256,13 +256,14 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
 void launch_error_norms(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, double *anorm,
                         double *unorm);
 
-void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, double *x, double *y,
+void launch_slots(const Ctx &c, const Launch &L, const PArrays &A, int32_t *slot);
+void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, double *x, double *y,
                          double *vx, double *vy, double *u, double *ax, double *ay, double *udot);
-void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const double *x,
+void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, const double *x,
                           const double *y, const double *vx, const double *vy, const double *u,
-                          const double *ax, const double *ay, const double *udot, bool have_acc);
+                          const double *ax, const double *ay, const double *udot);
 void launch_append(const Launch &L, const PArrays &A, int64_t n0, int64_t count, const double *buf);
-void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D,
+void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D, const int32_t *slot,
                            double *rho, double *cs, double *h);
 void launch_gather_neighbours(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
                               const Derived &D, int64_t *ids, double *dist, int32_t *img, bool exact_stored);

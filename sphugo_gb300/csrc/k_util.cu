@@ -16,51 +16,57 @@ static int grid_for(const Launch &L, int64_t n, int block) {
     return g < 1 ? 1 : g;
 }
 
-__global__ void k_gather_state(Ctx c, PArrays A, double *x, double *y, double *vx, double *vy,
+// Slot of each caller index: the transfers below run in the caller's order, so
+// that they read and write the caller's arrays, which may be pinned host memory
+// behind the host link, in whole lines, and the device's arrays at the slots.
+__global__ void k_slots(Ctx c, PArrays A, int32_t *slot) {
+    GRID_STRIDE(i, c.n) slot[A.id[i]] = (int32_t)i;
+}
+
+void launch_slots(const Ctx &c, const Launch &L, const PArrays &A, int32_t *slot) {
+    k_slots<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot);
+}
+
+__global__ void k_gather_state(Ctx c, PArrays A, const int32_t *slot, double *x, double *y, double *vx, double *vy,
                                double *u, double *ax, double *ay, double *udot) {
-    GRID_STRIDE(i, c.n) {
-        int32_t id = A.id[i];
-        double2 p = A.pos[i], v = A.vel[i], a = A.acc[i];
-        if (x) x[id] = p.x;
-        if (y) y[id] = p.y;
-        if (vx) vx[id] = v.x;
-        if (vy) vy[id] = v.y;
-        if (u) u[id] = A.u[i];
-        if (ax) ax[id] = a.x;
-        if (ay) ay[id] = a.y;
-        if (udot) udot[id] = A.udot[i];
+    GRID_STRIDE(t, c.n) {
+        const int32_t i = slot[t];
+        const double2 p = A.pos[i], v = A.vel[i], a = A.acc[i];
+        if (x) x[t] = p.x;
+        if (y) y[t] = p.y;
+        if (vx) vx[t] = v.x;
+        if (vy) vy[t] = v.y;
+        if (u) u[t] = A.u[i];
+        if (ax) ax[t] = a.x;
+        if (ay) ay[t] = a.y;
+        if (udot) udot[t] = A.udot[i];
     }
 }
 
-void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, double *x, double *y,
+void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, double *x, double *y,
                          double *vx, double *vy, double *u, double *ax, double *ay, double *udot) {
-    k_gather_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, x, y, vx, vy, u, ax, ay, udot);
+    k_gather_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot, x, y, vx, vy, u, ax, ay, udot);
 }
 
-// have_acc = 0: fresh upload, slot i holds particle i and the integrator
-// history (accelerations, predictions, radius guess) starts from zero.
-// have_acc = 1: replace the state of every particle in its current slot.
-__global__ void k_scatter_state(Ctx c, PArrays A, const double *x, const double *y, const double *vx,
+// slot = NULL: fresh upload, slot i holds particle i and the integrator
+// history (accelerations, predictions, radius guess) starts from zero; else
+// the state of every particle in its current slot is replaced.
+__global__ void k_scatter_state(Ctx c, PArrays A, const int32_t *slot, const double *x, const double *y, const double *vx,
                                 const double *vy, const double *u, const double *ax, const double *ay,
-                                const double *udot, int have_acc) {
-    GRID_STRIDE(i, c.n) {
-        int32_t id;
-        if (have_acc) {
-            id = A.id[i];
-        } else {
-            id = (int32_t)i;
-            A.id[i] = id;
-            A.hprev[i] = 0.f;
-        }
-        double2 v = make_double2(vx ? vx[id] : 0.0, vy ? vy[id] : 0.0);
-        double e = u ? u[id] : 0.0;
-        A.pos[i] = make_double2(x[id], y[id]);
+                                const double *udot) {
+    GRID_STRIDE(t, c.n) {
+        const int32_t i = slot ? slot[t] : (int32_t)t;
+        const double2 v = make_double2(vx ? vx[t] : 0.0, vy ? vy[t] : 0.0);
+        const double e = u ? u[t] : 0.0;
+        A.pos[i] = make_double2(x[t], y[t]);
         A.vel[i] = v;
         A.u[i] = e;
-        if (have_acc) {
-            A.acc[i] = make_double2(ax ? ax[id] : 0.0, ay ? ay[id] : 0.0);
-            A.udot[i] = udot ? udot[id] : 0.0;
+        if (slot) {
+            A.acc[i] = make_double2(ax ? ax[t] : 0.0, ay ? ay[t] : 0.0);
+            A.udot[i] = udot ? udot[t] : 0.0;
         } else {
+            A.id[i] = i;
+            A.hprev[i] = 0.f;
             A.acc[i] = make_double2(0.0, 0.0);
             A.udot[i] = 0.0;
         }
@@ -92,25 +98,25 @@ void launch_append(const Launch &L, const PArrays &A, int64_t n0, int64_t count,
     k_append<<<grid_for(L, count, 256), 256, 0, L.stream>>>(A, n0, count, buf);
 }
 
-void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const double *x,
+void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, const double *x,
                           const double *y, const double *vx, const double *vy, const double *u,
-                          const double *ax, const double *ay, const double *udot, bool have_acc) {
-    k_scatter_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, x, y, vx, vy, u, ax, ay, udot,
-                                                                 have_acc ? 1 : 0);
+                          const double *ax, const double *ay, const double *udot) {
+    k_scatter_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot, x, y, vx, vy, u, ax, ay, udot);
 }
 
-__global__ void k_gather_derived(Ctx c, PArrays A, Derived D, double *rho, double *cs, double *h) {
-    GRID_STRIDE(i, c.n) {
-        int32_t id = A.id[i];
-        if (rho) rho[id] = D.rho[i];
-        if (cs) cs[id] = D.c[i];
-        if (h) h[id] = D.h[i];
+// by caller index (slot given), or in the slots' own order of A.id
+__global__ void k_gather_derived(Ctx c, PArrays A, Derived D, const int32_t *slot, double *rho, double *cs, double *h) {
+    GRID_STRIDE(t, c.n) {
+        const int64_t i = slot ? slot[t] : t, o = slot ? t : A.id[t];
+        if (rho) rho[o] = D.rho[i];
+        if (cs) cs[o] = D.c[i];
+        if (h) h[o] = D.h[i];
     }
 }
 
-void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D,
+void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D, const int32_t *slot,
                            double *rho, double *cs, double *h) {
-    k_gather_derived<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, D, rho, cs, h);
+    k_gather_derived<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, D, slot, rho, cs, h);
 }
 
 // Reference layout: slot 0 = farthest (sim/nearest-neighbour.go:139-153 keeps

@@ -218,7 +218,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     if (cudaMemsetAsync(T.count, 0, T.ncells * sizeof(int32_t), st) != cudaSuccess)
         return nfail(SPH_ERR_CUDA, "sph_density_noalloc: clearing the cell table failed");
     k_noalloc_init<<<1, 1, 0, st>>>(S, d_sims, d_offs, d_flags);
-    launch_scatter_state(c, L, A, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false);
+    launch_scatter_state(c, L, A, nullptr, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     if (any_open) launch_bbox(c, L, A, PRED_INIT);
     launch_bin(c, L, A, T, PRED_INIT);
     launch_scan(c, L, T);
@@ -226,7 +226,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     launch_knn(c, L, B, D, T, MODE_EXACT64, tune);
     launch_density(c, L, B, D, MODE_EXACT64, nullptr);
     if (nbr_ids || nbr_dist) launch_gather_neighbours(c, L, B, B, D, nbr_ids, nbr_dist, nullptr, true);
-    if (rho || hsml) launch_gather_derived(c, L, B, D, rho, nullptr, hsml);
+    if (rho || hsml) launch_gather_derived(c, L, B, D, nullptr, rho, nullptr, hsml);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return nfail(SPH_ERR_CUDA, std::string("sph_density_noalloc: ") + cudaGetErrorString(e));
     unsigned f = 0;
