@@ -116,7 +116,7 @@ struct Ctx {
     int nsims;
     int64_t n;
     int k;
-    unsigned *flags;       // error word; flags[1]: tickets of k_bbox (zero between launches)
+    unsigned *flags;       // error word; flags[1]: tickets of k_bbox and k_knn (zero between launches)
 };
 
 // ---------------------------------------------------------------- helpers
@@ -214,12 +214,6 @@ __host__ __device__ inline void reset_reductions(SimDev &S) {
     S.bbox[1] = S.bbox[3] = 0ull;
 }
 
-// By the density kernels: the search is the last to read the reductions.
-__device__ __forceinline__ void reset_for_next_binning(const Ctx &c) {
-    if (blockIdx.x == 0)
-        for (int s = threadIdx.x; s < c.nsims; s += blockDim.x) reset_reductions(c.sims_rw[s]);
-}
-
 // ------------------------------------------------------------- launchers
 struct Launch {
     int sms;
@@ -245,8 +239,8 @@ struct KnnTune {
 void knn_init_attrs();
 void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D,
                 const Tables &T, int mode, const KnnTune &tune);
-// tune: the search's shape (NULL: a search without tiles); when the block
-// tiles computed the settled queries' densities, only the deferred are done
+// tune: the search's shape (NULL: a search without tiles); only the densities
+// that the search did not compute with its lists
 void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int mode,
                     const KnnTune *tune);
 void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D);

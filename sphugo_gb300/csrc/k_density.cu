@@ -89,7 +89,6 @@ __device__ __forceinline__ void wendland(double q, PairF &r) {
 // (74 registers, no spills either) and 556 at 9
 __global__ void __launch_bounds__(kPairWarps * 32, 8) k_density_fp64(DensityArgs a) {
     __shared__ DensityWarp smem[kPairWarps];
-    reset_for_next_binning(a.c);
     const int k = a.c.k, W = a.W;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     DensityWarp &sm = smem[w];

@@ -92,7 +92,8 @@ __device__ __forceinline__ bool exact_greater(const PArrays &B, unsigned long lo
 template <int MODE, int NR>
 __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m, float R, float epsabs,
                             uint32_t *skey, uint32_t *scode, uint32_t *sord, unsigned long long *sexact,
-                            int lane, float *Rnext) {
+                            int lane, float *Rnext, uint32_t *far) {
+    float *sd2 = reinterpret_cast<float *>(sexact);  // fused density: squared distances in list order (the keys are done with)
     using LS = ListShape<NR>;
     const int k = a.c.k;
     const PArrays &B = a.B;
@@ -158,12 +159,18 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
                     const int o = pos + __popc(bal & lanemask_lt());
                     const uint32_t sl = v[r] & LS::SMASK;
                     a.D.nbr[q * k + o] = (int32_t)scode[sl];
-                    a.D.d2f[q * k + o] = __uint_as_float(skey[sl]);
+                    if (a.fuse_density) sd2[o] = __uint_as_float(skey[sl]);
+                    else a.D.d2f[q * k + o] = __uint_as_float(skey[sl]);
                 }
                 if (is_top) {
                     const uint32_t sl = v[r] & LS::SMASK;
                     a.D.nbr[q * k + k - 1] = (int32_t)scode[sl];
-                    a.D.d2f[q * k + k - 1] = __uint_as_float(skey[sl]);
+                    if (a.fuse_density) {
+                        sd2[k - 1] = __uint_as_float(skey[sl]);
+                        *far = scode[sl];
+                    } else {
+                        a.D.d2f[q * k + k - 1] = __uint_as_float(skey[sl]);
+                    }
                 }
                 pos += __popc(bal);
             }
@@ -259,10 +266,42 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
     // ---- write the sorted list (slot 0 = nearest)
     for (int e = lane; e < k; e += 32) {
         a.D.nbr[q * k + e] = (int32_t)scode[sord[e]];
-        if (MODE == MODE_MIXED) a.D.d2f[q * k + e] = __uint_as_float(skey[sord[e]]);
+        if (MODE == MODE_MIXED) {
+            if (a.fuse_density) {
+                sd2[e] = __uint_as_float(skey[sord[e]]);
+                if (e == k - 1) *far = scode[sord[e]];
+            } else {
+                a.D.d2f[q * k + e] = __uint_as_float(skey[sord[e]]);
+            }
+        }
     }
     __syncwarp();
     return 0;
+}
+
+// The density of a query whose list the warp has just written (k_density_mixed's
+// arithmetic and order), from its squared distances in shared memory: a lane
+// per term, then the ordered sum.
+__device__ __forceinline__ bool density_of_list(const KnnArgs &a, const SimDev &S, int64_t q, float *sd2, uint32_t far, int lane) {
+    const int k = a.c.k;
+    const double dk2 = nbr_d2(S, a.B, a.B.pos[q], far);
+    const double h = emu_sqrt(dk2);
+    const float hf = __double2float_rn(h);
+    const float inv_hf = 1.f / hf;
+    for (int e = lane; e < k; e += 32) sd2[e] = kf_f32(S.kernel, fminf(sqrtf(sd2[e]) * inv_hf, 1.f));
+    __syncwarp();
+    KahanF acc;
+    for (int e = k - 1; e >= 0; e--) acc.add(sd2[e]);
+    if (lane == 0) {
+        const float rhof = S.ffm * (inv_hf * inv_hf) * acc.value_f();
+        const float csf = sqrtf(S.fgg1 * __double2float_rn(a.B.up[q]));
+        const float ctf = csf * csf / (S.fgamma * rhof);
+        a.D.rho[q] = rhof;
+        a.D.c[q] = csf;
+        a.D.h[q] = h;
+        a.D.derf[q] = make_float4(csf, rhof, hf, ctf);
+    }
+    return dk2 < 0.4;
 }
 
 // Cells holding more than kHeavyCell particles are not scanned whole: they are
@@ -477,7 +516,7 @@ __global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
             }
             __syncwarp();
             float Rn;
-            if (select_write<MODE, NR>(a, S, q, m, R, epsabs, skey, scode, sord, sexact, lane, &Rn)) {
+            if (select_write<MODE, NR>(a, S, q, m, R, epsabs, skey, scode, sord, sexact, lane, &Rn, (uint32_t *)rq)) {
                 Rlo = R;
                 R = Rn;
                 continue;
@@ -489,12 +528,30 @@ __global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
             if (!(fl & FLAG_KNN_FEW)) fl |= FLAG_KNN_ATTEMPTS;
             for (int e = lane; e < k; e += 32) {
                 a.D.nbr[q * k + e] = ((int32_t)q << kCodeShift) | 4;
-                if (MODE == MODE_MIXED) a.D.d2f[q * k + e] = 0.f;
+                if (MODE == MODE_MIXED) {
+                    if (a.fuse_density) reinterpret_cast<float *>(sexact)[e] = 0.f;
+                    else a.D.d2f[q * k + e] = 0.f;
+                }
             }
+            if (lane == 0) *(uint32_t *)rq = ((uint32_t)q << kCodeShift) | 4u;
+        }
+        if (MODE == MODE_MIXED && a.fuse_density) {
+            __syncwarp();
+            if (!density_of_list(a, S, q, reinterpret_cast<float *>(sexact), *(uint32_t *)rq, lane)) fl |= FLAG_SENTINEL;
         }
         __syncwarp();
     }
     if (fl && lane == 0) atomicOr(a.c.flags, fl);
+    // The last kernel to read the binning's reductions: its last block resets
+    // them for the next binning (and the ticket).
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.c.flags + 1, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {
+        for (int s = threadIdx.x; s < a.c.nsims; s += blockDim.x) reset_reductions(a.c.sims_rw[s]);
+        if (threadIdx.x == 0) a.c.flags[1] = 0u;
+    }
 }
 
 // ---------------------------------------------------------------- group tiles
@@ -939,9 +996,8 @@ __global__ void __launch_bounds__(kTileWarps * 32, (MODE == MODE_MIXED || NR > 2
 // ---------------------------------------------------------------- density
 // The mixed form's density (the FP64 forms': k_density.cu), one thread per
 // particle: all of them, or (use_defer) only the queries the block tiles left
-// to the per-query search, since the tiles computed the others' densities.
+// to the per-query search, where the tiles computed the others' densities.
 __global__ void __launch_bounds__(256, 4) k_density_mixed(KnnArgs a) {
-    reset_for_next_binning(a.c);
     const int k = a.c.k;
     const PArrays &B = a.B;
     unsigned fl = 0;
@@ -1143,6 +1199,13 @@ static void launch_rerank(const KnnArgs &a, const Launch &L) {
     else k_rerank<4><<<grid, 256, 0, L.stream>>>(a);
 }
 
+// Particles up to which the per-query search computes the densities of the
+// queries the mixed form's block tiles deferred: a warp per query adds its terms
+// with all lanes waiting on one chain, which costs less than a launch while the
+// queries are few (step at N = 10,000 65 -> 59 us, 100,000 98 -> 92; kNN and
+// density at N = 1,048,576 311 us both ways, clustered 4,194,304 1215 -> 1245).
+constexpr int64_t kKnnDensityMaxN = 524288;
+
 bool knn_fuses_density(int k, int mode, const KnnTune &tune) {
     const int nr = list_regs(k);
     return mode == MODE_MIXED && tune.tile && tune.block_warps > 0 && nr <= 4 &&
@@ -1170,6 +1233,7 @@ static void launch_knn_nr(const KnnArgs &args, const Launch &L, const KnnTune &t
         }
         KnnArgs d = args;
         d.use_defer = 1;
+        if (args.c.n > kKnnDensityMaxN) d.fuse_density = 0;
         k_knn<MODE, NR><<<std::max(resident, 1), kKnnBlock, smem, L.stream>>>(d);
         return;
     }
@@ -1208,11 +1272,13 @@ void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Deriv
         launch_density_fp64(c, L, B, D);
         return;
     }
+    const bool tiles = tune && D.defer && knn_fuses_density(c.k, mode, *tune);
+    if (tiles && c.n <= kKnnDensityMaxN) return;  // computed with the lists
     KnnArgs a{};
     a.c = c;
     a.B = B;
     a.D = D;
-    a.use_defer = tune && D.defer && knn_fuses_density(c.k, mode, *tune) ? 1 : 0;
+    a.use_defer = tiles ? 1 : 0;
     const int64_t dneed = (c.n + 255) / 256;
     const int dgrid = (int)std::max<int64_t>(1, std::min<int64_t>(dneed, (int64_t)L.sms * 8));
     k_density_mixed<<<dgrid, 256, 0, L.stream>>>(a);

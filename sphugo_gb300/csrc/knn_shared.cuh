@@ -13,8 +13,8 @@ struct KnnArgs {
     Derived D;
     const int32_t *start;
     float theta, hgrow;
-    int use_defer;  // per-query kernel / density: walk the deferred list instead of every particle
-    int fuse_density;  // mixed block tiles: each settled query's density computed with its list
+    int use_defer;  // per-query kernel: walk the deferred list instead of every particle
+    int fuse_density;  // mixed form with block tiles: each query's density computed with its list
     int rerank;  // FP64 forms, block tiles: a decided set whose order needs FP64 goes to the re-rank list
 };
 
@@ -97,8 +97,8 @@ __device__ __forceinline__ void rerank_lanes(const KnnArgs &a, bool mine, int64_
 // block-tile search (k_knn_block.cu): false when no block kernel serves the
 // list shape nr (the warp tiles do then)
 bool launch_knn_block(const KnnArgs &args, const Launch &L, int mode, int nr, int warps);
-// whether the block tiles compute the mixed form's densities of the queries
-// they settle (the density pass then covers only the deferred queries)
+// whether the search computes the mixed form's densities with the lists: the
+// block tiles for the queries they settle, the per-query search for the rest
 bool knn_fuses_density(int k, int mode, const KnnTune &tune);
 void knn_block_init_attrs();
 
