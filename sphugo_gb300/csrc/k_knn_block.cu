@@ -53,6 +53,12 @@ __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
 }
 
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // d2 in units of R^2 / 2^KB (qs = 2^KB / R^2) rounded to the nearest integer,
 // clamped to KB bits: d2 qs + 2^23 lies in [2^23, 2^24), whose floats are the
 // integers, so the mantissa is the key (no conversion instruction).
@@ -102,6 +108,35 @@ struct TopGroups {
     }
 };
 
+// The P smallest of A keys, ascending in v[0..P-1] (P a power of two, A - P a
+// smaller one); the rest after them, unordered. The first P and the others
+// sorted apart (Batcher), the smaller of each pair (v[P-1-i], v[P+i]) kept, a
+// bitonic sequence, and merged: for P = 64 of 96 958 comparators, the full sort
+// 1056 and with its wider live range slower than that (FP64 kNN stage, stress
+// k = 64 1565 -> 1428 us; k = 32, 298 comparators for the 32 of 40, 294 -> 292
+// at N = 1,048,576).
+template <int A, int P>
+struct LowSort {
+    uint32_t (&v)[A];
+    __device__ __forceinline__ void ce(int i, int j) {
+        const uint32_t lo = min(v[i], v[j]);
+        v[j] = max(v[i], v[j]);
+        v[i] = lo;
+    }
+    __device__ __forceinline__ void run() {
+        OddEvenSort<A>{v}.template sort<0, P>();
+        OddEvenSort<A>{v}.template sort<P, A - P>();
+#pragma unroll
+        for (int i = 0; i < A - P; i++) ce(P - 1 - i, P + i);
+#pragma unroll
+        for (int st = P / 2; st >= 1; st >>= 1) {
+#pragma unroll
+            for (int i = 0; i < P; i++)
+                if ((i & st) == 0) ce(i, i + st);
+        }
+    }
+};
+
 template <int WARPS, int NR>
 struct BlockSmem {
     static constexpr int Q = 32 * WARPS;           // queries per tile
@@ -111,7 +146,7 @@ struct BlockSmem {
     static constexpr uint32_t SMASK = (1u << SB) - 1u;
     static constexpr int CCAP = kCellCap < TCAP ? kCellCap : TCAP;
     static constexpr int LCAP = NR == 2 ? 40 : 24 * NR;  // list entries per query (k + 3 or more)
-    float2 rec[TCAP];        // FP32 position relative to the tile origin (during the build: cell words)
+    float2 rec[TCAP + 4];    // FP32 position relative to the tile origin (during the build: cell words); the scan reads up to 3 past
     uint32_t code[TCAP];     // (particle slot << kCodeShift) | image code
     uint16_t cstart[CCAP + 8];  // first record of each cell, cells row by row
     int32_t rx0[kRowCap], rx1[kRowCap], rpre[kRowCap + 1];
@@ -122,6 +157,7 @@ struct BlockSmem {
     union alignas(16) {
         uint32_t list[WARPS][LCAP + 1][32];
         float4 staging[TCAP];
+        uint8_t row[CCAP];  // row of each cell, before the copies
     } u;
 };
 using BS82 = BlockSmem<8, 2>;
@@ -276,6 +312,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
             }
             __syncthreads();
             const int ncell = tile_ok ? sm.rpre[ny] : 0;
+            // ---- the row of every cell (a warp per row; a binary search per cell
+            // took 190 instructions of a thread's 1,360 in the build)
+            if (tile_ok)
+                for (int r = w; r < ny; r += WARPS)
+                    for (int x = sm.rpre[r] + lane; x < sm.rpre[r + 1]; x += 32) sm.u.row[x] = (uint8_t)r;
+            __syncthreads();
             // ---- cell lookups, all in flight: cell c (row-major) -> first
             // particle, population; cells of image blocks carry their image
             constexpr int CPT = (CCAP + NT - 1) / NT;
@@ -289,11 +331,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                     cntv[i] = 0;
                     imgv[i] = 4;
                     if (c < ncell) {
-                        int lo = 0, hi = ny - 1;  // the row holding cell c: the last with rpre <= c
-                        while (lo < hi) {
-                            const int mid = (lo + hi + 1) >> 1;
-                            if (sm.rpre[mid] <= c) lo = mid; else hi = mid - 1;
-                        }
+                        const int lo = sm.u.row[c];
                         const int vy = BY0 + lo;
                         const int vx = sm.rx0[lo] + (c - sm.rpre[lo]);
                         const int wx = vx >> shift, wy = vy >> shift;  // image block (floor division)
@@ -414,24 +452,50 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                 const float Sx = sx0 * pw, Sy = sy0 * pw;
                 const float Re = R + tol, Re2 = Re * Re;
                 const int lx0 = x0 >> sh, lx1 = x1 >> sh;
-                for (int vy = y0 >> sh; vy <= (y1 >> sh); vy++) {
-                    // the chord of the disc in this row of cells
-                    const float ylo = (float)vy * Sy;
-                    const float dyc = fmaxf(fmaxf(ylo - pyr, pyr - (ylo + Sy)), 0.f);
-                    if (dyc > Re) continue;
-                    const float half = sqrtf(fmaxf(Re2 - dyc * dyc, 0.f)) * 1.0000005f;
-                    const int cx0 = max(lx0, (int)floorf((pxr - half) / Sx));
-                    const int cx1 = min(lx1, (int)floorf((pxr + half) / Sx));
-                    const int rr = vy - BY0;
-                    const int base = sm.rpre[rr] - sm.rx0[rr];
-                    int t = cx0 <= cx1 ? sm.cstart[base + cx0] : 0;
-                    const int e = cx0 <= cx1 ? sm.cstart[base + cx1 + 1] : 0;
-                    // four records per round, their loads issued together (the
-                    // round's tail repeats the row's last record and never passes)
-                    for (; t < e; t += 4) {
+                // the chord's ends need not be exact, only outside: the approximate
+                // root is raised by 2^-19 of itself, and the ends moved out by
+                // 2.4e-7 of the box, more than the products with 1 / Sx round
+                const float inv_Sx = 1.f / Sx, pad = 2.4e-7f * S.flmax;
+                // four rows at a time: their record ranges (start, and end above it in
+                // the high half; 0: none), then one loop over all four, so that the
+                // warp waits for its longest lane once per group and not once per row
+                const int vend = y1 >> sh;
+                for (int vb = y0 >> sh; vb <= vend; vb += 4) {
+                    uint32_t rg[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        // the chord of the disc in this row of cells
+                        const int vy = vb + u;
+                        const float ylo = (float)vy * Sy;
+                        const float dyc = fmaxf(fmaxf(ylo - pyr, pyr - (ylo + Sy)), 0.f);
+                        const float half = __fmaf_rn(sqrt_approx(fmaxf(Re2 - dyc * dyc, 0.f)), 1.0000019f, pad);
+                        const int cx0 = max(lx0, __float2int_rd((pxr - half) * inv_Sx));
+                        const int cx1 = min(lx1, __float2int_rd((pxr + half) * inv_Sx));
+                        rg[u] = 0u;
+                        if (vy <= vend && dyc <= Re && cx0 <= cx1) {
+                            const int rr = vy - BY0;
+                            const int base = sm.rpre[rr] - sm.rx0[rr];
+                            const uint32_t t0 = sm.cstart[base + cx0], t1 = sm.cstart[base + cx1 + 1];
+                            rg[u] = t0 < t1 ? (t1 << 16) | t0 : 0u;
+                        }
+                    }
+                    uint32_t n0 = 0u, n1 = 0u, n2 = 0u, n3 = 0u;  // the ranges, empty ones left out
+#pragma unroll
+                    for (int u = 3; u >= 0; u--) {
+                        if (rg[u]) {
+                            n3 = n2;
+                            n2 = n1;
+                            n1 = n0;
+                            n0 = rg[u];
+                        }
+                    }
+                    int t = (int)(n0 & 0xffffu), e = (int)(n0 >> 16);
+                    // four records per round, their loads issued together (what lies
+                    // past the row's end is read and never passes)
+                    while (t < e) {
                         float2 cc[4];
 #pragma unroll
-                        for (int u = 0; u < 4; u++) cc[u] = sm.rec[min(t + u, e - 1)];
+                        for (int u = 0; u < 4; u++) cc[u] = sm.rec[t + u];
 #pragma unroll
                         for (int u = 0; u < 4; u++) {
                             const float dx = cc[u].x - rqx, dy = cc[u].y - rqy;
@@ -439,6 +503,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                             const bool pass = d2 <= R2 && t + u != myself && t + u < e;
                             mylist[min(cnt, LCAP)][lane] = (key_of<KB>(d2, qs) << SB) | (uint32_t)(t + u);
                             cnt += pass ? 1 : 0;
+                        }
+                        t += 4;
+                        if (t >= e) {
+                            t = (int)(n1 & 0xffffu);
+                            e = (int)(n1 >> 16);
+                            n1 = n2;
+                            n2 = n3;
+                            n3 = 0u;
                         }
                     }
                 }
@@ -458,16 +530,24 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
             uint32_t kth = 0, kprv = 0, knx = 0xffffffffu;
             bool order_ok = true;
             auto sorted_path = [&]() {
-                if (ok) OddEvenSort<A>{arr}.run();
+                if (MODE != MODE_MIXED && k <= KSEL) {
+                    if (ok) LowSort<A, KSEL>{arr}.run();
+                } else {
+                    if (ok) OddEvenSort<A>{arr}.run();
+                }
 #pragma unroll
                 for (int i = 0; i < A; i++) {
                     kth = max(kth, i < k ? arr[i] : 0u);
                     kprv = max(kprv, i < k - 1 ? arr[i] : 0u);
                     knx = min(knx, i >= k ? arr[i] : 0xffffffffu);
-                    if (MODE != MODE_MIXED && i > 0 && i < k) {
-                        const float ki = (float)(arr[i] >> SB) * unit, kp = (float)(arr[i - 1] >> SB) * unit;
-                        order_ok = order_ok && (ki - kp > 2.f * (kEpsRel * ki + ea));
-                    }
+                }
+                if (MODE != MODE_MIXED) {
+                    // the order stands when every neighbour is more than 2 eps from the
+                    // next, eps taken at R (a query failing this is only re-ranked)
+                    const uint32_t need = (uint32_t)fminf(2.f * (kEpsRel * R2 + ea) / unit + 2.f, 4.0e9f);
+#pragma unroll
+                    for (int i = 1; i < A; i++)
+                        if (i < k) order_ok = order_ok && (arr[i] >> SB) - (arr[i - 1] >> SB) > need;
                 }
             };
             if constexpr (SEL) {
