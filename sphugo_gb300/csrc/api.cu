@@ -279,6 +279,7 @@ SimDev make_simdev(const sph_params &p, int64_t off, int64_t n, int64_t cell_off
     reset_reductions(S);
     S.tol = (float)(std::max(S.L[0], S.L[1]) * 4.0e-7);
     simdev_floats(S);
+    simdev_fcell(S);
     return S;
 }
 

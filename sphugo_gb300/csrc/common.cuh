@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <string>
 
@@ -70,6 +71,7 @@ struct SimDev {
     // FP32 copies used per query (no FP64 instruction in the search's hot path)
     float fs[2];           // finest cell side
     float fdtc[2];         // dth / finest cell side (the binning's drift in cell units)
+    float fcell[2];        // inv_s where it is a power of two and lo = 0 (cells per unit, exact), else 0
     float fimg_h[2], fimg_l[2]; // image shifts as float pairs (hi, lo)
     float flmax;           // max(L)
     float fmag;            // bound on |p + offset| of any particle image (the reference rounds it)
@@ -140,6 +142,18 @@ __device__ __forceinline__ uint32_t part1by1(uint32_t x) {
 }
 __device__ __forceinline__ uint32_t morton2(uint32_t cx, uint32_t cy) {
     return part1by1(cx) | (part1by1(cy) << 1);
+}
+
+// fcell of the periodic axes (an open axis's grid comes from its bounding box:
+// 0). From 1 up: a position beyond FP32 overflows with or without the product.
+inline void simdev_fcell(SimDev &S) {
+    for (int a = 0; a < 2; a++) {
+        const float fc = (float)S.inv_s[a];
+        uint32_t fb;
+        memcpy(&fb, &fc, 4);
+        const bool p2 = (fb & 0x7fffffu) == 0u && fc >= 1.f && (double)fc == S.inv_s[a];
+        S.fcell[a] = S.periodic[a] && p2 && S.lo[a] == 0.0 ? fc : 0.f;
+    }
 }
 
 // FP32 fields of a SimDev from its FP64 grid fields

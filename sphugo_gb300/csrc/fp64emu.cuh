@@ -204,6 +204,21 @@ __device__ __forceinline__ double emu_one_minus(double x) {
     return r;
 }
 
+static __device__ __noinline__ float emu_native_d2f(double x) { return __double2float_rn(x); }
+
+// RN_float(v): the significand rounded to 24 bits, ties to even. (The
+// hardware's conversion holds the FP64 unit as long as an addition.) Values
+// whose float would not be normal take it.
+__device__ __forceinline__ float emu_d2f(double v) {
+    const uint32_t ah = emu_hi(v), al = emu_lo(v);
+    const uint32_t e = (ah >> 20) & 0x7ffu;
+    const uint32_t q = emu_fsl(al, (ah & 0xfffffu) | 0x100000u, 3), rem = al & 0x1fffffffu;  // q: 24 bits
+    const uint32_t up = rem + (q & 1u) > 0x10000000u ? 1u : 0u;
+    float f = __uint_as_float((ah & 0x80000000u) | (((e - 897u) << 23) + q + up));
+    if (!(e - 897u < 253u)) f = emu_native_d2f(v);
+    return f;
+}
+
 // The float pair of v: hi = RN_float(v) and lo = RN_float(v - hi) (v - hi is
 // exact in binary64). hi rounds the 53-bit significand to 24 bits; the
 // remainder t = m - hi's significand 2^29 is an integer below 2^29 in

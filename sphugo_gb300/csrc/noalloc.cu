@@ -199,6 +199,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     reset_reductions(S);
     S.tol = (float)(std::max(S.L[0], S.L[1]) * 4.0e-7);
     simdev_floats(S);
+    simdev_fcell(S);
     T.ncells = (int64_t)1 << (2 * S.level);
     const bool any_open = !S.periodic[0] || !S.periodic[1];
 
