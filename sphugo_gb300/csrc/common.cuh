@@ -258,7 +258,6 @@ void launch_knn(const Ctx &c, const Launch &L, const PArrays &B, const Derived &
 void launch_density(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int mode,
                     const KnnTune *tune);
 void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D);
-void force_init_attrs();
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
                   const Derived &D, int mode, bool integrate);
 void launch_error_norms(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, double *anorm,

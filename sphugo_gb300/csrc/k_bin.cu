@@ -447,11 +447,15 @@ __global__ void k_permute(Ctx c, PArrays A, PArrays B, Tables T, int pred, int v
 
 void launch_permute(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
                     const Tables &T, int pred, bool velrec) {
-    const Pass p(L, c.n);
+    // a block per 256 particles: the copies of this pass, unlike the binning's
+    // atomics and scattered ids, gain from blocks in order (clustered
+    // N = 4,194,304 130 -> 121 us against 8 striding blocks per SM; the binning
+    // pass then takes 67 instead of 60)
+    const int block = Pass(L, c.n).block, grid = (int)((c.n + block - 1) / block);
     // the ranks' loads in front of the drift cost more than a launch once the
     // arrays outgrow L2 (clustered N = 4,194,304: 165 us against 130 + 21)
-    if (c.n > kRankPassN) k_permute<true><<<p.grid, p.block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
-    else k_permute<false><<<p.grid, p.block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
+    if (c.n > kRankPassN) k_permute<true><<<grid, block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
+    else k_permute<false><<<grid, block, 0, L.stream>>>(c, A, B, T, pred, velrec ? 1 : 0);
 }
 
 }  // namespace sphgpu

@@ -15,8 +15,9 @@
 // loads issued early changed nothing (542 us both).
 //
 // Measured against one thread per particle with three passes over its list
-// (density stage, us): N = 1000 49 -> 12, 10,000 61 -> 21, 100,000 107 -> 72,
-// 1,048,576 690 -> 540, clustered 4,194,304 2620 -> 2190.
+// (density stage, us): N = 1000 49 -> 12, 10,000 61 -> 21, 100,000 107 -> 70,
+// 1,048,576 690 -> 502 (540 with resident blocks of four warps striding over
+// the tiles), clustered 4,194,304 2620 -> 1893 (2190).
 #include "pair_tile.cuh"
 
 #include <algorithm>
@@ -29,7 +30,7 @@ struct DensityArgs {
     Ctx c;
     PArrays B;
     Derived D;
-    int W;
+    PairTiles tiles;
 };
 
 // what the pairs of a particle share: its position, h and h as a divisor
@@ -85,118 +86,115 @@ __device__ __forceinline__ void wendland(double q, PairF &r) {
     r.df = emu_mul_n(emu_mul_n(emu_mul_n(__dmul_rn(-10.0, q), a), a), a);
 }
 
-// 8 blocks (64 registers): 540 us at N = 1,048,576 against 565 at 6 blocks
-// (74 registers, no spills either) and 556 at 9
-__global__ void __launch_bounds__(kPairWarps * 32, 8) k_density_fp64(DensityArgs a) {
-    __shared__ DensityWarp smem[kPairWarps];
-    const int k = a.c.k, W = a.W;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    DensityWarp &sm = smem[w];
+// 32 blocks (64 registers): 502 us at N = 1,048,576 against 510 to 512 at 20,
+// 24 and 28 (no spills either)
+__global__ void __launch_bounds__(32, 32) k_density_fp64(DensityArgs a) {
+    __shared__ DensityWarp sm;
+    const int k = a.c.k, lane = threadIdx.x;
     const PArrays &B = a.B;
+    int W;
+    const int64_t q0 = a.tiles.first(blockIdx.x, W);
     const PairChunks ch(k, W);
     unsigned fl = 0;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kPairWarps + w) * W; q0 < a.c.n; q0 += (int64_t)gridDim.x * kPairWarps * W) {
-        const int np = (int)min((int64_t)W, a.c.n - q0);
-        const int32_t *nb = a.D.nbr + q0 * k;
-        double2 *dist = a.D.dist + q0 * k;
-        double h = 1.0, acc = 0.0;
-        if (lane < np) {
-            const int s = sim_of(a.c, q0 + lane);
-            const SimDev &S = a.c.sims[s];
-            const double2 P = B.pos[q0 + lane];
-            const double dk2 = nbr_d2(S, B, P, (uint32_t)nb[lane * k + k - 1]);
-            if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
-            h = emu_sqrt(dk2);
-            const EmuDivisor dh = emu_divisor(h);  // shared by the k quotients d/h
-            DensityRow &R = sm.row[lane];
-            R.x = P.x;
-            R.y = P.y;
-            R.h = h;
-            R.mb = dh.mb;
-            R.inv = dh.inv;
-            R.kernel = S.kernel;
-            R.sim = s;
-        }
-        const bool plain = __all_sync(0xffffffffu, emu_within<150>(h));
-        __syncwarp();
-        for (int c = 0, e_lo = k; c < ch.n; c++) {
-            const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce;
-            e_lo -= ce;
-            int nnear = 0;
-            for (int i0 = 0; i0 < np * ce; i0 += 32) {
-                const int i = i0 + lane;
-                bool near = false;
-                int slot = 0;
-                if (i < np * ce) {
-                    const int p = pair_row(i, magic), at = p * k + e_lo + (i - p * ce);
-                    slot = i + p * (st - ce);
-                    const DensityRow &R = sm.row[p];
-                    const uint32_t code = (uint32_t)nb[at];
-                    const double2 Q = B.pos[code >> kCodeShift];
-                    double px = R.x, py = R.y;
-                    if ((code & 15u) != 4u) {
-                        double ox, oy;
-                        img_shift(a.c.sims[R.sim], code & 15u, ox, oy);
-                        px = __dadd_rn(px, ox);
-                        py = __dadd_rn(py, oy);
-                    }
-                    const double dx = __dsub_rn(px, Q.x), dy = __dsub_rn(py, Q.y);
-                    PairF r;
-                    if (plain && emu_within<150>(dx) && emu_within<150>(dy)) {
-                        r.d = emu_sqrt_n(__dadd_rn(emu_mul_n(dx, dx), emu_mul_n(dy, dy)));
-                        const double q = emu_div_n(r.d, EmuDivisor{R.mb, R.inv, emu_hi(R.h)});  // in (0, 1]: d <= h
-                        const uint32_t qh = emu_hi(q);
-                        near = R.kernel != SPH_KERNEL_WENDLAND && qh < 0x3fe00000u;
-                        if (near) r.f = q;
-                        else if (R.kernel != SPH_KERNEL_WENDLAND) monahan_far(q, r);
-                        else wendland(q, r);
-                        if (qh == 0x3ff00000u) {  // q = 1: 1 - q = 0, which the products do not take
-                            r.f = 0.0;
-                            r.df = -0.0;
-                        }
-                    } else {
-                        r = pair_slow(dx, dy, R.h, R.kernel);
-                    }
-                    dist[at] = make_double2(r.d, r.df);
-                    sm.term[slot] = r.f;
+    const int np = (int)min((int64_t)W, a.c.n - q0);
+    const int32_t *nb = a.D.nbr + q0 * k;
+    double2 *dist = a.D.dist + q0 * k;
+    double h = 1.0, acc = 0.0;
+    if (lane < np) {
+        const int s = sim_of(a.c, q0 + lane);
+        const SimDev &S = a.c.sims[s];
+        const double2 P = B.pos[q0 + lane];
+        const double dk2 = nbr_d2(S, B, P, (uint32_t)nb[lane * k + k - 1]);
+        if (!(dk2 < 0.4)) fl |= FLAG_SENTINEL;
+        h = emu_sqrt(dk2);
+        const EmuDivisor dh = emu_divisor(h);  // shared by the k quotients d/h
+        DensityRow &R = sm.row[lane];
+        R.x = P.x;
+        R.y = P.y;
+        R.h = h;
+        R.mb = dh.mb;
+        R.inv = dh.inv;
+        R.kernel = S.kernel;
+        R.sim = s;
+    }
+    const bool plain = __all_sync(0xffffffffu, emu_within<150>(h));
+    __syncwarp();
+    for (int c = 0, e_lo = k; c < ch.n; c++) {
+        const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce;
+        e_lo -= ce;
+        int nnear = 0;
+        for (int i0 = 0; i0 < np * ce; i0 += 32) {
+            const int i = i0 + lane;
+            bool near = false;
+            int slot = 0;
+            if (i < np * ce) {
+                const int p = pair_row(i, magic), at = p * k + e_lo + (i - p * ce);
+                slot = i + p * (st - ce);
+                const DensityRow &R = sm.row[p];
+                const uint32_t code = (uint32_t)nb[at];
+                const double2 Q = B.pos[code >> kCodeShift];
+                double px = R.x, py = R.y;
+                if ((code & 15u) != 4u) {
+                    double ox, oy;
+                    img_shift(a.c.sims[R.sim], code & 15u, ox, oy);
+                    px = __dadd_rn(px, ox);
+                    py = __dadd_rn(py, oy);
                 }
-                const uint32_t bal = __ballot_sync(0xffffffffu, near);
-                if (near) sm.near[nnear + __popc(bal & lanemask_lt())] = (uint16_t)i;
-                nnear += __popc(bal);
+                const double dx = __dsub_rn(px, Q.x), dy = __dsub_rn(py, Q.y);
+                PairF r;
+                if (plain && emu_within<150>(dx) && emu_within<150>(dy)) {
+                    r.d = emu_sqrt_n(__dadd_rn(emu_mul_n(dx, dx), emu_mul_n(dy, dy)));
+                    const double q = emu_div_n(r.d, EmuDivisor{R.mb, R.inv, emu_hi(R.h)});  // in (0, 1]: d <= h
+                    const uint32_t qh = emu_hi(q);
+                    near = R.kernel != SPH_KERNEL_WENDLAND && qh < 0x3fe00000u;
+                    if (near) r.f = q;
+                    else if (R.kernel != SPH_KERNEL_WENDLAND) monahan_far(q, r);
+                    else wendland(q, r);
+                    if (qh == 0x3ff00000u) {  // q = 1: 1 - q = 0, which the products do not take
+                        r.f = 0.0;
+                        r.df = -0.0;
+                    }
+                } else {
+                    r = pair_slow(dx, dy, R.h, R.kernel);
+                }
+                dist[at] = make_double2(r.d, r.df);
+                sm.term[slot] = r.f;
             }
-            __syncwarp();
-            // the pairs with q < 1/2, with all lanes at work (a quarter of the
-            // pairs, but some of them in half of the rounds above)
-            for (int n = lane; n < nnear; n += 32) {
-                const int i = sm.near[n], p = pair_row(i, magic), slot = i + p * (st - ce);
-                double f, df;
-                monahan_near(sm.term[slot], f, df);
-                sm.term[slot] = f;
-                dist[p * k + e_lo + (i - p * ce)].y = df;
-            }
-            __syncwarp();
-            if (lane < np) {
-                const double *t = sm.term + lane * st;
-                for (int e = ce - 1; e >= 0; e--) acc = __dadd_rn(acc, t[e]);
-            }
-            __syncwarp();
-        }
-        if (lane < np) {
-            const int64_t q = q0 + lane;
-            const SimDev &S = a.c.sims[sim_of(a.c, q)];
-            const double gamma = S.gamma, up = B.up[q];
-            const double hh = emu_mul(h, h);
-            const double rho = emu_div(emu_mul(__dmul_rn(S.fpref, S.mass), acc), emu_divisor(hh), hh);
-            if (!(rho >= 0.0 && rho < 1.0e308)) fl |= FLAG_Q_RANGE;  // a NaN or infinite distance
-            const double cs = emu_sqrt(emu_mul(__dmul_rn(gamma, __dsub_rn(gamma, 1.0)), up));
-            const double grho = emu_mul(gamma, rho);
-            const double ct = emu_div(emu_mul(cs, cs), emu_divisor(grho), grho);
-            a.D.rho[q] = rho;
-            a.D.c[q] = cs;
-            a.D.h[q] = h;
-            a.D.der[q] = make_double4(cs, rho, h, ct);
+            const uint32_t bal = __ballot_sync(0xffffffffu, near);
+            if (near) sm.near[nnear + __popc(bal & lanemask_lt())] = (uint16_t)i;
+            nnear += __popc(bal);
         }
         __syncwarp();
+        // the pairs with q < 1/2, with all lanes at work (a quarter of the
+        // pairs, but some of them in half of the rounds above)
+        for (int n = lane; n < nnear; n += 32) {
+            const int i = sm.near[n], p = pair_row(i, magic), slot = i + p * (st - ce);
+            double f, df;
+            monahan_near(sm.term[slot], f, df);
+            sm.term[slot] = f;
+            dist[p * k + e_lo + (i - p * ce)].y = df;
+        }
+        __syncwarp();
+        if (lane < np) {
+            const double *t = sm.term + lane * st;
+            for (int e = ce - 1; e >= 0; e--) acc = __dadd_rn(acc, t[e]);
+        }
+        __syncwarp();
+    }
+    if (lane < np) {
+        const int64_t q = q0 + lane;
+        const SimDev &S = a.c.sims[sim_of(a.c, q)];
+        const double gamma = S.gamma, up = B.up[q];
+        const double hh = emu_mul(h, h);
+        const double rho = emu_div(emu_mul(__dmul_rn(S.fpref, S.mass), acc), emu_divisor(hh), hh);
+        if (!(rho >= 0.0 && rho < 1.0e308)) fl |= FLAG_Q_RANGE;  // a NaN or infinite distance
+        const double cs = emu_sqrt(emu_mul(__dmul_rn(gamma, __dsub_rn(gamma, 1.0)), up));
+        const double grho = emu_mul(gamma, rho);
+        const double ct = emu_div(emu_mul(cs, cs), emu_divisor(grho), grho);
+        a.D.rho[q] = rho;
+        a.D.c[q] = cs;
+        a.D.h[q] = h;
+        a.D.der[q] = make_double4(cs, rho, h, ct);
     }
     if (fl) atomicOr(a.c.flags, fl);
 }
@@ -206,13 +204,11 @@ __global__ void __launch_bounds__(kPairWarps * 32, 8) k_density_fp64(DensityArgs
 void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D) {
     static const int per_sm = [] {
         int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_fp64, kPairWarps * 32, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_fp64, 32, 0);
         return std::max(nb, 1);
     }();
-    DensityArgs a{c, B, D, pair_width(c.n, (int64_t)L.sms * per_sm * kPairWarps)};
-    const int64_t tiles = (c.n + a.W - 1) / a.W;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((tiles + kPairWarps - 1) / kPairWarps, (int64_t)L.sms * per_sm));
-    k_density_fp64<<<grid, kPairWarps * 32, 0, L.stream>>>(a);
+    DensityArgs a{c, B, D, PairTiles(c.n, (int64_t)L.sms * per_sm)};
+    k_density_fp64<<<a.tiles.grid(), 32, 0, L.stream>>>(a);
 }
 
 }  // namespace sphgpu

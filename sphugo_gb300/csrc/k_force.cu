@@ -10,16 +10,16 @@
 
 namespace sphgpu {
 
-// Resident blocks of the FP64 force per SM (96 registers, 38 KB): 1160 us at
-// N = 1,048,576; 4 blocks 1198, 6 (80 registers) slower still.
 // Particles up to which the mixed force deals its pairs over the lanes (force
 // stage with and without: N = 1000 12 and 18 us, 10,000 17 and 20, 20,000 20
 // and 20, 100,000 39 and 29: a thread per particle then fills the GPU, and
 // the factors' way through shared memory costs issue slots).
 constexpr int64_t kMixedPairsMaxN = 16384;
-constexpr int kMixedBlocks = 5;  // resident blocks per SM (31 KB each)
-constexpr int kForceBlocks = 5;
-// Tiles up to this width sum with three lanes per particle: 31 us at N = 10,000
+constexpr int kMixedBlocks = 20;  // resident blocks (warps) per SM (8 KB each)
+// Blocks (warps) of the FP64 force per SM asked of the compiler: 92 registers,
+// 9.5 KB, 21 resident.
+constexpr int kForceBlocks = 20;
+// Tiles up to this width sum with three lanes per particle: 29 us at N = 10,000
 // against 40 with one.
 constexpr int kSplitWidth = 10;
 
@@ -70,14 +70,16 @@ __device__ __forceinline__ void integrate_one(const SimDev &S, double2 &pos, dou
 // The mixed form, one thread per particle. Bound by its neighbour gathers (ncu,
 // uniform blast N = 1,048,576: L1 data path 69 % busy, 9 cycles of waiting on
 // loads per issued instruction); 80 registers: at the 10 or 12 resident blocks
-// that fewer would allow it ran 271 and 328 us against 217.
+// that fewer would allow it ran 271 and 328 us against 217. A block per 128
+// particles, not 16 blocks per SM striding over them: 217 -> 204, clustered
+// N = 4,194,304 790 -> 730; records loaded one or two pairs ahead: 260 to 335.
 __global__ void __launch_bounds__(128, 6) k_force_mixed(ForceArgs a) {
     const int k = a.c.k;
     const PArrays &B = a.B;
     const Derived &D = a.D;
     unsigned fl = 0;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < a.c.n;
-         q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (q < a.c.n) {
         const int s = sim_of(a.c, q);
         const SimDev &S = a.c.sims[s];
         const double2 P = B.pos[q];
@@ -168,101 +170,98 @@ __device__ __forceinline__ void kahan_fma(KahanF &s, float x, float f) {
     s.s = t;
 }
 
-__global__ void __launch_bounds__(kPairWarps * 32, kMixedBlocks) k_force_mixed_pairs(ForceArgs a, int W) {
-    __shared__ MixedWarp smem[kPairWarps];
-    const int k = a.c.k;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    MixedWarp &sm = smem[w];
+__global__ void __launch_bounds__(32, kMixedBlocks) k_force_mixed_pairs(ForceArgs a, PairTiles tiles) {
+    __shared__ MixedWarp sm;
+    const int k = a.c.k, lane = threadIdx.x;
+    int W;
+    const int64_t q0 = tiles.first(blockIdx.x, W);
     const PArrays &B = a.B;
     const Derived &D = a.D;
     const PairChunks ch(k, W);
     unsigned fl = 0;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kPairWarps + w) * W; q0 < a.c.n; q0 += (int64_t)gridDim.x * kPairWarps * W) {
-        const int np = (int)min((int64_t)W, a.c.n - q0);
-        const int32_t *nb = D.nbr + q0 * k;
-        if (lane < np) {
-            const int64_t q = q0 + lane;
-            const float4 di = D.derf[q];
-            MixedRow &R = sm.row[lane];
-            R.rec = B.rec[q];
-            R.vrec = B.vrec[q];
-            R.c = di.x; R.rho = di.y; R.h = di.z; R.cterm = di.w;
-            R.inv_h = 1.f / di.z;
-            R.sim = sim_of(a.c, q);
-        }
-        __syncwarp();
-        KahanF ax, ay, ed;
-        for (int c = 0, e_lo = k; c < ch.n; c++) {
-            const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
-            e_lo -= ce;
-            for (int i = lane; i < npair; i += 32) {
-                const int p = pair_row(i, magic), at = p * k + e_lo + (i - p * ce), slot = i + p * (st - ce);
-                const MixedRow &R = sm.row[p];
-                const SimDev &S = a.c.sims[R.sim];
-                const uint32_t code = (uint32_t)nb[at], j = code >> kCodeShift;
-                const float4 rj = __ldg(&B.rec[j]), vj = __ldg(&B.vrec[j]), dj = __ldg(&D.derf[j]);
-                const float4 vi = R.vrec;
-                float rabx, raby;  // r_AB = (q - offset) - p from float pairs
-                float_pair_rel(S, R.rec, rj, code & 15u, rabx, raby);
-                const float d2 = __fmaf_rn(rabx, rabx, raby * raby);
-                const float invd = rsqrtf(d2);
-                const float qq = fminf(d2 * invd * R.inv_h, 1.f);
-                const float drk = kdf_f32(S.kernel, qq);
-                const float vabx = (vj.x - vi.x) + (vj.z - vi.z);
-                const float vaby = (vj.y - vi.y) + (vj.w - vi.w);
-                const float dot = vabx * rabx + vaby * raby;
-                float piab = 0.f;
-                if (dot < 0.f) {
-                    const float cab = 0.5f * (R.c + dj.x);
-                    const float rhoab = 0.5f * (R.rho + dj.y);
-                    const float hab = 0.5f * (R.h + dj.z);
-                    // two-instruction quotients (<= 2 ulp; both denominators are
-                    // normal: d2 + eta^2 >= eta^2, rho_AB > 0)
-                    const float mu = __fdividef(dot * hab, d2 + S.fetasq);
-                    piab = __fdividef(mu * (S.fbeta * mu - S.falpha * cab), rhoab);
-                }
-                sm.rx[slot] = rabx;
-                sm.ry[slot] = raby;
-                sm.w[slot] = (piab + R.cterm + dj.w) * drk * invd;
-                sm.dot[slot] = dot;
-                sm.drk[slot] = drk;
-            }
-            __syncwarp();
-            if (lane < np) {
-                for (int e = ce - 1; e >= 0; e--) {
-                    const int t = lane * st + e;
-                    const float wt = sm.w[t];
-                    kahan_fma(ax, sm.rx[t], wt);
-                    kahan_fma(ay, sm.ry[t], wt);
-                    kahan_fma(ed, sm.dot[t], sm.drk[t]);
-                }
-            }
-            __syncwarp();
-        }
-        if (lane < np) {
-            const int64_t q = q0 + lane;
-            const MixedRow &R = sm.row[lane];
+    const int np = (int)min((int64_t)W, a.c.n - q0);
+    const int32_t *nb = D.nbr + q0 * k;
+    if (lane < np) {
+        const int64_t q = q0 + lane;
+        const float4 di = D.derf[q];
+        MixedRow &R = sm.row[lane];
+        R.rec = B.rec[q];
+        R.vrec = B.vrec[q];
+        R.c = di.x; R.rho = di.y; R.h = di.z; R.cterm = di.w;
+        R.inv_h = 1.f / di.z;
+        R.sim = sim_of(a.c, q);
+    }
+    __syncwarp();
+    KahanF ax, ay, ed;
+    for (int c = 0, e_lo = k; c < ch.n; c++) {
+        const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
+        e_lo -= ce;
+        for (int i = lane; i < npair; i += 32) {
+            const int p = pair_row(i, magic), at = p * k + e_lo + (i - p * ce), slot = i + p * (st - ce);
+            const MixedRow &R = sm.row[p];
             const SimDev &S = a.c.sims[R.sim];
-            const float inv_hf = R.inv_h;
-            const float ff = S.fdfm * (inv_hf * inv_hf * inv_hf);
-            const double axo = (double)(ax.value_f() * ff) + S.accel[0];
-            const double ayo = (double)(ay.value_f() * ff) + S.accel[1];
-            const double edot = (double)(R.cterm * ed.value_f() * S.fmass);
-            if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
-            double2 pos = B.pos[q], vel = B.vel[q];
-            double u = B.u[q];
-            if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
-            a.A.pos[q] = pos;
-            a.A.vel[q] = vel;
-            a.A.u[q] = u;
-            a.A.acc[q] = make_double2(axo, ayo);
-            a.A.udot[q] = edot;
-            a.A.id[q] = B.id[q];
-            a.A.hprev[q] = R.h;  // the smoothing length rounded to FP32
-            a.A.vp[q] = B.vp[q];
-            a.A.up[q] = B.up[q];
+            const uint32_t code = (uint32_t)nb[at], j = code >> kCodeShift;
+            const float4 rj = __ldg(&B.rec[j]), vj = __ldg(&B.vrec[j]), dj = __ldg(&D.derf[j]);
+            const float4 vi = R.vrec;
+            float rabx, raby;  // r_AB = (q - offset) - p from float pairs
+            float_pair_rel(S, R.rec, rj, code & 15u, rabx, raby);
+            const float d2 = __fmaf_rn(rabx, rabx, raby * raby);
+            const float invd = rsqrtf(d2);
+            const float qq = fminf(d2 * invd * R.inv_h, 1.f);
+            const float drk = kdf_f32(S.kernel, qq);
+            const float vabx = (vj.x - vi.x) + (vj.z - vi.z);
+            const float vaby = (vj.y - vi.y) + (vj.w - vi.w);
+            const float dot = vabx * rabx + vaby * raby;
+            float piab = 0.f;
+            if (dot < 0.f) {
+                const float cab = 0.5f * (R.c + dj.x);
+                const float rhoab = 0.5f * (R.rho + dj.y);
+                const float hab = 0.5f * (R.h + dj.z);
+                // two-instruction quotients (<= 2 ulp; both denominators are
+                // normal: d2 + eta^2 >= eta^2, rho_AB > 0)
+                const float mu = __fdividef(dot * hab, d2 + S.fetasq);
+                piab = __fdividef(mu * (S.fbeta * mu - S.falpha * cab), rhoab);
+            }
+            sm.rx[slot] = rabx;
+            sm.ry[slot] = raby;
+            sm.w[slot] = (piab + R.cterm + dj.w) * drk * invd;
+            sm.dot[slot] = dot;
+            sm.drk[slot] = drk;
         }
         __syncwarp();
+        if (lane < np) {
+            for (int e = ce - 1; e >= 0; e--) {
+                const int t = lane * st + e;
+                const float wt = sm.w[t];
+                kahan_fma(ax, sm.rx[t], wt);
+                kahan_fma(ay, sm.ry[t], wt);
+                kahan_fma(ed, sm.dot[t], sm.drk[t]);
+            }
+        }
+        __syncwarp();
+    }
+    if (lane < np) {
+        const int64_t q = q0 + lane;
+        const MixedRow &R = sm.row[lane];
+        const SimDev &S = a.c.sims[R.sim];
+        const float inv_hf = R.inv_h;
+        const float ff = S.fdfm * (inv_hf * inv_hf * inv_hf);
+        const double axo = (double)(ax.value_f() * ff) + S.accel[0];
+        const double ayo = (double)(ay.value_f() * ff) + S.accel[1];
+        const double edot = (double)(R.cterm * ed.value_f() * S.fmass);
+        if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
+        double2 pos = B.pos[q], vel = B.vel[q];
+        double u = B.u[q];
+        if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
+        a.A.pos[q] = pos;
+        a.A.vel[q] = vel;
+        a.A.u[q] = u;
+        a.A.acc[q] = make_double2(axo, ayo);
+        a.A.udot[q] = edot;
+        a.A.id[q] = B.id[q];
+        a.A.hprev[q] = R.h;  // the smoothing length rounded to FP32
+        a.A.vp[q] = B.vp[q];
+        a.A.up[q] = B.up[q];
     }
     if (fl) atomicOr(a.c.flags, fl);
 }
@@ -312,9 +311,10 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
 // one each: 1231 -> 1160.
 //
 // Against one warp per 32 particles, a lane each, with the approaching pairs
-// compacted per warp (force stage, us): N = 1000 112 -> 16, 10,000 154 -> 31,
-// 100,000 297 -> 148, 1,048,576 1750 -> 1160, clustered 4,194,304
-// 6800 -> 4520, stress 2,000,003 (k = 64) 6370 -> 4210.
+// compacted per warp (force stage, us): N = 1000 112 -> 14, 10,000 154 -> 29,
+// 100,000 297 -> 133 (149 with resident blocks of four warps striding over
+// tiles of one width), 1,048,576 1750 -> 1103 (1165), clustered 4,194,304
+// 6800 -> 4262 (4540), stress 2,000,003 (k = 64) 6370 -> 4004 (4210).
 struct ForceRow {
     double x, y, vx, vy;      // position and predicted velocity
     double c, rho, h, cterm;  // sound speed, density, smoothing length, c^2 / (gamma rho)
@@ -357,208 +357,193 @@ __device__ __noinline__ ForceTerms force_terms_slow(double rx, double ry, double
 
 __device__ __forceinline__ double emu_halve(double x) { return emu_double(emu_bits(x) - (1ull << 52)); }
 
-__global__ void __launch_bounds__(kPairWarps * 32, kForceBlocks) k_force_fp64(ForceArgs a, int W) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int k = a.c.k;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    ForceWarp &sm = reinterpret_cast<ForceWarp *>(smem_raw)[w];
+__global__ void __launch_bounds__(32, kForceBlocks) k_force_fp64(ForceArgs a, PairTiles tiles) {
+    __shared__ ForceWarp sm;
+    const int k = a.c.k, lane = threadIdx.x;
+    int W;
+    const int64_t q0 = tiles.first(blockIdx.x, W);
     const PArrays &B = a.B;
     const Derived &D = a.D;
     const PairChunks ch(k, W);
     unsigned fl = 0;
-    for (int64_t q0 = ((int64_t)blockIdx.x * kPairWarps + w) * W; q0 < a.c.n; q0 += (int64_t)gridDim.x * kPairWarps * W) {
-        const int np = (int)min((int64_t)W, a.c.n - q0);
-        const int32_t *nb = D.nbr + q0 * k;
-        const double2 *dist = D.dist + q0 * k;
-        if (lane < np) {
-            const int64_t q = q0 + lane;
-            const double2 P = B.pos[q], V = B.vp[q];
-            ForceRow &R = sm.row[lane];
-            R.x = P.x; R.y = P.y; R.vx = V.x; R.vy = V.y;
-            const double4 d = D.der[q];
-            R.c = d.x; R.rho = d.y; R.h = d.z; R.cterm = d.w;
+    const int np = (int)min((int64_t)W, a.c.n - q0);
+    const int32_t *nb = D.nbr + q0 * k;
+    const double2 *dist = D.dist + q0 * k;
+    if (lane < np) {
+        const int64_t q = q0 + lane;
+        const double2 P = B.pos[q], V = B.vp[q];
+        ForceRow &R = sm.row[lane];
+        R.x = P.x; R.y = P.y; R.vx = V.x; R.vy = V.y;
+        const double4 d = D.der[q];
+        R.c = d.x; R.rho = d.y; R.h = d.z; R.cterm = d.w;
+    }
+    __syncwarp();
+    double ax = 0.0, ay = 0.0, ed = 0.0;  // (three lanes per particle: ax alone, lane 3 p + component)
+    for (int c = 0, e_lo = k; c < ch.n; c++) {
+        const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
+        e_lo -= ce;
+        // ---- A
+        int nlist = 0, nrest = 0;
+        // a round's loads are issued a round (the neighbour's data) or two (its
+        // code) before their use
+        auto entry = [&](int i) {
+            const int p = pair_row(i, magic);
+            return p * k + e_lo + (i - p * ce);
+        };
+        uint32_t code1 = lane < npair ? (uint32_t)nb[entry(lane)] : 0u;
+        uint32_t code2 = lane + 32 < npair ? (uint32_t)nb[entry(lane + 32)] : 0u;
+        double2 V1 = B.vp[code1 >> kCodeShift], Q1 = B.pos[code1 >> kCodeShift];
+        for (int i0 = 0; i0 < npair; i0 += 32) {
+            const int i = i0 + lane;
+            bool approach = false;
+            const uint32_t code = code1;
+            const double2 V = V1, Q = Q1;
+            code1 = code2;
+            V1 = B.vp[code1 >> kCodeShift];
+            Q1 = B.pos[code1 >> kCodeShift];
+            code2 = i + 64 < npair ? (uint32_t)nb[entry(i + 64)] : 0u;
+            if (i < npair) {
+                const int p = pair_row(i, magic), slot = i + p * (st - ce);
+                const ForceRow &R = sm.row[p];
+                const double vx = __dsub_rn(V.x, R.vx), vy = __dsub_rn(V.y, R.vy);
+                double qx = Q.x, qy = Q.y;
+                if ((code & 15u) != 4u) {
+                    double ox, oy;
+                    img_shift(a.c.sims[sim_of(a.c, q0 + p)], code & 15u, ox, oy);
+                    qx = __dsub_rn(qx, ox);
+                    qy = __dsub_rn(qy, oy);
+                }
+                const double rx = __dsub_rn(qx, R.x), ry = __dsub_rn(qy, R.y);
+                double dot;
+                if (emu_within<150>(rx) && emu_within<150>(ry) && emu_within<150>(vx) && emu_within<150>(vy)) {
+                    dot = __dadd_rn(emu_mul_n(vx, rx), emu_mul_n(vy, ry));  // 0, or 2^-353 at least (no subnormal)
+                    approach = emu_hi(dot) > 0x80000000u;
+                } else {
+                    dot = force_dot_slow(rx, ry, vx, vy);
+                    approach = dot < 0.0;
+                }
+                sm.x[slot] = rx;
+                sm.y[slot] = ry;
+                sm.e[slot] = dot;
+            }
+            const uint32_t bal = __ballot_sync(0xffffffffu, approach);
+            const int before = __popc(bal & lanemask_lt());
+            if (i < npair) sm.list[approach ? nlist + before : npair - 1 - (nrest + lane - before)] = (uint16_t)i;
+            nlist += __popc(bal);
+            nrest = min(i0 + 32, npair) - nlist;
         }
         __syncwarp();
-        double ax = 0.0, ay = 0.0, ed = 0.0;  // (three lanes per particle: ax alone, lane 3 p + component)
-        for (int c = 0, e_lo = k; c < ch.n; c++) {
-            const int ce = ch.len(c), st = pair_stride(ce), magic = (65535 + ce) / ce, npair = np * ce;
-            e_lo -= ce;
-            // ---- A
-            int nlist = 0, nrest = 0;
-            // a round's loads are issued a round (the neighbour's data) or two (its
-            // code) before their use
-            auto entry = [&](int i) {
-                const int p = pair_row(i, magic);
-                return p * k + e_lo + (i - p * ce);
-            };
-            uint32_t code1 = lane < npair ? (uint32_t)nb[entry(lane)] : 0u;
-            uint32_t code2 = lane + 32 < npair ? (uint32_t)nb[entry(lane + 32)] : 0u;
-            double2 V1 = B.vp[code1 >> kCodeShift], Q1 = B.pos[code1 >> kCodeShift];
-            for (int i0 = 0; i0 < npair; i0 += 32) {
-                const int i = i0 + lane;
-                bool approach = false;
-                const uint32_t code = code1;
-                const double2 V = V1, Q = Q1;
-                code1 = code2;
-                V1 = B.vp[code1 >> kCodeShift];
-                Q1 = B.pos[code1 >> kCodeShift];
-                code2 = i + 64 < npair ? (uint32_t)nb[entry(i + 64)] : 0u;
-                if (i < npair) {
-                    const int p = pair_row(i, magic), slot = i + p * (st - ce);
-                    const ForceRow &R = sm.row[p];
-                    const double vx = __dsub_rn(V.x, R.vx), vy = __dsub_rn(V.y, R.vy);
-                    double qx = Q.x, qy = Q.y;
-                    if ((code & 15u) != 4u) {
-                        double ox, oy;
-                        img_shift(a.c.sims[sim_of(a.c, q0 + p)], code & 15u, ox, oy);
-                        qx = __dsub_rn(qx, ox);
-                        qy = __dsub_rn(qy, oy);
-                    }
-                    const double rx = __dsub_rn(qx, R.x), ry = __dsub_rn(qy, R.y);
-                    double dot;
-                    if (emu_within<150>(rx) && emu_within<150>(ry) && emu_within<150>(vx) && emu_within<150>(vy)) {
-                        dot = __dadd_rn(emu_mul_n(vx, rx), emu_mul_n(vy, ry));  // 0, or 2^-353 at least (no subnormal)
-                        approach = emu_hi(dot) > 0x80000000u;
-                    } else {
-                        dot = force_dot_slow(rx, ry, vx, vy);
-                        approach = dot < 0.0;
-                    }
-                    sm.x[slot] = rx;
-                    sm.y[slot] = ry;
-                    sm.e[slot] = dot;
-                }
-                const uint32_t bal = __ballot_sync(0xffffffffu, approach);
-                const int before = __popc(bal & lanemask_lt());
-                if (i < npair) sm.list[approach ? nlist + before : npair - 1 - (nrest + lane - before)] = (uint16_t)i;
-                nlist += __popc(bal);
-                nrest = min(i0 + 32, npair) - nlist;
+        // ---- B, the approaching pairs first: one round at most holds both kinds
+        int at = lane < npair ? entry(sm.list[lane]) : 0;
+        double2 dd1 = dist[at];  // (NNDists, dF)
+        const double4 *der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);  // (c, rho, h, c^2 / (gamma rho))
+        double c1 = 0.0, rho1 = 0.0, h1 = 0.0, ct1 = der1->w;
+        if (lane < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
+        for (int n = lane; n < npair; n += 32) {
+            const double2 dd = dd1;
+            const double cj = c1, rhoj = rho1, hj = h1, ctj = ct1;
+            if (n + 32 < npair) {
+                at = entry(sm.list[n + 32]);
+                dd1 = dist[at];
+                der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);
+                ct1 = der1->w;
+                if (n + 32 < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
             }
-            __syncwarp();
-            // ---- B, the approaching pairs first: one round at most holds both kinds
-            int at = lane < npair ? entry(sm.list[lane]) : 0;
-            double2 dd1 = dist[at];  // (NNDists, dF)
-            const double4 *der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);  // (c, rho, h, c^2 / (gamma rho))
-            double c1 = 0.0, rho1 = 0.0, h1 = 0.0, ct1 = der1->w;
-            if (lane < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
-            for (int n = lane; n < npair; n += 32) {
-                const double2 dd = dd1;
-                const double cj = c1, rhoj = rho1, hj = h1, ctj = ct1;
-                if (n + 32 < npair) {
-                    at = entry(sm.list[n + 32]);
-                    dd1 = dist[at];
-                    der1 = D.der + ((uint32_t)nb[at] >> kCodeShift);
-                    ct1 = der1->w;
-                    if (n + 32 < nlist) { c1 = der1->x; rho1 = der1->y; h1 = der1->z; }
+            const int i = sm.list[n], p = pair_row(i, magic), slot = i + p * (st - ce);
+            const ForceRow &R = sm.row[p];
+            const double rx = sm.x[slot], ry = sm.y[slot], dot = sm.e[slot];
+            const bool in_r = emu_within<150>(rx) && emu_within<150>(ry);
+            double sum = R.cterm;  // Pi + cA (0 + cA = cA)
+            if (n < nlist) {
+                const SimDev &S = a.c.sims[sim_of(a.c, q0 + p)];
+                const double alpha = S.alpha, beta = S.beta;
+                const double c2 = __dadd_rn(R.c, cj), rho2 = __dadd_rn(R.rho, rhoj), h2 = __dadd_rn(R.h, hj);
+                bool ok = in_r && emu_within<400>(dot) && emu_within<150>(c2) && emu_within<150>(rho2) &&
+                          emu_within<150>(h2) && emu_within<150>(alpha) && emu_within<150>(beta);
+                double pi = 0.0;
+                if (ok) {
+                    const double den = __dadd_rn(__dadd_rn(emu_mul_n(rx, rx), emu_mul_n(ry, ry)), S.etasq);
+                    const double mu = emu_div_n(emu_mul_n(dot, emu_halve(h2)), emu_divisor(den));
+                    const double num = __dadd_rn(emu_mul_n(emu_mul_n(emu_neg(alpha), emu_halve(c2)), mu),
+                                                 emu_mul_n(emu_mul_n(beta, mu), mu));
+                    pi = emu_div_n(num, emu_divisor(emu_halve(rho2)));
+                    ok = emu_within<300>(den) && emu_within<300>(mu) && emu_within<800>(num);
                 }
-                const int i = sm.list[n], p = pair_row(i, magic), slot = i + p * (st - ce);
-                const ForceRow &R = sm.row[p];
-                const double rx = sm.x[slot], ry = sm.y[slot], dot = sm.e[slot];
-                const bool in_r = emu_within<150>(rx) && emu_within<150>(ry);
-                double sum = R.cterm;  // Pi + cA (0 + cA = cA)
-                if (n < nlist) {
-                    const SimDev &S = a.c.sims[sim_of(a.c, q0 + p)];
-                    const double alpha = S.alpha, beta = S.beta;
-                    const double c2 = __dadd_rn(R.c, cj), rho2 = __dadd_rn(R.rho, rhoj), h2 = __dadd_rn(R.h, hj);
-                    bool ok = in_r && emu_within<400>(dot) && emu_within<150>(c2) && emu_within<150>(rho2) &&
-                              emu_within<150>(h2) && emu_within<150>(alpha) && emu_within<150>(beta);
-                    double pi = 0.0;
-                    if (ok) {
-                        const double den = __dadd_rn(__dadd_rn(emu_mul_n(rx, rx), emu_mul_n(ry, ry)), S.etasq);
-                        const double mu = emu_div_n(emu_mul_n(dot, emu_halve(h2)), emu_divisor(den));
-                        const double num = __dadd_rn(emu_mul_n(emu_mul_n(emu_neg(alpha), emu_halve(c2)), mu),
-                                                     emu_mul_n(emu_mul_n(beta, mu), mu));
-                        pi = emu_div_n(num, emu_divisor(emu_halve(rho2)));
-                        ok = emu_within<300>(den) && emu_within<300>(mu) && emu_within<800>(num);
-                    }
-                    if (!ok) pi = force_pi_slow(rx, ry, dot, c2, rho2, h2, alpha, beta, S.etasq);
-                    sum = __dadd_rn(pi, sum);
-                }
-                // the terms r_AB (Pi + cA + cB) dF / NNDists and v_AB . r_AB dF
-                sum = __dadd_rn(sum, ctj);
-                const double d = dd.x, drk = dd.y;
-                // a zero dF (always so for the farthest neighbour) makes zero terms, whose
-                // signs do not matter to the sums, which are never -0
-                const bool dz = emu_is_zero(drk), dot0 = emu_is_zero(dot);
-                ForceTerms t;
-                if (in_r && emu_within<150>(sum) && emu_within<150>(d) && (dz || emu_within<150>(drk)) &&
-                    (emu_within<400>(dot) || dot0)) {
-                    const EmuDivisor dv = emu_divisor(d);  // shared by both quotients
-                    t.x = emu_div_n(emu_mul_n(emu_mul_n(rx, sum), drk), dv);
-                    t.y = emu_div_n(emu_mul_n(emu_mul_n(ry, sum), drk), dv);
-                    t.e = emu_mul_n(dot, drk);
-                    if (dz) t.x = t.y = 0.0;
-                    if (dz || dot0) t.e = 0.0;
-                } else {
-                    t = force_terms_slow(rx, ry, dot, sum, drk, d);
-                }
-                sm.x[slot] = t.x;
-                sm.y[slot] = t.y;
-                sm.e[slot] = t.e;
+                if (!ok) pi = force_pi_slow(rx, ry, dot, c2, rho2, h2, alpha, beta, S.etasq);
+                sum = __dadd_rn(pi, sum);
             }
-            __syncwarp();
-            // ---- C
-            if (W <= kSplitWidth) {
-                if (lane < 3 * np) {
-                    const int p = lane / 3, comp = lane - 3 * p;
-                    const double *t = (comp == 0 ? sm.x : comp == 1 ? sm.y : sm.e) + p * st;
-                    for (int e = ce - 1; e >= 0; e--) ax = __dadd_rn(ax, t[e]);
-                }
-            } else if (lane < np) {
-                const int t = lane * st;
-                for (int e = ce - 1; e >= 0; e--) {
-                    ax = __dadd_rn(ax, sm.x[t + e]);
-                    ay = __dadd_rn(ay, sm.y[t + e]);
-                    ed = __dadd_rn(ed, sm.e[t + e]);
-                }
+            // the terms r_AB (Pi + cA + cB) dF / NNDists and v_AB . r_AB dF
+            sum = __dadd_rn(sum, ctj);
+            const double d = dd.x, drk = dd.y;
+            // a zero dF (always so for the farthest neighbour) makes zero terms, whose
+            // signs do not matter to the sums, which are never -0
+            const bool dz = emu_is_zero(drk), dot0 = emu_is_zero(dot);
+            ForceTerms t;
+            if (in_r && emu_within<150>(sum) && emu_within<150>(d) && (dz || emu_within<150>(drk)) &&
+                (emu_within<400>(dot) || dot0)) {
+                const EmuDivisor dv = emu_divisor(d);  // shared by both quotients
+                t.x = emu_div_n(emu_mul_n(emu_mul_n(rx, sum), drk), dv);
+                t.y = emu_div_n(emu_mul_n(emu_mul_n(ry, sum), drk), dv);
+                t.e = emu_mul_n(dot, drk);
+                if (dz) t.x = t.y = 0.0;
+                if (dz || dot0) t.e = 0.0;
+            } else {
+                t = force_terms_slow(rx, ry, dot, sum, drk, d);
             }
-            __syncwarp();
+            sm.x[slot] = t.x;
+            sm.y[slot] = t.y;
+            sm.e[slot] = t.e;
         }
+        __syncwarp();
+        // ---- C
         if (W <= kSplitWidth) {
-            const double s = ax;
-            const int l3 = min(3 * lane, 29);
-            ax = __shfl_sync(0xffffffffu, s, l3);
-            ay = __shfl_sync(0xffffffffu, s, l3 + 1);
-            ed = __shfl_sync(0xffffffffu, s, l3 + 2);
-        }
-        if (lane < np) {
-            const int64_t q = q0 + lane;
-            const ForceRow &R = sm.row[lane];
-            const SimDev &S = a.c.sims[sim_of(a.c, q)];
-            const double hi = R.h;
-            const double h3 = emu_mul(emu_mul(hi, hi), hi);
-            const double f = emu_div(emu_mul(S.mass, S.dfpref), emu_divisor(h3), h3);
-            const double axo = __dadd_rn(emu_mul(ax, f), S.accel[0]);
-            const double ayo = __dadd_rn(emu_mul(ay, f), S.accel[1]);
-            const double edot = emu_mul(emu_mul(R.cterm, ed), S.mass);
-            if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
-            double2 pos = make_double2(R.x, R.y), vel = B.vel[q];
-            double u = B.u[q];
-            if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
-            a.A.pos[q] = pos;
-            a.A.vel[q] = vel;
-            a.A.u[q] = u;
-            a.A.acc[q] = make_double2(axo, ayo);
-            a.A.udot[q] = edot;
-            a.A.id[q] = B.id[q];
-            a.A.hprev[q] = (float)hi;
-            a.A.vp[q] = make_double2(R.vx, R.vy);
-            a.A.up[q] = B.up[q];
+            if (lane < 3 * np) {
+                const int p = lane / 3, comp = lane - 3 * p;
+                const double *t = (comp == 0 ? sm.x : comp == 1 ? sm.y : sm.e) + p * st;
+                for (int e = ce - 1; e >= 0; e--) ax = __dadd_rn(ax, t[e]);
+            }
+        } else if (lane < np) {
+            const int t = lane * st;
+            for (int e = ce - 1; e >= 0; e--) {
+                ax = __dadd_rn(ax, sm.x[t + e]);
+                ay = __dadd_rn(ay, sm.y[t + e]);
+                ed = __dadd_rn(ed, sm.e[t + e]);
+            }
         }
         __syncwarp();
     }
+    if (W <= kSplitWidth) {
+        const double s = ax;
+        const int l3 = min(3 * lane, 29);
+        ax = __shfl_sync(0xffffffffu, s, l3);
+        ay = __shfl_sync(0xffffffffu, s, l3 + 1);
+        ed = __shfl_sync(0xffffffffu, s, l3 + 2);
+    }
+    if (lane < np) {
+        const int64_t q = q0 + lane;
+        const ForceRow &R = sm.row[lane];
+        const SimDev &S = a.c.sims[sim_of(a.c, q)];
+        const double hi = R.h;
+        const double h3 = emu_mul(emu_mul(hi, hi), hi);
+        const double f = emu_div(emu_mul(S.mass, S.dfpref), emu_divisor(h3), h3);
+        const double axo = __dadd_rn(emu_mul(ax, f), S.accel[0]);
+        const double ayo = __dadd_rn(emu_mul(ay, f), S.accel[1]);
+        const double edot = emu_mul(emu_mul(R.cterm, ed), S.mass);
+        if (!is_finite(axo) || !is_finite(ayo) || !is_finite(edot)) fl |= FLAG_Q_RANGE;
+        double2 pos = make_double2(R.x, R.y), vel = B.vel[q];
+        double u = B.u[q];
+        if (a.integrate) integrate_one(S, pos, vel, u, axo, ayo, edot);
+        a.A.pos[q] = pos;
+        a.A.vel[q] = vel;
+        a.A.u[q] = u;
+        a.A.acc[q] = make_double2(axo, ayo);
+        a.A.udot[q] = edot;
+        a.A.id[q] = B.id[q];
+        a.A.hprev[q] = (float)hi;
+        a.A.vp[q] = make_double2(R.vx, R.vy);
+        a.A.up[q] = B.up[q];
+    }
     if (fl) atomicOr(a.c.flags, fl);
-}
-
-constexpr size_t kForceSmem = kPairWarps * sizeof(ForceWarp);
-static int g_force_blocks;  // resident blocks per SM (set before any capture)
-
-// Sets the shared-memory limit of the FP64 force kernel and records its
-// occupancy; must run before any stream capture.
-void force_init_attrs() {
-    cudaFuncSetAttribute(k_force_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForceSmem);
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64, kPairWarps * 32, kForceSmem);
-    g_force_blocks = std::max(nb, 1);
 }
 
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
@@ -570,22 +555,21 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
     a.D = D;
     a.integrate = integrate ? 1 : 0;
     if (mode != MODE_MIXED) {
-        const int nb = std::max(g_force_blocks, 1);
-        const int W = pair_width(c.n, (int64_t)L.sms * nb * kPairWarps);
-        const int64_t tiles = (c.n + W - 1) / W;
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((tiles + kPairWarps - 1) / kPairWarps, (int64_t)L.sms * nb));
-        k_force_fp64<<<grid, kPairWarps * 32, kForceSmem, L.stream>>>(a, W);
+        static const int per_sm = [] {
+            int nb = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64, 32, 0);
+            return std::max(nb, 1);
+        }();
+        const PairTiles t(c.n, (int64_t)L.sms * per_sm);
+        k_force_fp64<<<t.grid(), 32, 0, L.stream>>>(a, t);
         return;
     }
     if (c.n <= kMixedPairsMaxN) {
-        const int W = pair_width(c.n, (int64_t)L.sms * kMixedBlocks * kPairWarps);
-        const int64_t tiles = (c.n + W - 1) / W;
-        const int grid = (int)std::max<int64_t>(1, (tiles + kPairWarps - 1) / kPairWarps);
-        k_force_mixed_pairs<<<grid, kPairWarps * 32, 0, L.stream>>>(a, W);
+        const PairTiles t(c.n, (int64_t)L.sms * kMixedBlocks);
+        k_force_mixed_pairs<<<t.grid(), 32, 0, L.stream>>>(a, t);
         return;
     }
-    const int64_t need = (c.n + 127) / 128;
-    k_force_mixed<<<(int)std::min<int64_t>(need, (int64_t)L.sms * 16), 128, 0, L.stream>>>(a);
+    k_force_mixed<<<(int)((c.n + 127) / 128), 128, 0, L.stream>>>(a);
 }
 
 // ------------------------------------------------------------ error norms

@@ -19,7 +19,6 @@
 
 namespace sphgpu {
 
-constexpr int kPairWarps = 4;    // warps per block (each works alone)
 constexpr int kPairSlots = 288;  // terms a warp's tile holds: W (chunk | 1) at most
 
 // A row of ce terms is kept at an odd stride (in doubles), so that the lanes
@@ -38,16 +37,28 @@ constexpr bool pair_rows_fit() {
 }
 static_assert(pair_rows_fit(), "a tile's terms fit its slots at every width");
 
-// Particles per tile for n particles on the warps the GPU holds at once: equal
-// shares in one pass; or in two when full tiles would leave less than an
-// eighth of a pass over (force stage at N = 100,000, 1.03 passes: 148 us at 17
-// particles, 168 at 32); else full tiles, whose lanes are all at work in the
-// ordered sums (density stage at N = 200,001, 1.28 passes: 157 us at 32, 171
-// at 21).
-inline int pair_width(int64_t n, int64_t resident_warps) {
-    const int64_t passes = n <= 32 * resident_warps ? 1 : n <= 36 * resident_warps ? 2 : 0;
-    return passes ? (int)((n + resident_warps * passes - 1) / (resident_warps * passes)) : 32;
-}
+// The tiles of n particles on a GPU that holds `resident` warps at once: as
+// many full passes of 32 particles a warp as there are, and the rest in equal
+// shares, one per resident warp. A tile is a block of one warp, so that the
+// next tile starts as soon as a warp is free; with a resident block for every
+// slot striding over the tiles, a pass of which a few warps had one tile more
+// than the others left the rest idle.
+struct PairTiles {
+    int64_t full;  // tiles of 32 particles, first
+    int W;         // width of the others
+    int64_t n;
+    PairTiles(int64_t n_, int64_t resident) : n(n_) {
+        full = n / (32 * resident) * resident;
+        W = (int)((n - 32 * full + resident - 1) / resident);
+        if (W < 1) W = 1;
+    }
+    int grid() const { return (int)(full + (n - 32 * full + W - 1) / W); }
+    // first particle of tile t, and its width
+    __device__ __forceinline__ int64_t first(int64_t t, int &w) const {
+        w = t < full ? 32 : W;
+        return t < full ? 32 * t : 32 * full + (t - full) * W;
+    }
+};
 
 // Chunk c = 0, 1, ... of a list of k entries, farthest first: entries
 // [lo, lo + ce); the chunks' lengths differ by at most one.
