@@ -41,6 +41,8 @@ struct alignas(16) DensityRow {
     int32_t sim;
 };
 
+static_assert(pair_rows_fit(kPairSlots), "a tile's terms fit its slots at every width");
+
 struct DensityWarp {
     DensityRow row[32];
     double term[kPairSlots];   // F(q) of the chunk's pairs (q itself for those waiting in near)
@@ -94,7 +96,7 @@ __global__ void __launch_bounds__(32, 32) k_density_fp64(DensityArgs a) {
     const PArrays &B = a.B;
     int W;
     const int64_t q0 = a.tiles.first(blockIdx.x, W);
-    const PairChunks ch(k, W);
+    const PairChunks ch(k, W, kPairSlots);
     unsigned fl = 0;
     const int np = (int)min((int64_t)W, a.c.n - q0);
     const int32_t *nb = a.D.nbr + q0 * k;

@@ -16,9 +16,19 @@ namespace sphgpu {
 // the factors' way through shared memory costs issue slots).
 constexpr int64_t kMixedPairsMaxN = 16384;
 constexpr int kMixedBlocks = 20;  // resident blocks (warps) per SM (8 KB each)
-// Blocks (warps) of the FP64 force per SM asked of the compiler: 92 registers,
-// 9.5 KB, 21 resident.
-constexpr int kForceBlocks = 20;
+// The FP64 force is compiled twice: with 92 registers and chunks of nine entries
+// at 32 particles, 21 warps resident per SM, and with 72 and seven, 25 resident.
+// The second hides more latency over many passes, but each of its warps takes
+// longer and a short run ends later: beyond two passes of the first (force
+// stage, us, first and second: N = 50,000 81 and 86, 100,000 133 and 140,
+// 120,000 150 and 161, 150,000 194 and 178, 200,001 333 and 349, 250,000 303
+// and 290, 300,000 338 and 330, 500,000 544 and 533, 1,048,576 1103 and 1034,
+// clustered 4,194,304 4262 and 4040; k = 16 and 64 at 250,000 164 and 159, 599
+// and 580). 192 slots at 26 warps 1080 and 4112, 160 at 30 (64 registers,
+// spills) 1103 and 4203.
+constexpr int kForceBlocks = 20, kForceBlocksMany = 25;
+constexpr int kForceSlotsMany = 224;
+constexpr int kForceWidePasses = 2;
 // Tiles up to this width sum with three lanes per particle: 29 us at N = 10,000
 // against 40 with one.
 constexpr int kSplitWidth = 10;
@@ -177,7 +187,7 @@ __global__ void __launch_bounds__(32, kMixedBlocks) k_force_mixed_pairs(ForceArg
     const int64_t q0 = tiles.first(blockIdx.x, W);
     const PArrays &B = a.B;
     const Derived &D = a.D;
-    const PairChunks ch(k, W);
+    const PairChunks ch(k, W, kPairSlots);
     unsigned fl = 0;
     const int np = (int)min((int64_t)W, a.c.n - q0);
     const int32_t *nb = D.nbr + q0 * k;
@@ -303,8 +313,8 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
 // infinities and NaNs) take the hardware's arithmetic out of line. Every
 // operation and its order are the reference's, so the results stay bit-exact.
 //
-// Bound (ncu, uniform blast N = 1,048,576, k = 32): FP64 pipe 67 %, ALU 52 %,
-// issue 60 % busy; moving work either way between the two pipes (the sums
+// Bound (ncu, uniform blast N = 1,048,576, k = 32): FP64 pipe 72 %, ALU 57 %,
+// issue 67 % busy; moving work either way between the two pipes (the sums
 // cA + cB, hA + hB, rhoA + rhoB on the integer pipe, the dot product or r^2 on
 // the FP64 unit) changed nothing or cost up to 5 %. The loads are issued a
 // round early: 1335 -> 1231 us; one loop for both kinds of pairs instead of
@@ -313,18 +323,20 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
 // Against one warp per 32 particles, a lane each, with the approaching pairs
 // compacted per warp (force stage, us): N = 1000 112 -> 14, 10,000 154 -> 29,
 // 100,000 297 -> 133 (149 with resident blocks of four warps striding over
-// tiles of one width), 1,048,576 1750 -> 1103 (1165), clustered 4,194,304
-// 6800 -> 4262 (4540), stress 2,000,003 (k = 64) 6370 -> 4004 (4210).
+// tiles of one width), 1,048,576 1750 -> 1034 (1165), clustered 4,194,304
+// 6800 -> 4040 (4540), stress 2,000,003 (k = 64) 6370 -> 3843 (4210).
 struct ForceRow {
     double x, y, vx, vy;      // position and predicted velocity
     double c, rho, h, cterm;  // sound speed, density, smoothing length, c^2 / (gamma rho)
 };
 
+template <int SLOTS>
 struct ForceWarp {
-    double x[kPairSlots], y[kPairSlots];  // r_AB, then the acceleration terms
-    double e[kPairSlots];                 // v_AB . r_AB, then the du/dt terms
+    static_assert(pair_rows_fit(SLOTS), "a tile's terms fit its slots at every width");
+    double x[SLOTS], y[SLOTS];  // r_AB, then the acceleration terms
+    double e[SLOTS];            // v_AB . r_AB, then the du/dt terms
     ForceRow row[32];
-    uint16_t list[kPairSlots];            // approaching pairs from the front, the others from the back
+    uint16_t list[SLOTS];       // approaching pairs from the front, the others from the back
 };
 
 struct Vec2D {
@@ -357,14 +369,15 @@ __device__ __noinline__ ForceTerms force_terms_slow(double rx, double ry, double
 
 __device__ __forceinline__ double emu_halve(double x) { return emu_double(emu_bits(x) - (1ull << 52)); }
 
-__global__ void __launch_bounds__(32, kForceBlocks) k_force_fp64(ForceArgs a, PairTiles tiles) {
-    __shared__ ForceWarp sm;
+template <int SLOTS, int BLOCKS>
+__global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTiles tiles) {
+    __shared__ ForceWarp<SLOTS> sm;
     const int k = a.c.k, lane = threadIdx.x;
     int W;
     const int64_t q0 = tiles.first(blockIdx.x, W);
     const PArrays &B = a.B;
     const Derived &D = a.D;
-    const PairChunks ch(k, W);
+    const PairChunks ch(k, W, SLOTS);
     unsigned fl = 0;
     const int np = (int)min((int64_t)W, a.c.n - q0);
     const int32_t *nb = D.nbr + q0 * k;
@@ -546,6 +559,23 @@ __global__ void __launch_bounds__(32, kForceBlocks) k_force_fp64(ForceArgs a, Pa
     if (fl) atomicOr(a.c.flags, fl);
 }
 
+// resident blocks (warps) per SM of a form of the FP64 force
+template <int SLOTS, int BLOCKS>
+static int force_blocks() {
+    static const int per_sm = [] {
+        int nb = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64<SLOTS, BLOCKS>, 32, 0);
+        return std::max(nb, 1);
+    }();
+    return per_sm;
+}
+
+template <int SLOTS, int BLOCKS>
+static void launch_force_fp64(const ForceArgs &a, const Launch &L) {
+    const PairTiles t(a.c.n, (int64_t)L.sms * force_blocks<SLOTS, BLOCKS>());
+    k_force_fp64<SLOTS, BLOCKS><<<t.grid(), 32, 0, L.stream>>>(a, t);
+}
+
 void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays &A,
                   const Derived &D, int mode, bool integrate) {
     ForceArgs a;
@@ -555,13 +585,9 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
     a.D = D;
     a.integrate = integrate ? 1 : 0;
     if (mode != MODE_MIXED) {
-        static const int per_sm = [] {
-            int nb = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_force_fp64, 32, 0);
-            return std::max(nb, 1);
-        }();
-        const PairTiles t(c.n, (int64_t)L.sms * per_sm);
-        k_force_fp64<<<t.grid(), 32, 0, L.stream>>>(a, t);
+        const bool wide = c.n <= (int64_t)kForceWidePasses * 32 * L.sms * force_blocks<kPairSlots, kForceBlocks>();
+        if (wide) launch_force_fp64<kPairSlots, kForceBlocks>(a, L);
+        else launch_force_fp64<kForceSlotsMany, kForceBlocksMany>(a, L);
         return;
     }
     if (c.n <= kMixedPairsMaxN) {

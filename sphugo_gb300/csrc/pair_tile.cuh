@@ -25,17 +25,16 @@ constexpr int kPairSlots = 288;  // terms a warp's tile holds: W (chunk | 1) at 
 // of the ordered sums, one row each, meet every bank pair once.
 __host__ __device__ constexpr int pair_stride(int ce) { return ce | 1; }
 // Entries per chunk at tile width W: the most, up to 32, whose rows fit.
-__host__ __device__ constexpr int pair_chunk(int W) {
-    const int t = kPairSlots / W, c = t & 1 ? t : t - 1;
+__host__ __device__ constexpr int pair_chunk(int W, int slots) {
+    const int t = slots / W, c = t & 1 ? t : t - 1;
     return c < 32 ? c : 32;
 }
-constexpr bool pair_rows_fit() {
+constexpr bool pair_rows_fit(int slots) {
     for (int W = 1; W <= 32; W++)
-        for (int ce = 1; ce <= pair_chunk(W); ce++)
-            if (W * pair_stride(ce) > kPairSlots) return false;
+        for (int ce = 1; ce <= pair_chunk(W, slots); ce++)
+            if (W * pair_stride(ce) > slots) return false;
     return true;
 }
-static_assert(pair_rows_fit(), "a tile's terms fit its slots at every width");
 
 // The tiles of n particles on a GPU that holds `resident` warps at once: as
 // many full passes of 32 particles a warp as there are, and the rest in equal
@@ -64,8 +63,8 @@ struct PairTiles {
 // [lo, lo + ce); the chunks' lengths differ by at most one.
 struct PairChunks {
     int n, base, extra;  // chunks; shortest length; how many are one longer
-    __device__ __forceinline__ PairChunks(int k, int W) {
-        n = (k + pair_chunk(W) - 1) / pair_chunk(W);
+    __device__ __forceinline__ PairChunks(int k, int W, int slots) {
+        n = (k + pair_chunk(W, slots) - 1) / pair_chunk(W, slots);
         base = k / n;
         extra = k - base * n;
     }
