@@ -61,10 +61,11 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 
 // d2 in units of R^2 / 2^KB (qs = 2^KB / R^2) rounded to the nearest integer,
 // clamped to KB bits: d2 qs + 2^23 lies in [2^23, 2^24), whose floats are the
-// integers, so the mantissa is the key (no conversion instruction).
+// integers, so the mantissa is the key (no conversion instruction). The
+// exponent above it is left for the caller's shift by 32 - KB bits to drop.
 template <int KB>
 __device__ __forceinline__ uint32_t key_of(float d2, float qs) {
-    return min(__float_as_uint(__fmaf_rn(d2, qs, 8388608.f)) - 0x4B000000u, (1u << KB) - 1u);
+    return min(__float_as_uint(__fmaf_rn(d2, qs, 8388608.f)), 0x4B000000u + (1u << KB) - 1u);
 }
 
 // The G largest of A keys (A a multiple of G, G a power of two): A / G
@@ -502,7 +503,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                         const float dx = cc[u].x - rqx, dy = cc[u].y - rqy;
                         const float d2 = __fmaf_rn(dx, dx, dy * dy);
                         const bool pass = d2 <= R2 && t + u != myself && t + u < e;
-                        mylist[min(cnt, LCAP)][lane] = (key_of<KB>(d2, qs) << SB) | (uint32_t)(t + u);
+                        mylist[min(cnt, LCAP)][lane] = (key_of<KB>(d2, qs) << SB) + (uint32_t)(t + u);
                         cnt += pass ? 1 : 0;
                     }
                     t += 4;
@@ -597,6 +598,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                 // reference's rounding, then the FP32 kernel sum over the
                 // squared distances written here, which then need not be stored
                 const bool fuse = a.fuse_density != 0;
+                const int kernel = S.kernel;
                 double hq = 0.0;
                 float inv_hf = 0.f;
                 if (fuse) {
@@ -623,7 +625,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
                     out4[c] = make_int4((int)cd[0], (int)cd[1], (int)cd[2], (int)cd[3]);
                     if (fuse) {
 #pragma unroll
-                        for (int u = 3; u >= 0; u--) acc.add(kf_f32(S.kernel, fminf(sqrtf(dd[u]) * inv_hf, 1.f)));
+                        for (int u = 3; u >= 0; u--) acc.add(kf_f32(kernel, fminf(sqrtf(dd[u]) * inv_hf, 1.f)));
                     } else {
                         o24[c] = make_float4(dd[0], dd[1], dd[2], dd[3]);
                     }
