@@ -302,7 +302,7 @@ void enqueue_eval(sph_handle *h, int pred, bool integrate, bool events = false) 
     };
     mark(0);
     if (h->any_open) launch_bbox(c, L, h->A, pred);
-    launch_bin(c, L, h->A, h->T, pred);
+    launch_bin(c, L, h->A, h->T, h->D.ndefer, pred);
     mark(1);
     launch_scan(c, L, h->T);
     mark(2);

@@ -235,7 +235,7 @@ struct Launch {
 };
 
 void launch_bbox(const Ctx &c, const Launch &L, const PArrays &A, int pred);  // and the grids of open axes
-void launch_bin(const Ctx &c, const Launch &L, const PArrays &A, const Tables &T, int pred);
+void launch_bin(const Ctx &c, const Launch &L, const PArrays &A, const Tables &T, int32_t *ndefer, int pred);
 void launch_scan(const Ctx &c, const Launch &L, const Tables &T);
 void launch_permute(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
                     const Tables &T, int pred, bool velrec);

@@ -1219,7 +1219,6 @@ static void launch_knn_nr(const KnnArgs &args, const Launch &L, const KnnTune &t
     const int resident = L.sms * std::max(tune.blocks_per_sm, 1);
     if (tune.tile && args.D.defer) {
         // group tiles, then the per-query kernel over the deferred queries
-        cudaMemsetAsync(args.D.ndefer, 0, 2 * sizeof(int32_t), L.stream);
         KnnArgs b = args;
         b.rerank = MODE != MODE_MIXED && args.c.k <= kRerankMaxK ? 1 : 0;
         if (tune.block_warps > 0 && launch_knn_block(b, L, MODE, NR, tune.block_warps)) {

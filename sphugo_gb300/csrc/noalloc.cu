@@ -221,7 +221,7 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     k_noalloc_init<<<1, 1, 0, st>>>(S, d_sims, d_offs, d_flags);
     launch_scatter_state(c, L, A, nullptr, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
     if (any_open) launch_bbox(c, L, A, PRED_INIT);
-    launch_bin(c, L, A, T, PRED_INIT);
+    launch_bin(c, L, A, T, nullptr, PRED_INIT);
     launch_scan(c, L, T);
     launch_permute(c, L, A, B, T, PRED_INIT, false);
     launch_knn(c, L, B, D, T, MODE_EXACT64, tune);
