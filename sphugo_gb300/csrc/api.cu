@@ -899,8 +899,8 @@ int sph_get_neighbours(sph_handle *h, int64_t *ids, double *dist, int32_t *img) 
     int64_t *di = (int64_t *)h->d_nbr_io;
     double *dd = (double *)(di + nk);
     int32_t *dm = (int32_t *)(dd + nk);
-    launch_gather_neighbours(h->ctx(), h->launch(), h->A, h->B, h->D, ids ? di : nullptr,
-                             dist ? dd : nullptr, img ? dm : nullptr, h->mode == MODE_EXACT64);
+    launch_gather_neighbours(h->ctx(), h->launch(), h->B, h->D, ids ? di : nullptr, dist ? dd : nullptr,
+                             img ? dm : nullptr);
     CUDA_TRY(cudaGetLastError());
     if (ids) CUDA_TRY(cudaMemcpyAsync(ids, di, nk * 8, cudaMemcpyDeviceToHost, h->stream));
     if (dist) CUDA_TRY(cudaMemcpyAsync(dist, dd, nk * 8, cudaMemcpyDeviceToHost, h->stream));

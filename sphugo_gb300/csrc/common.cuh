@@ -272,8 +272,8 @@ void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const
 void launch_append(const Launch &L, const PArrays &A, int64_t n0, int64_t count, const double *buf);
 void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D, const int32_t *slot,
                            double *rho, double *cs, double *h);
-void launch_gather_neighbours(const Ctx &c, const Launch &L, const PArrays &A, const PArrays &B,
-                              const Derived &D, int64_t *ids, double *dist, int32_t *img, bool exact_stored);
+void launch_gather_neighbours(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int64_t *ids,
+                              double *dist, int32_t *img, double *rho = nullptr, double *h = nullptr);
 void launch_diagnostics(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D,
                         int64_t lo, int64_t hi, double *scratch);
 int knn_occupancy_blocks(int block, int cap, int mode);

@@ -122,51 +122,96 @@ void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, cons
 // Reference layout: slot 0 = farthest (sim/nearest-neighbour.go:139-153 keeps
 // NNDists descending); dist = sqrt of the reference's squared distance. Lists
 // are re-sorted here by (squared distance, particle id, image code): the
-// mixed form stores its neighbour set unordered.
-constexpr int kMaxK = 128;
-
-__global__ void k_gather_nbrs(Ctx c, PArrays B, Derived D, int64_t *ids, double *dist, int32_t *img) {
-    const int k = c.k;
-    GRID_STRIDE(i, c.n) {
-        const int s = sim_of(c, i);
-        const SimDev &S = c.sims[s];
+// mixed form stores its neighbour set unordered. A warp per query, E
+// consecutive entries per lane (k <= 32 E): the keys of the list in one round,
+// then odd-even transposition until nothing moves, one round for the lists
+// that the FP64 forms leave in order. A NaN distance moves nothing past it. One
+// thread per query, with an insertion sort in local memory, took 35 us at
+// N = 4096, k = 32; this form 6.
+template <int E>
+__global__ void __launch_bounds__(256) k_gather_nbrs(Ctx c, PArrays B, Derived D, int64_t *ids, double *dist, int32_t *img,
+                                                     double *rho, double *h) {
+    const int k = c.k, lane = threadIdx.x & 31;
+    for (int64_t i = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); i < c.n;
+         i += (int64_t)gridDim.x * (blockDim.x >> 5)) {
+        const SimDev &S = c.sims[sim_of(c, i)];
         const int64_t idq = B.id[i];
         const double2 P = B.pos[i];
-        double d2[kMaxK];
-        uint32_t cd[kMaxK];
-        for (int e = 0; e < k; e++) {
-            const uint32_t code = (uint32_t)D.nbr[i * k + e];
-            double ox, oy;
-            img_shift(S, code & 15u, ox, oy);
-            const double2 Q = B.pos[code >> kCodeShift];
-            const double v = dist_sq_ref(P.x, P.y, ox, oy, Q.x, Q.y);
-            int f = e - 1;
-            while (f >= 0) {
-                bool gt = d2[f] > v;
-                if (d2[f] == v) {
-                    const int32_t ia = B.id[cd[f] >> kCodeShift], ib = B.id[code >> kCodeShift];
-                    gt = ia != ib ? ia > ib : (cd[f] & 15u) > (code & 15u);
-                }
-                if (!gt) break;
-                d2[f + 1] = d2[f];
-                cd[f + 1] = cd[f];
-                f--;
+        uint64_t key[E], tag[E];  // squared distance; particle id and image code
+#pragma unroll
+        for (int r = 0; r < E; r++) {
+            const int e = lane * E + r;
+            key[r] = ~0ull;  // past the end: a NaN
+            tag[r] = 0ull;
+            if (e < k) {
+                const uint32_t code = (uint32_t)D.nbr[i * k + e];
+                key[r] = emu_bits(nbr_d2(S, B, P, code));
+                tag[r] = ((uint64_t)(uint32_t)B.id[code >> kCodeShift] << 4) | (code & 15u);
             }
-            d2[f + 1] = v;
-            cd[f + 1] = code;
         }
-        for (int e = 0; e < k; e++) {
-            const int64_t o = idq * k + (k - 1 - e);
-            if (ids) ids[o] = B.id[cd[e] >> kCodeShift];
-            if (img) img[o] = (int32_t)(cd[e] & 15u);
-            if (dist) dist[o] = __dsqrt_rn(d2[e]);
+        // (squared distances are not negative: their bits are in their order)
+        auto greater = [](uint64_t k0, uint64_t t0, uint64_t k1, uint64_t t1) {
+            return k0 <= 0x7ff0000000000000ull && (k0 > k1 || (k0 == k1 && t0 > t1));
+        };
+        for (bool moved = true; moved;) {
+            bool m = false;
+            auto exchange = [&](int x) {  // entries x, x + 1 of this lane
+                if (greater(key[x], tag[x], key[x + 1], tag[x + 1])) {
+                    const uint64_t ks = key[x], ts = tag[x];
+                    key[x] = key[x + 1];
+                    tag[x] = tag[x + 1];
+                    key[x + 1] = ks;
+                    tag[x + 1] = ts;
+                    m = true;
+                }
+            };
+            // this lane's last entry against the next lane's first (lanes of the
+            // given parity and their successors)
+            auto across = [&](int parity) {
+                const bool low = (lane & 1) == parity;
+                const int other = low ? min(lane + 1, 31) : max(lane - 1, 0);
+                const uint64_t mk = low ? key[E - 1] : key[0], mt = low ? tag[E - 1] : tag[0];
+                const uint64_t ok = __shfl_sync(0xffffffffu, mk, other), ot = __shfl_sync(0xffffffffu, mt, other);
+                if (other != lane && (low ? greater(mk, mt, ok, ot) : greater(ok, ot, mk, mt))) {
+                    if (low) {
+                        key[E - 1] = ok;
+                        tag[E - 1] = ot;
+                    } else {
+                        key[0] = ok;
+                        tag[0] = ot;
+                    }
+                    m = true;
+                }
+            };
+#pragma unroll
+            for (int r = 0; r + 1 < E; r += 2) exchange(r);
+#pragma unroll
+            for (int r = 1; r + 1 < E; r += 2) exchange(r);
+            across(0);
+            across(1);
+            moved = __any_sync(0xffffffffu, m);
         }
+#pragma unroll
+        for (int r = 0; r < E; r++) {
+            const int e = lane * E + r;
+            if (e < k) {
+                const int64_t o = idq * k + (k - 1 - e);
+                if (ids) ids[o] = (int64_t)(tag[r] >> 4);
+                if (img) img[o] = (int32_t)(tag[r] & 15u);
+                if (dist) dist[o] = emu_sqrt(emu_double(key[r]));
+            }
+        }
+        if (rho && lane == 0) rho[idq] = D.rho[i];
+        if (h && lane == 0) h[idq] = D.h[i];
     }
 }
 
-void launch_gather_neighbours(const Ctx &c, const Launch &L, const PArrays &, const PArrays &B,
-                              const Derived &D, int64_t *ids, double *dist, int32_t *img, bool) {
-    k_gather_nbrs<<<grid_for(L, c.n, 128), 128, 0, L.stream>>>(c, B, D, ids, dist, img);
+void launch_gather_neighbours(const Ctx &c, const Launch &L, const PArrays &B, const Derived &D, int64_t *ids,
+                              double *dist, int32_t *img, double *rho, double *h) {
+    const int grid = grid_for(L, (c.n + 7) / 8, 1);  // eight queries per block
+    if (c.k <= 32) k_gather_nbrs<1><<<grid, 256, 0, L.stream>>>(c, B, D, ids, dist, img, rho, h);
+    else if (c.k <= 64) k_gather_nbrs<2><<<grid, 256, 0, L.stream>>>(c, B, D, ids, dist, img, rho, h);
+    else k_gather_nbrs<4><<<grid, 256, 0, L.stream>>>(c, B, D, ids, dist, img, rho, h);
 }
 
 // ---- diagnostics: deterministic sums over the caller's particle order.

@@ -78,12 +78,28 @@ void carve_parrays(Carve &c, PArrays &P) {
     P.vrec = nullptr;
 }
 
-// writes the simulation constants, offsets and the error word into scratch
-__global__ void k_noalloc_init(SimDev S, SimDev *sims, int64_t *offs, unsigned *flags) {
-    sims[0] = S;
-    offs[0] = 0;
-    offs[1] = S.n;
-    flags[0] = flags[1] = 0u;
+// Writes the simulation constants, offsets and the error word into scratch,
+// clears the cell table (the scratch keeps the previous call's contents) and
+// sets the particles, at rest, in the caller's order: one launch where a memset
+// and two kernels took three.
+__global__ void __launch_bounds__(256) k_noalloc_init(SimDev S, SimDev *sims, int64_t *offs, unsigned *flags, int32_t *count,
+                                                      int64_t ncells, PArrays A, const double *x, const double *y) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    if (i == 0) {
+        sims[0] = S;
+        offs[0] = 0;
+        offs[1] = S.n;
+        flags[0] = flags[1] = 0u;
+    }
+    for (int64_t t = i; t < ncells; t += threads) count[t] = 0;
+    if (i < S.n) {
+        const double2 zero = make_double2(0.0, 0.0);
+        A.pos[i] = make_double2(x[i], y[i]);
+        A.vel[i] = A.vp[i] = A.acc[i] = zero;
+        A.u[i] = A.up[i] = A.udot[i] = 0.0;
+        A.id[i] = (int32_t)i;
+        A.hprev[i] = 0.f;
+    }
 }
 
 const double kMonahanPref = 0x1.5d3b3e3583243p+3;  // 6*40/(pi*7), sim/sph.go:266
@@ -215,19 +231,15 @@ extern "C" int sph_density_noalloc(const sph_params *p, const double *x, const d
     Launch L{ds.sms, st};
     KnnTune tune{128, p->k + 16, 0.5f, 1.04f, ds.blocks_per_sm[p->k]};
 
-    // the array keeps the previous call's contents: clear what starts at zero
-    if (cudaMemsetAsync(T.count, 0, T.ncells * sizeof(int32_t), st) != cudaSuccess)
-        return nfail(SPH_ERR_CUDA, "sph_density_noalloc: clearing the cell table failed");
-    k_noalloc_init<<<1, 1, 0, st>>>(S, d_sims, d_offs, d_flags);
-    launch_scatter_state(c, L, A, nullptr, x, y, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+    k_noalloc_init<<<(n + 255) / 256, 256, 0, st>>>(S, d_sims, d_offs, d_flags, T.count, T.ncells, A, x, y);
     if (any_open) launch_bbox(c, L, A, PRED_INIT);
     launch_bin(c, L, A, T, nullptr, PRED_INIT);
     launch_scan(c, L, T);
     launch_permute(c, L, A, B, T, PRED_INIT, false);
     launch_knn(c, L, B, D, T, MODE_EXACT64, tune);
     launch_density(c, L, B, D, MODE_EXACT64, nullptr);
-    if (nbr_ids || nbr_dist) launch_gather_neighbours(c, L, B, B, D, nbr_ids, nbr_dist, nullptr, true);
-    if (rho || hsml) launch_gather_derived(c, L, B, D, nullptr, rho, nullptr, hsml);
+    if (nbr_ids || nbr_dist) launch_gather_neighbours(c, L, B, D, nbr_ids, nbr_dist, nullptr, rho, hsml);
+    else if (rho || hsml) launch_gather_derived(c, L, B, D, nullptr, rho, nullptr, hsml);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return nfail(SPH_ERR_CUDA, std::string("sph_density_noalloc: ") + cudaGetErrorString(e));
     unsigned f = 0;
