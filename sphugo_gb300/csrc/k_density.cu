@@ -26,6 +26,8 @@ namespace sphgpu {
 
 namespace {
 
+constexpr int kDensityNarrow = 10;
+
 struct DensityArgs {
     Ctx c;
     PArrays B;
@@ -209,7 +211,7 @@ void launch_density_fp64(const Ctx &c, const Launch &L, const PArrays &B, const 
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_density_fp64, 32, 0);
         return std::max(nb, 1);
     }();
-    DensityArgs a{c, B, D, PairTiles(c.n, (int64_t)L.sms * per_sm)};
+    DensityArgs a{c, B, D, PairTiles(c.n, L.sms, per_sm, kDensityNarrow)};
     k_density_fp64<<<a.tiles.grid(), 32, 0, L.stream>>>(a);
 }
 

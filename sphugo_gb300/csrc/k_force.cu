@@ -29,6 +29,8 @@ constexpr int kMixedBlocks = 20;  // resident blocks (warps) per SM (8 KB each)
 constexpr int kForceBlocks = 20, kForceBlocksMany = 25;
 constexpr int kForceSlotsMany = 224;
 constexpr int kForceWidePasses = 2;
+// (force stage at N = 16,000: 35 us at six particles per warp, 37 at eight, 39 at ten)
+constexpr int kForceNarrow = 6;
 // Tiles up to this width sum with three lanes per particle: 29 us at N = 10,000
 // against 40 with one.
 constexpr int kSplitWidth = 10;
@@ -572,7 +574,7 @@ static int force_blocks() {
 
 template <int SLOTS, int BLOCKS>
 static void launch_force_fp64(const ForceArgs &a, const Launch &L) {
-    const PairTiles t(a.c.n, (int64_t)L.sms * force_blocks<SLOTS, BLOCKS>());
+    const PairTiles t(a.c.n, L.sms, force_blocks<SLOTS, BLOCKS>(), kForceNarrow);
     k_force_fp64<SLOTS, BLOCKS><<<t.grid(), 32, 0, L.stream>>>(a, t);
 }
 
@@ -591,7 +593,7 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
         return;
     }
     if (c.n <= kMixedPairsMaxN) {
-        const PairTiles t(c.n, (int64_t)L.sms * kMixedBlocks);
+        const PairTiles t(c.n, L.sms, kMixedBlocks, kForceNarrow);
         k_force_mixed_pairs<<<t.grid(), 32, 0, L.stream>>>(a, t);
         return;
     }

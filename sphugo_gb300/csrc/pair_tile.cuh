@@ -15,6 +15,8 @@
 // one thread per particle computed them one after the other in a few resident
 // warps (N = 10,000: 313 warps on 608 sub-partitions).
 #pragma once
+#include <algorithm>
+
 #include "physics.cuh"
 
 namespace sphgpu {
@@ -38,18 +40,25 @@ constexpr bool pair_rows_fit(int slots) {
 
 // The tiles of n particles on a GPU that holds `resident` warps at once: as
 // many full passes of 32 particles a warp as there are, and the rest in equal
-// shares, one per resident warp. A tile is a block of one warp, so that the
-// next tile starts as soon as a warp is free; with a resident block for every
-// slot striding over the tiles, a pass of which a few warps had one tile more
-// than the others left the rest idle.
+// shares, one per resident warp, or, up to `narrow` particles each, three per
+// sub-partition: a tile's ordered sums are an addition instruction per entry of
+// the list whatever its width, so that with one particle per warp the FP64 unit
+// spends its time on them (density and force stage, us, one particle per
+// resident warp and three warps per sub-partition: N = 2000 14.6, 18.4 and 12.5,
+// 16.4; 4096 20.5, 20.5 and 14.4, 20.5; 10,000 22.0, 28.7 and 18.4, 28.7;
+// density alone 24,000 30.7 and, at 10, 26.6). A tile is a block of one warp,
+// so that the next tile starts as soon as a warp is free; with a resident
+// block for every slot striding over the tiles, a pass of which a few warps had
+// one tile more than the others left the rest idle.
 struct PairTiles {
     int64_t full;  // tiles of 32 particles, first
     int W;         // width of the others
     int64_t n;
-    PairTiles(int64_t n_, int64_t resident) : n(n_) {
+    PairTiles(int64_t n_, int sms, int warps_per_sm, int narrow) : n(n_) {
+        const int64_t resident = (int64_t)sms * warps_per_sm, few = (int64_t)sms * 12;
         full = n / (32 * resident) * resident;
-        W = (int)((n - 32 * full + resident - 1) / resident);
-        if (W < 1) W = 1;
+        const int64_t rest = n - 32 * full, share = (rest + resident - 1) / resident, wide = (rest + few - 1) / few;
+        W = (int)std::max<int64_t>({share, std::min<int64_t>(wide, narrow), 1});
     }
     int grid() const { return (int)(full + (n - 32 * full + W - 1) / W); }
     // first particle of tile t, and its width
