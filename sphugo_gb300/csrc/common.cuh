@@ -157,7 +157,7 @@ inline void simdev_fcell(SimDev &S) {
 }
 
 // FP32 fields of a SimDev from its FP64 grid fields
-__host__ __device__ inline void simdev_floats(SimDev &S) {
+inline void simdev_floats(SimDev &S) {
     for (int a = 0; a < 2; a++) {
         S.fs[a] = (float)S.s[a];
         S.fdtc[a] = (float)(S.dth * S.inv_s[a]);
