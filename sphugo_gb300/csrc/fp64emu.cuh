@@ -146,23 +146,6 @@ __device__ __forceinline__ bool emu_within(double x) {
 
 __device__ __forceinline__ bool emu_is_zero(double x) { return ((emu_hi(x) * 2u) | emu_lo(x)) == 0u; }
 
-// RN(x + y) for x, y > 0 whose exponents differ by less than 32: the smaller
-// significand shifted right, its lost bits kept whole in one word below.
-__device__ __forceinline__ double emu_addp_n(double x, double y) {
-    const uint64_t a = emu_bits(x), b = emu_bits(y);
-    const uint64_t g = a > b ? a : b, l = a > b ? b : a;
-    const uint32_t gh = (uint32_t)(g >> 32), lh = (uint32_t)(l >> 32), l0 = (uint32_t)l;
-    const uint32_t d = (gh >> 20) - (lh >> 20);
-    const uint32_t l1 = (lh & 0xfffffu) | 0x100000u;
-    const uint64_t sh = ((uint64_t)(l1 >> d) << 32) | __funnelshift_r(l0, l1, d);
-    const uint32_t w1 = __funnelshift_r(0u, l0, d);
-    const uint64_t S = ((((uint64_t)((gh & 0xfffffu) | 0x100000u)) << 32) | (uint32_t)g) + sh;  // [2^52, 2^54)
-    const uint32_t Sh = (uint32_t)(S >> 32), Sl = (uint32_t)S;
-    const uint32_t s = Sh >> 21;
-    const uint32_t eh = (gh & 0xfff00000u) - 0x100000u + (s << 20);
-    return emu_round_pack((Sh >> s) + eh, __funnelshift_r(Sl, Sh, s), __funnelshift_r(w1, Sl, s), w1 & s);
-}
-
 // RN(x y): the unchecked product, or the hardware's when an operand lies
 // outside [2^-500, 2^500) (zeros, subnormals, infinities and NaNs included)
 __device__ __forceinline__ double emu_mul(double x, double y) {
