@@ -51,7 +51,7 @@ HEAD_KIND, HEAD_N, HEAD_K, HEAD_DT, HEAD_SEED, HEAD_RUN = "clustered", 4_194_304
 METRIC = "particle-steps/s on 1 GB300: mixed/batched vs plain FP64 GPU at stated rel. error"
 TOLERANCES = {"neighbour_sets": "bit-exact", "fp64": "bit-exact", "fp64_fast": 1e-12,
               "mixed_rho": 1e-5, "mixed_accel_normalised": 1e-4, "mixed_udot_normalised": 1e-4}
-FORM_NAMES = {"Exact": "SPH_PREC_FP64 (bit-exact)", "Fast": "SPH_PREC_FP64_FAST (FMA, <=1e-12)",
+FORM_NAMES = {"Exact": "SPH_PREC_FP64 (bit-exact)", "Fast": "SPH_PREC_FP64_FAST (the kernels of SPH_PREC_FP64)",
               "Mixed": "SPH_PREC_MIXED (FP32 relative-coordinate Kahan sums, FP64 kNN decisions/h/integrator)"}
 HBM_FALLBACK_GBS = 6800.0
 
@@ -94,11 +94,11 @@ def auto_level(n):
 # integer pipes work beside the FP64 unit, which issues two lanes per SM per
 # clock. Their achieved FP64-slot rate can therefore exceed the FP64 unit's
 # own issue ceiling (frac > 1).
-FP64_NOTE = ("the density computes its multiplications, square roots and divisions, the force its "
-             "multiplications and divisions, with integer instructions beside the FP64 unit (bit-identical "
-             "to the hardware instructions; sph_selftest_fp64emu), so frac can exceed 1 against the FP64 "
-             "unit's issue ceiling; ncu on the clustered workload at N = 1,048,576: force FP64 pipe 67 %, "
-             "ALU pipe 52 %, issue slots 56 % busy; density 72 %, 62 %, 63 %")
+FP64_NOTE = ("the density and the force compute their multiplications, square roots and divisions with integer "
+             "instructions beside the FP64 unit (bit-identical to the hardware instructions; "
+             "sph_selftest_fp64emu), so frac can exceed 1 against the FP64 unit's issue ceiling; ncu on the "
+             "clustered workload at N = 1,048,576: force FP64 pipe 73 %, ALU pipe 57 %, issue slots 67 % busy; "
+             "density 68 %, 67 %, 70 %")
 
 
 def algorithmic(k, div, sqrt, lo_frac, visc_frac):
