@@ -17,18 +17,19 @@ namespace sphgpu {
 constexpr int64_t kMixedPairsMaxN = 16384;
 constexpr int kMixedBlocks = 20;  // resident blocks (warps) per SM (8 KB each)
 // The FP64 force is compiled twice: with 92 registers and chunks of nine entries
-// at 32 particles, 21 warps resident per SM, and with 72 and seven, 25 resident.
-// The second hides more latency over many passes, but each of its warps takes
-// longer and a short run ends later: beyond two passes of the first (force
-// stage, us, first and second: N = 50,000 81 and 86, 100,000 133 and 140,
-// 120,000 150 and 161, 150,000 194 and 178, 200,001 333 and 349, 250,000 303
-// and 290, 300,000 338 and 330, 500,000 544 and 533, 1,048,576 1103 and 1034,
-// clustered 4,194,304 4262 and 4040; k = 16 and 64 at 250,000 164 and 159, 599
-// and 580). 192 slots at 26 warps 1080 and 4112, 160 at 30 (64 registers,
-// spills) 1103 and 4203.
+// at 32 particles, 20 warps resident per SM, and with 72 and seven, 25 resident.
+// The second hides more latency, but each of its warps takes longer: it runs
+// beyond one pass of its own (121,600 particles), except where the first takes
+// just two (97,280 each; from one and a half of the second's on, up to 204,288).
+// Force stage, us, first and second: N = 50,000 81 and 86, 100,000 133 and 140,
+// 110,000 137 and 157; 130,000 173 and 167, 140,000 185 and 171, 170,000 212
+// and 205; 200,000 237 and 243; 250,000 303 and 290, 300,000 338 and 330,
+// 500,000 544 and 533, 1,048,576 1103 and 1034, clustered 4,194,304 4262 and
+// 4040; the same at k = 16, 45 and 64 (N = 110,000, 140,000, 200,000: k = 64 268
+// and 315, 367 and 342, 464 and 481). 192 slots at 26 warps 1080 and 4112, 160
+// at 30 (64 registers, spills) 1103 and 4203.
 constexpr int kForceBlocks = 20, kForceBlocksMany = 25;
 constexpr int kForceSlotsMany = 224;
-constexpr int kForceWidePasses = 2;
 // (force stage at N = 16,000: 35 us at six particles per warp, 37 at eight, 39 at ten)
 constexpr int kForceNarrow = 6;
 // Tiles up to this width sum with three lanes per particle: 29 us at N = 10,000
@@ -587,7 +588,9 @@ void launch_force(const Ctx &c, const Launch &L, const PArrays &B, const PArrays
     a.D = D;
     a.integrate = integrate ? 1 : 0;
     if (mode != MODE_MIXED) {
-        const bool wide = c.n <= (int64_t)kForceWidePasses * 32 * L.sms * force_blocks<kPairSlots, kForceBlocks>();
+        const int64_t pass1 = 32ll * L.sms * force_blocks<kPairSlots, kForceBlocks>();
+        const int64_t pass2 = 32ll * L.sms * force_blocks<kForceSlotsMany, kForceBlocksMany>();
+        const bool wide = c.n <= pass2 || (2 * c.n > 3 * pass2 && 10 * c.n <= 21 * pass1);
         if (wide) launch_force_fp64<kPairSlots, kForceBlocks>(a, L);
         else launch_force_fp64<kForceSlotsMany, kForceBlocksMany>(a, L);
         return;

@@ -96,7 +96,7 @@ def test_mixed_force_same_bits_pair_by_pair(gpu, n, k, kernel):
 
 
 # one past a full pass of 32 particles per resident warp, in the force
-# (3,192 warps), in the density (4,864), and past two of them
-@pytest.mark.parametrize("n", [102_145, 155_649, 204_289, 311_297])
+# (3,040 or 3,800 warps), in the density (4,864), and past two of them
+@pytest.mark.parametrize("n", [97_281, 121_601, 155_649, 182_401, 204_289, 311_297])
 def test_full_tiles_and_a_rest(gpu, oracle, n):
     check(oracle, ics.periodic_config(n, 13, 1e-5), flow(n, 14))
