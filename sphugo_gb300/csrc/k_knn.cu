@@ -317,8 +317,13 @@ __host__ __device__ constexpr size_t knn_warp_bytes(int nr) {
     return (size_t)32 * nr * 20 + (size_t)kRefineQueue * sizeof(int4);
 }
 
+// Bound by the latency of a warp's chain, so the more warps the better: 64
+// registers (a candidate's image constants are selected by its code where they
+// are used; as six more values per cell, handed on by shuffles, they took 80,
+// three blocks per SM: kNN stage N = 10,000 22.5 -> 21.7 us, k = 64 34 -> 32,
+// clustered N = 4,194,304 1092 -> 1079, mixed 1040 -> 1023).
 template <int MODE, int NR>
-__global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
+__global__ void __launch_bounds__(256, 4) k_knn(KnnArgs a) {
     using LS = ListShape<NR>;
     constexpr int CAP = LS::CAP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -416,7 +421,6 @@ __global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
                 const float CSx = sx0 * cpw, CSy = sy0 * cpw;
                 int cbase = 0, cnt = 0;
                 uint32_t img = 4;
-                float Ax = pr.x, Bx = 0.f, Cx = pr.z, Ay = pr.y, By = 0.f, Cy = pr.w;
                 bool heavy = false;
                 if (have) {
                     const int wx = vx >> cshift, wy = vy >> cshift;  // floor division by 2^cshift
@@ -429,10 +433,6 @@ __global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
                         cnt = __ldg(a.start + coff + ((int64_t)(mo + 1) << (2 * csh))) - j0;
                         heavy = cnt > kHeavyCell && csh > 0;
                         img = (uint32_t)((1 - wx) * 3 + (1 - wy));
-                        // image i = -w: hi part of q - i*d exact (Sterbenz) when i = +1,
-                        // of p + i*d when i = -1
-                        if (wx < 0) { Bx = dXh; Cx = cxp; } else if (wx > 0) { Ax = axm; Cx = cxm; }
-                        if (wy < 0) { By = dYh; Cy = cyp; } else if (wy > 0) { Ay = aym; Cy = cym; }
                         cbase = j0;
                     }
                 }
@@ -462,15 +462,15 @@ __global__ void __launch_bounds__(256, 3) k_knn(KnnArgs a) {
                     }
                     const int j = __shfl_sync(0xffffffffu, cbase, src) + t;
                     const uint32_t simg = __shfl_sync(0xffffffffu, img, src);
-                    const float sAx = __shfl_sync(0xffffffffu, Ax, src), sBx = __shfl_sync(0xffffffffu, Bx, src);
-                    const float sCx = __shfl_sync(0xffffffffu, Cx, src), sAy = __shfl_sync(0xffffffffu, Ay, src);
-                    const float sBy = __shfl_sync(0xffffffffu, By, src), sCy = __shfl_sync(0xffffffffu, Cy, src);
                     bool pass = false;
                     float d2 = 0.f;
                     if (t < tot && j != (int)q) {
                         const float4 r = __ldg(&B.rec[j]);
-                        const float dx = ((r.x - sBx) - sAx) + (r.z - sCx);
-                        const float dy = ((r.y - sBy) - sAy) + (r.w - sCy);
+                        // image i = -w: hi part of q - i*d exact (Sterbenz) when i = +1,
+                        // of p + i*d when i = -1 (the subtraction of 0 is exact)
+                        const bool xm = simg < 3u, xp = simg > 5u, ym = (0x049u >> simg) & 1u, yp = (0x124u >> simg) & 1u;
+                        const float dx = ((r.x - (xp ? dXh : 0.f)) - (xm ? axm : pr.x)) + (r.z - (xp ? cxp : xm ? cxm : pr.z));
+                        const float dy = ((r.y - (yp ? dYh : 0.f)) - (ym ? aym : pr.y)) + (r.w - (yp ? cyp : ym ? cym : pr.w));
                         d2 = __fmaf_rn(dx, dx, dy * dy);
                         pass = d2 <= R2;
                     }
