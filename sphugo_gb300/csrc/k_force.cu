@@ -61,10 +61,10 @@ __device__ __forceinline__ bool is_finite(double x) { return (emu_hi(x) & 0x7ff0
 __device__ __forceinline__ void integrate_one(const SimDev &S, double2 &pos, double2 &vel, double &u,
                                               double ax, double ay, double udot) {
     const double dth = S.dth;
-    const double dt2 = emu_mul(2.0, dth);  // exact, as is 2 udot: (2 udot) dth = udot (2 dth)
+    const double dt2 = emu_mul(2.0, dth);
     vel.x = __dadd_rn(vel.x, emu_mul(ax, dt2));
     vel.y = __dadd_rn(vel.y, emu_mul(ay, dt2));
-    u = __dadd_rn(u, emu_mul(udot, dt2));
+    u = __dadd_rn(u, emu_mul(emu_mul(udot, 2.0), dth));
     pos.x = __dadd_rn(pos.x, emu_mul(vel.x, dth));
     pos.y = __dadd_rn(pos.y, emu_mul(vel.y, dth));
     const bool fx = !is_nan(pos.x), fy = !is_nan(pos.y);
