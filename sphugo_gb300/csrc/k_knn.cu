@@ -18,7 +18,8 @@
 //      (a warp-uniform decision) until the list holds >= k and <= CAP entries
 //      and provably holds every candidate that can rank in the top k;
 //   4. the list is sorted by a register bitonic network on 32-bit keys
-//      (truncated FP32 squared distance | list slot);
+//      (truncated FP32 squared distance | list slot), entries of one truncated
+//      value then by their full ones;
 //   5. every order the FP32 values cannot decide (entries within 2 eps of each
 //      other) is settled with the reference's FP64 squared distance, ties
 //      broken by (particle id, image code); the FP64 forms settle all of them.
@@ -188,12 +189,28 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
 #pragma unroll
     for (int r = 0; r < NR; r++) sord[(r << 5) | lane] = v[r] & LS::SMASK;
     __syncwarp();
-    // tau: the largest FP32 value among the first k in truncated order (>= the k-th smallest)
-    float tmax = 0.f;
-    for (int e = lane; e < k; e += 32) tmax = fmaxf(tmax, __uint_as_float(skey[sord[e]]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
-    tau = tmax;
+    // Entries whose truncated values are equal stand in slot order: odd-even
+    // transposition by the full values, where any is out of place. The breaks
+    // below look at neighbours only, so three such entries would otherwise be cut
+    // into runs that are not in order themselves.
+    bool inv = false;
+    for (int e = lane; e + 1 < m; e += 32) inv |= skey[sord[e + 1]] < skey[sord[e]];
+    while (__any_sync(0xffffffffu, inv)) {
+        inv = false;
+        __syncwarp();
+        for (int parity = 0; parity < 2; parity++) {
+            for (int e = 2 * lane + parity; e + 1 < m; e += 64) {
+                const uint32_t sa = sord[e], sb = sord[e + 1];
+                if (skey[sb] < skey[sa]) {
+                    sord[e] = sb;
+                    sord[e + 1] = sa;
+                    inv = true;
+                }
+            }
+            __syncwarp();
+        }
+    }
+    tau = __uint_as_float(skey[sord[k - 1]]);
     eps = eps_of(tau, epsabs * R);
     if (tau + 3.f * eps > R2 * (1.f - 4.8e-7f)) {
         *Rnext = sqrtf((tau + 3.f * eps) * 1.00002f) * 1.0001f;
