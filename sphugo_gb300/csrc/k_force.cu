@@ -312,9 +312,23 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
 //      particle, or, for tiles of few particles, per particle and component.
 // Sums and differences run on the FP64 unit (75 cycles a warp instruction),
 // products and quotients on the integer pipes, unchecked behind range tests
-// (fp64emu.cuh); pairs that fail one (zero components, values outside 2^+-150,
-// infinities and NaNs) take the hardware's arithmetic out of line. Every
-// operation and its order are the reference's, so the results stay bit-exact.
+// (fp64emu.cuh); pairs that fail one are settled out of line. Every operation and
+// its order are the reference's, so the results stay bit-exact.
+//
+// Zeros fail the range tests, and whole states have them: a lattice or rows
+// (r_AB), a state at rest (v_AB), a cold gas (c, and with it cA + cB), viscosity
+// off. Out of line they stay on the integer pipes, with the products by zero left
+// out; only values outside 2^+-150, infinities, NaNs and coincident particles take
+// the hardware's arithmetic. Zero components of r_AB, which lie between others in
+// nearly every round, are kept in line: their slot holds kForZero, whose square is
+// lost in the other component's, and is marked, and the marked components' terms
+// are set to 0 before phase C. Force stage, us, k = 28, with the hardware's
+// arithmetic for all of them and so: perfect lattice at rest, N = 250,000, 765 and
+// 273 (a jittered moving one 262 both ways), N = 1,048,576 2604 and 739 (949 and
+// 953), cold gas moving 2957 and 1048, at rest 3135 and 667, alpha = 0 1602 and
+// 1009, viscosity off 1964 and 914. Zero components out of line too: 424 for the
+// first; in a form of phase B of its own, for chunks that have them: 0.5 to 2 % more
+// for every other state.
 //
 // Bound (ncu, uniform blast N = 1,048,576, k = 32): FP64 pipe 72 %, ALU 57 %,
 // issue 67 % busy; moving work either way between the two pipes (the sums
@@ -335,25 +349,64 @@ struct ForceRow {
 
 template <int SLOTS>
 struct ForceWarp {
-    static_assert(pair_rows_fit(SLOTS), "a tile's terms fit its slots at every width");
+    static_assert(SLOTS % 32 == 0 && pair_rows_fit(SLOTS), "a tile's terms fit its slots at every width");
     double x[SLOTS], y[SLOTS];  // r_AB, then the acceleration terms
     double e[SLOTS];            // v_AB . r_AB, then the du/dt terms
     ForceRow row[32];
     uint16_t list[SLOTS];       // approaching pairs from the front, the others from the back
+    uint32_t zx[SLOTS / 32], zy[SLOTS / 32];  // bits of the slots whose x (y) is kForZero
+    int marked;                 // the last chunk that has such slots
+    __device__ __forceinline__ bool zero_x(int slot) const { return zx[slot >> 5] >> (slot & 31) & 1u; }
+    __device__ __forceinline__ bool zero_y(int slot) const { return zy[slot >> 5] >> (slot & 31) & 1u; }
 };
+
+// A zero component of r_AB beside one within 2^+-150: its square, 2^-680, lies 380
+// binades below the other one's.
+constexpr double kForZero = 0x1p-340;
 
 struct Vec2D {
     double x, y;
 };
 
-// v_AB . r_AB with hardware arithmetic
-__device__ __noinline__ double force_dot_slow(double rx, double ry, double vx, double vy) {
+__device__ __forceinline__ bool in_range_or_zero(double x) { return emu_within<150>(x) || emu_is_zero(x); }
+__device__ __forceinline__ double emu_halve(double x) { return emu_double(emu_bits(x) - (1ull << 52)); }
+
+// Phase A of a pair that fails its range test: r_AB into the slot, and v_AB . r_AB
+// of operands in range or zero, else with hardware arithmetic
+template <typename Warp>
+__device__ __noinline__ double force_pair_slow(Warp &sm, int slot, int chunk, double rx, double ry, double vx, double vy) {
+    const bool mx = emu_is_zero(rx) && emu_within<150>(ry), my = emu_is_zero(ry) && emu_within<150>(rx);
+    sm.x[slot] = mx ? kForZero : rx;
+    sm.y[slot] = my ? kForZero : ry;
+    if (mx) atomicOr(&sm.zx[slot >> 5], 1u << (slot & 31));
+    if (my) atomicOr(&sm.zy[slot >> 5], 1u << (slot & 31));
+    if (mx || my) sm.marked = chunk;
+    if (in_range_or_zero(rx) && in_range_or_zero(ry) && in_range_or_zero(vx) && in_range_or_zero(vy)) {
+        const bool zx = emu_is_zero(vx) || emu_is_zero(rx), zy = emu_is_zero(vy) || emu_is_zero(ry);
+        if (zx && zy) return 0.0;
+        if (zx) return emu_mul_n(vy, ry);
+        if (zy) return emu_mul_n(vx, rx);
+    }
     return __dadd_rn(__dmul_rn(vx, rx), __dmul_rn(vy, ry));
 }
 
-// Pi (sim/sph.go:370-390) with hardware arithmetic, from the sums cA + cB, ...
+// Pi (sim/sph.go:370-390) from the sums cA + cB, ..., of operands in range or
+// zero (cA + cB, alpha, beta), else with hardware arithmetic
 __device__ __noinline__ double force_pi_slow(double rx, double ry, double dot, double c2, double rho2, double h2,
                                              double alpha, double beta, double etasq) {
+    const bool z1 = emu_is_zero(alpha) || emu_is_zero(c2), z2 = emu_is_zero(beta);
+    if (emu_within<350>(rx) && emu_within<350>(ry) && emu_within<400>(dot) && emu_within<150>(rho2) &&
+        emu_within<150>(h2) && in_range_or_zero(alpha) && in_range_or_zero(c2) && in_range_or_zero(beta)) {
+        const double den = __dadd_rn(__dadd_rn(emu_mul_n(rx, rx), emu_mul_n(ry, ry)), etasq);
+        const double mu = emu_div_n(emu_mul_n(dot, emu_halve(h2)), emu_divisor(den));
+        if (emu_within<300>(den) && emu_within<300>(mu)) {
+            if (z1 && z2) return 0.0;
+            const double t1 = z1 ? 0.0 : emu_mul_n(emu_mul_n(emu_neg(alpha), emu_halve(c2)), mu);
+            const double t2 = z2 ? 0.0 : emu_mul_n(emu_mul_n(beta, mu), mu);
+            const double num = z1 ? t2 : z2 ? t1 : __dadd_rn(t1, t2);
+            if (emu_within<800>(num)) return emu_div_n(num, emu_divisor(emu_halve(rho2)));
+        }
+    }
     const double cab = __dmul_rn(0.5, c2), rhoab = __dmul_rn(0.5, rho2), hab = __dmul_rn(0.5, h2);
     const double r2 = __dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry));
     const double mu = __ddiv_rn(__dmul_rn(dot, hab), __dadd_rn(r2, etasq));
@@ -364,13 +417,26 @@ struct ForceTerms {
     double x, y, e;
 };
 
-// a pair's terms with hardware arithmetic
-__device__ __noinline__ ForceTerms force_terms_slow(double rx, double ry, double dot, double sum3, double drk, double d) {
+// a pair's terms of operands in range or zero, else with hardware arithmetic
+template <typename Warp>
+__device__ __noinline__ ForceTerms force_terms_slow(const Warp &sm, int slot, double rx, double ry, double dot, double sum3,
+                                                    double drk, double d) {
+    if (sm.zero_x(slot)) rx = 0.0;
+    if (sm.zero_y(slot)) ry = 0.0;
+    const bool zd = emu_is_zero(dot) || emu_is_zero(drk), zx = emu_is_zero(rx), zy = emu_is_zero(ry), zs = emu_is_zero(sum3);
+    if (in_range_or_zero(rx) && in_range_or_zero(ry) && in_range_or_zero(sum3) && emu_within<150>(d) && in_range_or_zero(drk) &&
+        (emu_within<400>(dot) || emu_is_zero(dot))) {
+        ForceTerms t{0.0, 0.0, zd ? 0.0 : emu_mul_n(dot, drk)};
+        if (zs || emu_is_zero(drk) || (zx && zy)) return t;
+        const EmuDivisor dv = emu_divisor(d);
+        const double v = emu_div_n(emu_mul_n(emu_mul_n(zx ? ry : rx, sum3), drk), dv);
+        if (zx) t.y = v; else t.x = v;
+        if (!zx && !zy) t.y = emu_div_n(emu_mul_n(emu_mul_n(ry, sum3), drk), dv);
+        return t;
+    }
     return ForceTerms{__ddiv_rn(__dmul_rn(__dmul_rn(rx, sum3), drk), d), __ddiv_rn(__dmul_rn(__dmul_rn(ry, sum3), drk), d),
                       __dmul_rn(dot, drk)};
 }
-
-__device__ __forceinline__ double emu_halve(double x) { return emu_double(emu_bits(x) - (1ull << 52)); }
 
 template <int SLOTS, int BLOCKS>
 __global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTiles tiles) {
@@ -393,6 +459,8 @@ __global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTile
         const double4 d = D.der[q];
         R.c = d.x; R.rho = d.y; R.h = d.z; R.cterm = d.w;
     }
+    if (lane < SLOTS / 32) sm.zx[lane] = sm.zy[lane] = 0u;
+    if (lane == 0) sm.marked = -1;
     __syncwarp();
     double ax = 0.0, ay = 0.0, ed = 0.0;  // (three lanes per particle: ax alone, lane 3 p + component)
     for (int c = 0, e_lo = k; c < ch.n; c++) {
@@ -434,12 +502,12 @@ __global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTile
                 if (emu_within<150>(rx) && emu_within<150>(ry) && emu_within<150>(vx) && emu_within<150>(vy)) {
                     dot = __dadd_rn(emu_mul_n(vx, rx), emu_mul_n(vy, ry));  // 0, or 2^-353 at least (no subnormal)
                     approach = emu_hi(dot) > 0x80000000u;
+                    sm.x[slot] = rx;
+                    sm.y[slot] = ry;
                 } else {
-                    dot = force_dot_slow(rx, ry, vx, vy);
-                    approach = dot < 0.0;
+                    dot = force_pair_slow(sm, slot, c, rx, ry, vx, vy);
+                    approach = emu_bits(dot) > kEmuSign && !is_nan(dot);
                 }
-                sm.x[slot] = rx;
-                sm.y[slot] = ry;
                 sm.e[slot] = dot;
             }
             const uint32_t bal = __ballot_sync(0xffffffffu, approach);
@@ -468,7 +536,7 @@ __global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTile
             const int i = sm.list[n], p = pair_row(i, magic), slot = i + p * (st - ce);
             const ForceRow &R = sm.row[p];
             const double rx = sm.x[slot], ry = sm.y[slot], dot = sm.e[slot];
-            const bool in_r = emu_within<150>(rx) && emu_within<150>(ry);
+            const bool in_r = emu_within<350>(rx) && emu_within<350>(ry);  // (kForZero included; the products below stay normal)
             double sum = R.cterm;  // Pi + cA (0 + cA = cA)
             if (n < nlist) {
                 const SimDev &S = a.c.sims[sim_of(a.c, q0 + p)];
@@ -504,13 +572,21 @@ __global__ void __launch_bounds__(32, BLOCKS) k_force_fp64(ForceArgs a, PairTile
                 if (dz) t.x = t.y = 0.0;
                 if (dz || dot0) t.e = 0.0;
             } else {
-                t = force_terms_slow(rx, ry, dot, sum, drk, d);
+                t = force_terms_slow(sm, slot, rx, ry, dot, sum, drk, d);
             }
             sm.x[slot] = t.x;
             sm.y[slot] = t.y;
             sm.e[slot] = t.e;
         }
         __syncwarp();
+        if (sm.marked == c) {  // the marked components' terms (0 times a NaN or an infinity stays)
+            for (int slot = lane; slot < np * st; slot += 32) {
+                if (sm.zero_x(slot) && !is_nan(sm.x[slot])) sm.x[slot] = 0.0;
+                if (sm.zero_y(slot) && !is_nan(sm.y[slot])) sm.y[slot] = 0.0;
+            }
+            __syncwarp();
+            if (lane < SLOTS / 32) sm.zx[lane] = sm.zy[lane] = 0u;
+        }
         // ---- C
         if (W <= kSplitWidth) {
             if (lane < 3 * np) {

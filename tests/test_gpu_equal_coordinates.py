@@ -1,6 +1,7 @@
-"""Lattices and rows are ordinary initial states: pairs on a common row or
-column cost the FP64 density about what others do. (Their bits:
-test_gpu_near_ties.py, test_gpu_pair_tiles.py.)"""
+"""Lattices and rows, states at rest, cold gases and runs without viscosity are
+ordinary: pairs with zeros among their operands cost the FP64 density and force
+about what others do. (Their bits: test_gpu_near_ties.py and
+test_gpu_pair_tiles.py; pairs with several of these zeros together here.)"""
 import numpy as np
 import pytest
 
@@ -40,3 +41,39 @@ def test_density_of_a_lattice(gpu):
     instructions a pair and for the spread of short kernels."""
     at, jit = stages(lattice()), stages(lattice(1))
     assert at["density"] < 1.5 * jit["density"], (at, jit)
+
+
+@pytest.mark.parametrize("name,state", [
+    ("lattice at rest", dict(xy=lattice())), ("lattice, cold", dict(xy=lattice(), v=0.1, u=0.0)),
+    ("cold", dict(xy=lattice(1), v=0.1, u=0.0)), ("cold at rest", dict(xy=lattice(1), u=0.0)),
+    ("no alpha", dict(xy=lattice(1), v=0.1, alpha=0.0)), ("inviscid", dict(xy=lattice(1), v=0.1, alpha=0.0, beta=0.0))])
+def test_force_of_states_with_zeros(gpu, name, state):
+    """1.6 to 3.3 times a jittered warm lattice's time with the hardware's
+    arithmetic for such pairs; 0.7 to 1.1 without."""
+    at, jit = stages(**state), stages(lattice(1), v=0.1)
+    assert at["force_integrate"] < 1.4 * jit["force_integrate"], (name, at, jit)
+
+
+@pytest.mark.parametrize("m", [23, 61])
+@pytest.mark.parametrize("alpha,beta", [(1.0, 2.0), (0.0, 2.0), (1.0, 0.0), (0.0, 0.0)])
+def test_zeros_together(gpu, oracle, m, alpha, beta):
+    """Zeros in r_AB, v_AB, c and the viscosities in one state, coincident
+    coordinates beside differences below 2^-150, and energies that are zero for
+    some of the particles."""
+    n, r = m * m, np.random.default_rng(6)
+    x, y = [a.ravel() for a in np.meshgrid((np.arange(m) + 0.5) / m, (np.arange(m) + 0.5) / m)]
+    jx, jy = x + np.where(r.random(n) < 0.5, 0.0, r.uniform(-0.2, 0.2, n) / m), y.copy()
+    for vx, vy in ((np.zeros(n), np.zeros(n)), (r.integers(-1, 2, n) * 0.25, r.integers(-1, 2, n) * 0.25),
+                   (r.integers(-1, 2, n) * 1e-50, r.integers(-1, 2, n) * 0.5)):
+        for u in (np.zeros(n), np.where(r.random(n) < 0.5, 0.0, 1.0), np.ones(n)):
+            conf = ics.periodic_config(n, 20, 1e-5, alpha=alpha, beta=beta)
+            for px, py in ((x, y), (jx, jy)):
+                g = S.Simulation(conf, px, py, vx, vy, u)
+                o = oracle.OracleSim(oracle.make_params(n, 20, dth=conf.DeltaTHalf, alpha=alpha, beta=beta), px, py, vx, vy, u)
+                for steps in (1, 2):
+                    g.Step(steps)
+                    o.step(steps)
+                    got, want = {**g.state(), **g.derived()}, o.state()
+                    for key in got:
+                        assert np.array_equal(got[key], want[key]), (key, int(np.sum(got[key] != want[key])))
+                g.close()
