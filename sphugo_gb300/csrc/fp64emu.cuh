@@ -154,6 +154,14 @@ __device__ __forceinline__ double emu_mul(double x, double y) {
     return r;
 }
 
+// RN(x x): as emu_mul, but a zero, which differences of coordinates on a lattice
+// often are, squares without the hardware
+__device__ __forceinline__ double emu_sq(double x) {
+    double r = emu_mul_n(x, x);
+    if (!emu_within<500>(x)) r = emu_is_zero(x) ? 0.0 : emu_native_mul(x, x);
+    return r;
+}
+
 // u as a float, truncated
 __device__ __forceinline__ float emu_u2f_rz(uint32_t u) {
 #ifdef __CUDA_ARCH__

@@ -1124,10 +1124,16 @@ int knn_tile_occupancy_blocks(int k, int mode) {
 // the undecided runs by the same key; elsewhere the FP32 order agrees with
 // it). One warp per query, E consecutive entries per lane (k <= 32 E <= 128;
 // the block tiles' lists have at most 80): the keys of the list in one round,
-// then odd-even transposition until nothing moves, which is two or three
-// rounds since only near-equal neighbours are out of place. One thread per
-// query, with the keys in local memory, took 36 us at N = 10,000 for its
-// latency alone and 169 us at the clustered N = 4,194,304; this form 5 and 85.
+// then odd-even transposition until the list is in order, which it mostly is at
+// once or after a round or two, since only near-equal neighbours are out of place.
+// One thread per query, with the keys in local memory, took 36 us at N = 10,000
+// for its latency alone and 169 us at the clustered N = 4,194,304; this form 5
+// and about 78. On a perfect lattice, where every list has equal distances, the
+// check before each round and one comparison for both sides of a pair brought
+// N = 1,048,576, k = 28 from 513 to 385 us (350 with a thread per query) and the
+// kNN stage at N = 250,000 from 242 to 208 (212). Ids loaded at the first
+// equal pair and carried along: 602; a second pass by id over lists that have
+// equal pairs: 497.
 constexpr int kRerankMaxK = 80;
 
 template <int E>
@@ -1152,17 +1158,27 @@ __global__ void __launch_bounds__(256) k_rerank(KnnArgs a) {
                 key[r] = (unsigned long long)__double_as_longlong(nbr_d2(S, a.B, P, code[r]));
             }
         }
-        for (bool moved = true; moved;) {
-            bool m = false;
+        auto greater = [&](unsigned long long k0, uint32_t c0, unsigned long long k1, uint32_t c1) {
+            return k0 != k1 ? k0 > k1 : k0 != ~0ull && exact_greater(a.B, k0, c0, k1, c1);
+        };
+        bool changed = false;
+        for (;;) {
+            // in order already, as half of the lists are, and lattices' mostly
+            const unsigned long long nk = __shfl_down_sync(0xffffffffu, key[0], 1);
+            const uint32_t nc = __shfl_down_sync(0xffffffffu, code[0], 1);
+            bool m = lane < 31 && greater(key[E - 1], code[E - 1], nk, nc);
+#pragma unroll
+            for (int r = 0; r + 1 < E; r++) m |= greater(key[r], code[r], key[r + 1], code[r + 1]);
+            if (!__any_sync(0xffffffffu, m)) break;
+            changed = true;
             auto exchange = [&](int x, int y) {  // entries x < y of this lane
-                if (exact_greater(a.B, key[x], code[x], key[y], code[y])) {
+                if (greater(key[x], code[x], key[y], code[y])) {
                     const unsigned long long t = key[x];
                     key[x] = key[y];
                     key[y] = t;
                     const uint32_t c = code[x];
                     code[x] = code[y];
                     code[y] = c;
-                    m = true;
                 }
             };
             // this lane's last entry against the next lane's first (lanes of the
@@ -1174,10 +1190,7 @@ __global__ void __launch_bounds__(256) k_rerank(KnnArgs a) {
                 const uint32_t mc = low ? code[E - 1] : code[0];
                 const unsigned long long ok = __shfl_sync(0xffffffffu, mine, other);
                 const uint32_t oc = __shfl_sync(0xffffffffu, mc, other);
-                const bool pair = other != lane;
-                const unsigned long long lk = low ? mine : ok, hk = low ? ok : mine;
-                const uint32_t lc = low ? mc : oc, hc = low ? oc : mc;
-                if (pair && lk != hk ? lk > hk : pair && lk != ~0ull && exact_greater(a.B, lk, lc, hk, hc)) {
+                if (other != lane && greater(mine, mc, ok, oc) == low) {  // (a strict order; two past the end may trade places)
                     if (low) {
                         key[E - 1] = ok;
                         code[E - 1] = oc;
@@ -1185,22 +1198,16 @@ __global__ void __launch_bounds__(256) k_rerank(KnnArgs a) {
                         key[0] = ok;
                         code[0] = oc;
                     }
-                    m = true;
                 }
             };
-            if (E == 1) {
-                across(0);
-                across(1);
-            } else {
 #pragma unroll
-                for (int r = 0; r + 1 < E; r += 2) exchange(r, r + 1);
+            for (int r = 0; r + 1 < E; r += 2) exchange(r, r + 1);
 #pragma unroll
-                for (int r = 1; r + 1 < E; r += 2) exchange(r, r + 1);
-                across(0);
-                across(1);
-            }
-            moved = __any_sync(0xffffffffu, m);
+            for (int r = 1; r + 1 < E; r += 2) exchange(r, r + 1);
+            across(0);
+            across(1);
         }
+        if (!changed) continue;
 #pragma unroll
         for (int r = 0; r < E; r++) {
             const int e = lane * E + r;

@@ -140,7 +140,7 @@ __device__ __forceinline__ double dist_sq_ref(double px, double py, double ox, d
                                               double qx, double qy) {
     double dx = __dsub_rn(__dadd_rn(px, ox), qx);
     double dy = __dsub_rn(__dadd_rn(py, oy), qy);
-    return __dadd_rn(emu_mul(dx, dx), emu_mul(dy, dy));
+    return __dadd_rn(emu_sq(dx), emu_sq(dy));
 }
 
 // image code (i+1)*3+(j+1) -> shift (i*dX, j*dY), as float64(i)*deltaX in
@@ -157,7 +157,7 @@ __device__ __forceinline__ double nbr_d2(const SimDev &S, const PArrays &B, doub
     if ((code & 15u) == 4u) {
         // no offset: p + 0 = p (and -0 + 0 = +0 squares to the same value)
         const double dx = __dsub_rn(P.x, Q.x), dy = __dsub_rn(P.y, Q.y);
-        return __dadd_rn(emu_mul(dx, dx), emu_mul(dy, dy));
+        return __dadd_rn(emu_sq(dx), emu_sq(dy));
     }
     double ox, oy;
     img_shift(S, code & 15u, ox, oy);

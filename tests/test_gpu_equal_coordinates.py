@@ -13,16 +13,16 @@ pytestmark = pytest.mark.gpu
 M = 500
 
 
-def lattice(j=0.0):
-    """An M x M lattice in the unit box, moved by up to 0.3 of a site times j."""
+def lattice(j=0.0, m=M):
+    """An m x m lattice in the unit box, moved by up to 0.3 of a site times j."""
     r = np.random.default_rng(1)
-    x, y = [a.ravel() for a in np.meshgrid((np.arange(M) + 0.5) / M, (np.arange(M) + 0.5) / M)]
-    return x + j * r.uniform(-0.3, 0.3, M * M) / M, y + j * r.uniform(-0.3, 0.3, M * M) / M
+    x, y = [a.ravel() for a in np.meshgrid((np.arange(m) + 0.5) / m, (np.arange(m) + 0.5) / m)]
+    return x + j * r.uniform(-0.3, 0.3, m * m) / m, y + j * r.uniform(-0.3, 0.3, m * m) / m
 
 
 def stages(xy, v=0.0, u=1.0, alpha=1.0, beta=2.0):
     """Stage times in milliseconds, the fastest of three profiles of four steps."""
-    n, r = M * M, np.random.default_rng(2)
+    n, r = len(xy[0]), np.random.default_rng(2)
     conf = ics.periodic_config(n, 28, 1e-6, alpha=alpha, beta=beta)
     s = S.Simulation(conf, *xy, r.normal(0, 1, n) * v, r.normal(0, 1, n) * v, np.full(n, u))
     s.Step(1)
@@ -41,6 +41,14 @@ def test_density_of_a_lattice(gpu):
     instructions a pair and for the spread of short kernels."""
     at, jit = stages(lattice()), stages(lattice(1))
     assert at["density"] < 1.5 * jit["density"], (at, jit)
+
+
+def test_search_of_a_lattice(gpu):
+    """Every list of a perfect lattice has equal distances and is ordered again
+    in FP64: 2.7 times a jittered one's search, 3.3 before lists in order were
+    left as they are."""
+    at, jit = stages(lattice(0, 1024)), stages(lattice(1, 1024))
+    assert at["knn"] < 3.0 * jit["knn"], (at, jit)
 
 
 @pytest.mark.parametrize("name,state", [

@@ -66,3 +66,22 @@ def test_three_near_ties_in_a_long_list(gpu, oracle):
     n, r = 100_003, np.random.default_rng(12)
     x, y, _, _, u = ics.uniform_blast(n, 12)
     against_oracle(oracle, ics.periodic_config(n, 128, 1e-5), (x, y, r.normal(0, 0.3, n), r.normal(0, 0.3, n), u), steps=1)
+
+
+# lists of up to 32, 64 and 80 entries (each closes a shell, so that the tiles decide the sets)
+@pytest.mark.parametrize("k,path", [(28, 8), (28, 4), (60, 4), (80, 4)])
+def test_equal_distances_in_block_tiles(gpu, oracle, k, path):
+    """A lattice whose distances within a shell are equal in FP64, its ids in
+    random order: the block tiles' lists are ordered by (distance, id, image)."""
+    m, r = 64, np.random.default_rng(5)
+    n = m * m
+    x, y = lattice(m)
+    p = r.permutation(n)
+    z, conf = np.zeros(n), ics.periodic_config(n, k, 1e-6)
+    arrs = (x[p], y[p], z, z, np.ones(n))
+    against_oracle(oracle, conf, arrs, steps=2, path=path)
+    g = S.Simulation(conf, *arrs)
+    g.SetSearch(path)
+    g.Step(2)
+    assert g.search_stats()[1] < n // 2
+    g.close()
