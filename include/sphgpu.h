@@ -188,18 +188,19 @@ int sph_step_profiled(sph_handle *h, int32_t nsteps, double stage_ms[SPH_NUM_STA
 int32_t sph_kernels_per_step(sph_handle *h);
 /* Neighbour search path (no reference counterpart): tiles of candidate
  * records in shared memory scanned by one thread per query, the queries they
- * cannot settle finished by the per-query search. 1 (default) = the default
- * for k and the particle count (block tiles of 8 warps = 256 consecutive
- * particles for k <= 37, of 4 warps for k <= 80, else one tile per warp; in
- * the FP64 forms the per-query search up to 16,384 particles); 4 or 8 = block
- * tiles of that many warps; 2 = one tile per warp (32 particles); 0 =
- * per-query search for every particle. The neighbour sets and every FP64
+ * cannot settle finished by the per-query search. 1 = the default tile shape
+ * for k (block tiles of 8 warps = 256 consecutive particles for k <= 37, of 4
+ * warps for k <= 80, else one tile per warp); 4 or 8 = block tiles of that many
+ * warps; 2 = one tile per warp (32 particles); 0 = per-query search for every
+ * particle. Without a call (or sph_autotune): 1, but 0 in the FP64 forms up to
+ * 16,384 particles (sph_append included). The neighbour sets and every FP64
  * result are identical on every path; the mixed form's FP32 sums may differ
  * in the last bits (they follow the list order). SPH_ERR_ARG for a shape
  * that k does not allow. */
 int sph_set_search(sph_handle *h, int32_t tiles);
 /* Queries of the last force evaluation and how many of them the group-tile
- * search left to the per-query search (all of them with tiles off). */
+ * search left to the per-query search (all of them where that is the chosen
+ * path). */
 int sph_search_stats(sph_handle *h, int64_t *queries, int64_t *deferred);
 /* Autotuner (no reference counterpart): on a freshly uploaded state (before
  * the first step) it times forces-only evaluations over a small grid of the

@@ -1118,8 +1118,8 @@ int sph_set_search(sph_handle *h, int32_t tiles) {
     const int bdef = default_block_warps(h->k);
     if ((tiles == 4 || tiles == 8) && tiles > bdef)
         return fail(SPH_ERR_ARG, "no block tiles of that many warps for this k");
-    h->search_default = tiles == 1;
-    const int tile = tiles == 1 ? (default_per_query(h->n, h->mode) ? 0 : 1) : tiles ? 1 : 0;
+    h->search_default = false;
+    const int tile = tiles ? 1 : 0;
     const int block = tiles == 1 ? bdef : tiles == 2 ? 0 : tiles == 0 ? h->tune.block_warps : tiles;
     if (h->tune.tile != tile || h->tune.block_warps != block) {
         h->tune.tile = tile;

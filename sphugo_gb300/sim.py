@@ -140,7 +140,7 @@ class SphConfig:
 
 
 def _set_search(h, tiles):
-    """True / 1: tiles of the default shape; 2: one tile per warp; 4 or 8:
+    """True / 1: tiles of the default shape for k; 2: one tile per warp; 4 or 8:
     block tiles of that many warps; False / 0: per-query search."""
     L.check(L.load().sph_set_search(h, int(tiles)))
 
@@ -293,13 +293,16 @@ class Simulation:
         return _autotune(self._h, use_cache)
 
     def SetSearch(self, tiles=True):
-        """Neighbour search path: True / 1 tiles of the default shape, 8 or 4
-        block tiles of that many warps, 2 one tile per warp, False / 0 the
-        per-query search; every path returns the same neighbour sets."""
+        """Neighbour search path: True / 1 tiles of the default shape for k, 8 or
+        4 block tiles of that many warps, 2 one tile per warp, False / 0 the
+        per-query search; every path returns the same neighbour sets. Without a
+        call: tiles, but the per-query search in the FP64 forms up to 16,384
+        particles."""
         _set_search(self._h, tiles)
 
     def search_stats(self) -> tuple:
-        """(queries, deferred to the per-query search) of the last force evaluation."""
+        """(queries, those left to the per-query search) of the last force
+        evaluation; all of them where that search is the chosen path."""
         return _search_stats(self._h)
 
     def Save(self, path: str):

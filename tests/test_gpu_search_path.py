@@ -1,0 +1,38 @@
+"""Which search a handle runs, seen by how many queries are left to the
+per-query one: without a choice that search for FP64 handles of up to 16,384
+particles and tiles for the others; an explicit choice of tiles is one."""
+import numpy as np
+import pytest
+
+from sphugo_gb300 import ics
+from sphugo_gb300 import sim as S
+
+pytestmark = pytest.mark.gpu
+
+
+def run(n, k, precision="Exact", path=None, steps=2):
+    x, y, vx, vy, u = ics.uniform_blast(n, 9)
+    s = S.Simulation(ics.periodic_config(n, k, 1e-5, precision), x, y, vx, vy, u)
+    if path is not None:
+        s.SetSearch(path)
+    s.Step(steps)
+    return s
+
+
+@pytest.mark.parametrize("n,k", [(6000, 8), (6000, 32), (6000, 64), (16_384, 100), (16_384, 128)])
+def test_tiles_on_request(gpu, n, k):
+    """1 means tiles at every particle count; their results are the default's."""
+    a, b, c = run(n, k), run(n, k, path=True), run(n, k, path=0)
+    assert a.search_stats() == (n, n) and c.search_stats() == (n, n)
+    assert b.search_stats()[1] < (n if k > 80 else n // 4)
+    sa, sb = a.state(), b.state()
+    for key in sa:
+        assert np.array_equal(sa[key], sb[key]), key
+    for p, q in zip(a.neighbours(), b.neighbours()):
+        assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("n,precision,tiles", [(16_384, "Exact", False), (16_385, "Exact", True), (6000, "Mixed", True)])
+def test_default(gpu, n, precision, tiles):
+    d = run(n, 32, precision).search_stats()[1]
+    assert d < n // 4 if tiles else d == n
