@@ -64,6 +64,8 @@ int default_block_warps(int k) {
 constexpr int64_t kPerQueryMaxN = 16384;
 bool default_per_query(int64_t n, int mode) { return mode != MODE_MIXED && n <= kPerQueryMaxN; }
 
+constexpr float kDefaultTheta = 0.5f, kDefaultHgrow = 1.04f;
+
 int auto_level(int64_t n) {
     // about one to four particles per finest cell
     double l = std::floor(0.5 * std::log2(std::max<double>((double)n, 2.0) / 2.0) + 0.5);
@@ -463,8 +465,8 @@ int create_impl(const sph_params *params, const int64_t *counts, int32_t nsims, 
     knn_init_attrs();
     h->tune.block = 256;
     h->tune.cap = (int)(k + 16);
-    h->tune.theta = 0.5f;
-    h->tune.hgrow = 1.04f;
+    h->tune.theta = kDefaultTheta;
+    h->tune.hgrow = kDefaultHgrow;
     h->tune.blocks_per_sm = std::max(1, knn_occupancy_blocks(h->tune.block, h->tune.cap, kernel_mode(h->mode)));
     h->tune.tile = default_per_query(n, h->mode) ? 0 : 1;
     h->tune.tile_blocks_per_sm = std::max(1, knn_tile_occupancy_blocks((int)k, kernel_mode(h->mode)));
@@ -586,7 +588,7 @@ std::string tune_cache_path() {
 }
 
 struct TuneChoice {
-    float theta = 0.5f, hgrow = 1.04f;
+    float theta = kDefaultTheta, hgrow = kDefaultHgrow;
     int delta = 0, tile = 1, block = 8;
     double ms = 0.0;
 };
@@ -1215,7 +1217,7 @@ int sph_autotune(sph_handle *h, int32_t use_cache, char *report, int32_t report_
                 h->tune.tile = tiles[v];
                 h->tune.block_warps = blocks[v];
                 h->tune.theta = thetas[v];
-                h->tune.hgrow = 1.04f;
+                h->tune.hgrow = kDefaultHgrow;
                 destroy_graphs(h);
                 double ms = 0.0;
                 if ((rc = time_forces(h, reps, &ms))) return rc;
@@ -1226,7 +1228,7 @@ int sph_autotune(sph_handle *h, int32_t use_cache, char *report, int32_t report_
                     best.tile = tiles[v];
                     best.block = blocks[v];
                     best.delta = delta;
-                    best.hgrow = 1.04f;
+                    best.hgrow = kDefaultHgrow;
                 }
             }
         }
@@ -1400,7 +1402,11 @@ int sph_load(sph_handle *h, const char *path) {
     }
     if ((rc = check_checkpoint(h, hd, bufs))) return rc;
     if (hd.level_delta != h->level_delta && (rc = apply_levels(h, hd.level_delta))) return rc;
-    h->search_default = false;  // the saved run's search
+    // the saved run's search: a choice of its own, or (the settings do not tell an
+    // equal choice apart) the default, which then goes on following the count
+    h->search_default = hd.tile == (default_per_query(h->n, h->mode) ? 0 : 1) &&
+                        hd.block_warps == default_block_warps(h->k) && hd.theta == kDefaultTheta &&
+                        hd.hgrow == kDefaultHgrow && hd.level_delta == 0;
     if (hd.theta != h->tune.theta || hd.hgrow != h->tune.hgrow || hd.tile != h->tune.tile ||
         hd.block_warps != h->tune.block_warps) {
         h->tune.theta = hd.theta;

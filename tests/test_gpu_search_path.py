@@ -4,6 +4,7 @@ particles and tiles for the others; an explicit choice of tiles is one."""
 import numpy as np
 import pytest
 
+from sphugo_gb300 import _lib as L
 from sphugo_gb300 import ics
 from sphugo_gb300 import sim as S
 
@@ -36,3 +37,33 @@ def test_tiles_on_request(gpu, n, k):
 def test_default(gpu, n, precision, tiles):
     d = run(n, 32, precision).search_stats()[1]
     assert d < n // 4 if tiles else d == n
+
+
+def append(s, gpu, x, y):
+    L.check(gpu.sph_append(s._h, len(x), L.dptr(x), L.dptr(y), None, None, None, None))
+    s.n += len(x)
+
+
+@pytest.mark.parametrize("path", [None, 8, 2])
+def test_default_goes_on_after_a_checkpoint(gpu, tmp_path, path):
+    """A run below 16,384 particles, saved, loaded and grown beyond by sph_append
+    takes the search that the uninterrupted run takes, with its results; a choice
+    of tiles stays."""
+    n, more, k = 16_000, 900, 32
+    r = np.random.default_rng(4)
+    x, y = r.random(more), r.random(more)
+    a = run(n, k, path=path)
+    a.Save(tmp_path / "s.ck")
+    xi, yi, vx, vy, u = ics.uniform_blast(n, 9)
+    b = S.Simulation(ics.periodic_config(n, k, 1e-5), xi, yi, vx, vy, u)
+    b.Load(tmp_path / "s.ck")
+    a.Step(1)
+    b.Step(1)
+    assert a.search_stats() == b.search_stats()
+    for s in (a, b):
+        append(s, gpu, x, y)
+        s.Step(2)
+        assert s.search_stats()[0] == n + more and s.search_stats()[1] < n // 4
+    sa, sb = a.state(), b.state()
+    for key in sa:
+        assert np.array_equal(sa[key], sb[key]), key
