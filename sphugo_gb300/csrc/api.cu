@@ -528,6 +528,23 @@ int stage_in(sph_handle *h, double *staging, const double *src, const double **d
     *dev = staging;
     return SPH_OK;
 }
+// The map (in the binning's scratch) to the caller's order for a transfer with an
+// array in place; a transfer through staging arrays alone runs in the slots' order,
+// without one, unless it reads more than kSlotOrderMaxN particles out: its scattered
+// writes then cost more than scattered reads once the arrays outgrow L2. Pageable
+// host arrays, us, caller's order and the slots': set_state N = 10,000 108 and 103,
+// 1,048,576 570 and 535, 4,194,304 2668 and 2168; get_state 10,000 106 and 98,
+// 1,048,576 496 and 492, 2,097,152 933 and 1156, 4,194,304 1870 and 2578; get_derived
+// 51 and 41, 195 and 187, 350 and 335, 699 and 728.
+constexpr int64_t kSlotOrderMaxN = (int64_t)1 << 20;
+template <typename T>
+const int32_t *slots_for(sph_handle *h, T *const *dev, int arrays, bool out) {
+    bool map = out && h->n > kSlotOrderMaxN;
+    for (int i = 0; i < arrays; i++) map |= dev[i] && (dev[i] < h->d_io || dev[i] >= h->d_io + h->io_doubles);
+    if (!map) return nullptr;
+    launch_slots(h->ctx(), h->launch(), h->A, h->T.tmp);
+    return h->T.tmp;
+}
 // Where a kernel leaves n values for the caller: in place, or in the staging
 // array, which copy_out then brings over.
 double *stage_out(sph_handle *h, double *staging, double *dst) {
@@ -709,7 +726,7 @@ int sph_upload(sph_handle *h, const double *x, const double *y, const double *vx
     const double *src[5] = {x, y, vx, vy, u}, *d[5];
     for (int i = 0; i < 5; i++)
         if (int rc = stage_in(h, h->d_io + i * n, src[i], &d[i])) return rc;
-    launch_scatter_state(h->ctx(), h->launch(), h->A, nullptr, d[0], d[1], d[2], d[3], d[4], nullptr, nullptr, nullptr);
+    launch_scatter_state(h->ctx(), h->launch(), h->A, nullptr, d[0], d[1], d[2], d[3], d[4], nullptr, nullptr, nullptr, true);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->step = 0;
@@ -828,8 +845,7 @@ int sph_set_state(sph_handle *h, const double *x, const double *y, const double 
     const double *src[8] = {x, y, vx, vy, u, ax, ay, udot}, *d[8];
     for (int i = 0; i < 8; i++)
         if (int rc = stage_in(h, h->d_io + i * n, src[i], &d[i])) return rc;
-    launch_slots(h->ctx(), h->launch(), h->A, h->T.tmp);  // (binning scratch)
-    launch_scatter_state(h->ctx(), h->launch(), h->A, h->T.tmp, d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7]);
+    launch_scatter_state(h->ctx(), h->launch(), h->A, slots_for(h, d, 8, false), d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], false);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return SPH_OK;
@@ -843,8 +859,7 @@ int sph_get_state(sph_handle *h, double *x, double *y, double *vx, double *vy, d
     const int64_t n = h->n;
     double *dst[8] = {x, y, vx, vy, u, ax, ay, udot}, *d[8];
     for (int i = 0; i < 8; i++) d[i] = stage_out(h, h->d_io + i * n, dst[i]);
-    launch_slots(h->ctx(), h->launch(), h->A, h->T.tmp);
-    launch_gather_state(h->ctx(), h->launch(), h->A, h->T.tmp, d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7]);
+    launch_gather_state(h->ctx(), h->launch(), h->A, slots_for(h, d, 8, true), d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7]);
     CUDA_TRY(cudaGetLastError());
     for (int i = 0; i < 8; i++)
         if (int rc = copy_out(h, dst[i], d[i], h->d_io + i * n)) return rc;
@@ -859,8 +874,7 @@ int sph_get_derived(sph_handle *h, double *rho, double *c, double *hsml) {
     const int64_t n = h->n;
     double *dst[3] = {rho, c, hsml}, *d[3];
     for (int i = 0; i < 3; i++) d[i] = stage_out(h, h->d_io + i * n, dst[i]);
-    launch_slots(h->ctx(), h->launch(), h->A, h->T.tmp);
-    launch_gather_derived(h->ctx(), h->launch(), h->A, h->D, h->T.tmp, d[0], d[1], d[2]);
+    launch_gather_derived(h->ctx(), h->launch(), h->A, h->D, slots_for(h, d, 3, true), d[0], d[1], d[2]);
     CUDA_TRY(cudaGetLastError());
     for (int i = 0; i < 3; i++)
         if (int rc = copy_out(h, dst[i], d[i], h->d_io + i * n)) return rc;
@@ -1178,8 +1192,7 @@ int sph_autotune(sph_handle *h, int32_t use_cache, char *report, int32_t report_
     const int64_t n = h->n;
     double *d = h->d_io;
     // keep the uploaded state (caller order) to restore it afterwards
-    launch_slots(h->ctx(), h->launch(), h->A, h->T.tmp);
-    launch_gather_state(h->ctx(), h->launch(), h->A, h->T.tmp, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n, nullptr,
+    launch_gather_state(h->ctx(), h->launch(), h->A, nullptr, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n, nullptr,
                         nullptr, nullptr);
     CUDA_TRY(cudaGetLastError());
     int rc;
@@ -1253,7 +1266,7 @@ int sph_autotune(sph_handle *h, int32_t use_cache, char *report, int32_t report_
     if ((rc = apply_levels(h, best.delta))) return rc;
     // back to the uploaded state
     launch_scatter_state(h->ctx(), h->launch(), h->A, nullptr, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n, nullptr, nullptr,
-                         nullptr);
+                         nullptr, true);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     h->evaluated = false;

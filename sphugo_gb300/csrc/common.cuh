@@ -268,7 +268,7 @@ void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, const 
                          double *vx, double *vy, double *u, double *ax, double *ay, double *udot);
 void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, const double *x,
                           const double *y, const double *vx, const double *vy, const double *u,
-                          const double *ax, const double *ay, const double *udot);
+                          const double *ax, const double *ay, const double *udot, bool fresh);
 void launch_append(const Launch &L, const PArrays &A, int64_t n0, int64_t count, const double *buf);
 void launch_gather_derived(const Ctx &c, const Launch &L, const PArrays &A, const Derived &D, const int32_t *slot,
                            double *rho, double *cs, double *h);

@@ -16,9 +16,10 @@ static int grid_for(const Launch &L, int64_t n, int block) {
     return g < 1 ? 1 : g;
 }
 
-// Slot of each caller index: the transfers below run in the caller's order, so
-// that they read and write the caller's arrays, which may be pinned host memory
-// behind the host link, in whole lines, and the device's arrays at the slots.
+// Slot of each caller index: transfers with an array in pinned host memory run in
+// the caller's order, so that they read and write it behind the host link in whole
+// lines, and the device's arrays at the slots. Without slots they run in the slots'
+// order, scattering to or gathering from the staging arrays.
 __global__ void k_slots(Ctx c, PArrays A, int32_t *slot) {
     GRID_STRIDE(i, c.n) slot[A.id[i]] = (int32_t)i;
 }
@@ -30,16 +31,16 @@ void launch_slots(const Ctx &c, const Launch &L, const PArrays &A, int32_t *slot
 __global__ void k_gather_state(Ctx c, PArrays A, const int32_t *slot, double *x, double *y, double *vx, double *vy,
                                double *u, double *ax, double *ay, double *udot) {
     GRID_STRIDE(t, c.n) {
-        const int32_t i = slot[t];
+        const int64_t i = slot ? slot[t] : t, o = slot ? t : A.id[t];
         const double2 p = A.pos[i], v = A.vel[i], a = A.acc[i];
-        if (x) x[t] = p.x;
-        if (y) y[t] = p.y;
-        if (vx) vx[t] = v.x;
-        if (vy) vy[t] = v.y;
-        if (u) u[t] = A.u[i];
-        if (ax) ax[t] = a.x;
-        if (ay) ay[t] = a.y;
-        if (udot) udot[t] = A.udot[i];
+        if (x) x[o] = p.x;
+        if (y) y[o] = p.y;
+        if (vx) vx[o] = v.x;
+        if (vy) vy[o] = v.y;
+        if (u) u[o] = A.u[i];
+        if (ax) ax[o] = a.x;
+        if (ay) ay[o] = a.y;
+        if (udot) udot[o] = A.udot[i];
     }
 }
 
@@ -48,22 +49,23 @@ void launch_gather_state(const Ctx &c, const Launch &L, const PArrays &A, const 
     k_gather_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot, x, y, vx, vy, u, ax, ay, udot);
 }
 
-// slot = NULL: fresh upload, slot i holds particle i and the integrator
-// history (accelerations, predictions, radius guess) starts from zero; else
-// the state of every particle in its current slot is replaced.
+// fresh: an upload, slot i holds particle i and the integrator history
+// (accelerations, predictions, radius guess) starts from zero; else the state of
+// every particle in its current slot is replaced.
 __global__ void k_scatter_state(Ctx c, PArrays A, const int32_t *slot, const double *x, const double *y, const double *vx,
                                 const double *vy, const double *u, const double *ax, const double *ay,
-                                const double *udot) {
+                                const double *udot, int fresh) {
     GRID_STRIDE(t, c.n) {
         const int32_t i = slot ? slot[t] : (int32_t)t;
-        const double2 v = make_double2(vx ? vx[t] : 0.0, vy ? vy[t] : 0.0);
-        const double e = u ? u[t] : 0.0;
-        A.pos[i] = make_double2(x[t], y[t]);
+        const int64_t o = slot || fresh ? t : A.id[t];
+        const double2 v = make_double2(vx ? vx[o] : 0.0, vy ? vy[o] : 0.0);
+        const double e = u ? u[o] : 0.0;
+        A.pos[i] = make_double2(x[o], y[o]);
         A.vel[i] = v;
         A.u[i] = e;
-        if (slot) {
-            A.acc[i] = make_double2(ax ? ax[t] : 0.0, ay ? ay[t] : 0.0);
-            A.udot[i] = udot ? udot[t] : 0.0;
+        if (!fresh) {
+            A.acc[i] = make_double2(ax ? ax[o] : 0.0, ay ? ay[o] : 0.0);
+            A.udot[i] = udot ? udot[o] : 0.0;
         } else {
             A.id[i] = i;
             A.hprev[i] = 0.f;
@@ -100,8 +102,8 @@ void launch_append(const Launch &L, const PArrays &A, int64_t n0, int64_t count,
 
 void launch_scatter_state(const Ctx &c, const Launch &L, const PArrays &A, const int32_t *slot, const double *x,
                           const double *y, const double *vx, const double *vy, const double *u,
-                          const double *ax, const double *ay, const double *udot) {
-    k_scatter_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot, x, y, vx, vy, u, ax, ay, udot);
+                          const double *ax, const double *ay, const double *udot, bool fresh) {
+    k_scatter_state<<<grid_for(L, c.n, 256), 256, 0, L.stream>>>(c, A, slot, x, y, vx, vy, u, ax, ay, udot, fresh ? 1 : 0);
 }
 
 // by caller index (slot given), or in the slots' own order of A.id
