@@ -91,7 +91,7 @@ __device__ __forceinline__ bool exact_greater(const PArrays &B, unsigned long lo
 // Returns 0 when written, or 1 when the k-th FP32 value lies too close to the
 // search radius R for the list to be complete (*Rnext: a radius that is).
 template <int MODE, int NR>
-__device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m, float R, float epsabs,
+__device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m, float R, float ea,
                             uint32_t *skey, uint32_t *scode, uint32_t *sord, unsigned long long *sexact,
                             int lane, float *Rnext, uint32_t *far) {
     float *sd2 = reinterpret_cast<float *>(sexact);  // fused density: squared distances in list order (the keys are done with)
@@ -139,13 +139,13 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
         const uint32_t g2 = __reduce_max_sync(0xffffffffu, cand2);
         const uint32_t nties = __popc(__ballot_sync(0xffffffffu, top == gtop));
         tau = __uint_as_float(gtop & 0x7fffffffu);
-        eps = eps_of(tau, epsabs * R);
+        eps = eps_of(tau, ea);
         if (tau + 3.f * eps > R2 * (1.f - 4.8e-7f)) {
             *Rnext = sqrtf((tau + 3.f * eps) * 1.00002f) * 1.0001f;
             return 1;
         }
         const float fd = __uint_as_float(dropped_min), f2 = __uint_as_float(g2 & 0x7fffffffu);
-        const bool set_ok = (m == k) || (fd - tau > 2.f * eps_of(fd, epsabs * R));
+        const bool set_ok = (m == k) || (fd - tau > 2.f * eps_of(fd, ea));
         const bool top_ok = nties == 1 && (k == 1 || tau - f2 > 2.f * eps);
         if (set_ok && top_ok) {
             // write the kept entries in slot order, the farthest last
@@ -211,7 +211,7 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
         }
     }
     tau = __uint_as_float(skey[sord[k - 1]]);
-    eps = eps_of(tau, epsabs * R);
+    eps = eps_of(tau, ea);
     if (tau + 3.f * eps > R2 * (1.f - 4.8e-7f)) {
         *Rnext = sqrtf((tau + 3.f * eps) * 1.00002f) * 1.0001f;
         __syncwarp();
@@ -231,7 +231,7 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
     bool unc = false;
     for (int e = lane; e + 1 < send; e += 32) {
         const float fa = __uint_as_float(skey[sord[e]]), fb = __uint_as_float(skey[sord[e + 1]]);
-        unc |= (fb - fa) <= 2.f * eps_of(fb, epsabs * R);
+        unc |= (fb - fa) <= 2.f * eps_of(fb, ea);
     }
     if (__any_sync(0xffffffffu, unc)) {
         const double2 P = B.pos[q];
@@ -240,9 +240,9 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
             bool need = false;
             if (e + 1 < send) {
                 const float fn = __uint_as_float(skey[sord[e + 1]]);
-                need |= (fn - fe) <= 2.f * eps_of(fn, epsabs * R);
+                need |= (fn - fe) <= 2.f * eps_of(fn, ea);
             }
-            if (e > 0) need |= (fe - __uint_as_float(skey[sord[e - 1]])) <= 2.f * eps_of(fe, epsabs * R);
+            if (e > 0) need |= (fe - __uint_as_float(skey[sord[e - 1]])) <= 2.f * eps_of(fe, ea);
             if (need) {
                 const uint32_t code = scode[sord[e]];
                 double ox, oy;
@@ -258,7 +258,7 @@ __device__ int select_write(const KnnArgs &a, const SimDev &S, int64_t q, int m,
                 bool brk = (e + 1 == send);
                 if (!brk) {
                     const float fa = __uint_as_float(skey[sord[e]]), fb = __uint_as_float(skey[sord[e + 1]]);
-                    brk = (fb - fa) > 2.f * eps_of(fb, epsabs * R);
+                    brk = (fb - fa) > 2.f * eps_of(fb, ea);
                 }
                 if (brk) {
                     // insertion sort of the run [rs, e] by (exact d2, id, image)
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256, 4) k_knn(KnnArgs a) {
             }
             __syncwarp();
             float Rn;
-            if (select_write<MODE, NR>(a, S, q, m, R, epsabs, skey, scode, sord, sexact, lane, &Rn, (uint32_t *)rq)) {
+            if (select_write<MODE, NR>(a, S, q, m, R, epsabs * R, skey, scode, sord, sexact, lane, &Rn, (uint32_t *)rq)) {
                 Rlo = R;
                 R = Rn;
                 continue;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, (MODE == MODE_MIXED || NR > 2
         const float pxr = pr.x + pr.z, pyr = pr.y + pr.w;
         // a radius guess well inside one period (no self image can come within R)
         const float Rcap = 0.25f * fminf(sx0, sy0) * (float)G;
-        bool defer_all = __any_sync(FULL, valid && !(R > 0.f && R < Rcap));
+        bool defer_all = __any_sync(FULL, valid && !(R >= kTileMinR && R < Rcap));
         int x0 = INT_MAX, x1 = INT_MIN, y0 = INT_MAX, y1 = INT_MIN;
         if (valid && !defer_all) {
             const float Re = R + tol;

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
         }
         // a radius guess well inside one period (no self image within R)
         const float Rcap = 0.25f * fminf(sx0, sy0) * (float)G;
-        const bool rok = R > 0.f && R < Rcap;
+        const bool rok = R >= kTileMinR && R < Rcap;
         defer_lanes(a, mine && !rok, q, lane);
         bool valid = mine && rok;
         const float pxr = pr.x + pr.z, pyr = pr.y + pr.w;
@@ -455,8 +455,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? (NR <= 2 ? 3 : 1) : (
             const float Re = R + tol, Re2 = Re * Re;
             const int lx0 = x0 >> sh, lx1 = x1 >> sh;
             // the chord's ends need not be exact, only outside: the approximate
-            // root is raised by 2^-19 of itself, and the ends moved out by
-            // 2.4e-7 of the box, more than the products with 1 / Sx round
+            // root is raised by 2^-19 of itself, and the ends moved out by 2.4e-7 of
+            // the box, more than their three FP32 roundings (the end, 1 / Sx, their
+            // product) at |end| <= 1.25 L move them, 2.2e-7; S.tol lies behind that. A
+            // radicand below 2^-126, which the root flushes to 0, is less than Re^2
+            // exceeds R^2 by: R >= kTileMinR, and Re^2 - R^2 > 2 R S.tol > 3.2e-6 R^2 since
+            // R < L / 4
             const float inv_Sx = 1.f / Sx, pad = 2.4e-7f * S.flmax;
             // four rows at a time: their record ranges (start, and end above it in
             // the high half; 0: none), then one loop over all four, so that the

@@ -23,6 +23,10 @@ struct KnnArgs {
 // reference's own rounding of (p + offset) adds ~2^-53 L absolute per axis.
 constexpr float kEpsRel = 9.5367431640625e-7f;  // 2^-20 (about 8x the bound)
 
+// The least search radius the tiles take: below it (boxes under 4e-15 or so) the
+// keys' scale 2^23 / R^2 and unit would leave FP32's normal range.
+constexpr float kTileMinR = 0x1p-52f;
+
 __device__ __forceinline__ float eps_of(float d2, float abs_term) { return kEpsRel * d2 + abs_term; }
 
 // Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their
