@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(256, 4) k_knn(KnnArgs a) {
             }
             __syncwarp();
             float Rn;
-            if (select_write<MODE, NR>(a, S, q, m, R, epsabs * R, skey, scode, sord, sexact, lane, &Rn, (uint32_t *)rq)) {
+            if (select_write<MODE, NR>(a, S, q, m, R, __fmaf_rn(epsabs, R, kEpsSubnormal), skey, scode, sord, sexact, lane, &Rn, (uint32_t *)rq)) {
                 Rlo = R;
                 R = Rn;
                 continue;

@@ -27,6 +27,10 @@ constexpr float kEpsRel = 9.5367431640625e-7f;  // 2^-20 (about 8x the bound)
 // keys' scale 2^23 / R^2 and unit would leave FP32's normal range.
 constexpr float kTileMinR = 0x1p-52f;
 
+// the products' rounding once they leave FP32's normal range (boxes below 1e-17
+// or so): a few units of 2^-149
+constexpr float kEpsSubnormal = 1.2e-44f;
+
 __device__ __forceinline__ float eps_of(float d2, float abs_term) { return kEpsRel * d2 + abs_term; }
 
 // Batcher's odd-even merge sort (K. E. Batcher, "Sorting networks and their

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("k,path", [(32, 8), (21, 8), (45, 4), (90, 2)])
-@pytest.mark.parametrize("box", [2.0**-20, 1e-9, 2.0**-40, 1e-13, 2.0**-46, 2.0**-50, 2.0**-53, 3e-18])
+@pytest.mark.parametrize("box", [2.0**-20, 1e-9, 2.0**-40, 1e-13, 2.0**-46, 2.0**-50, 2.0**-53, 3e-18, 1e-18, 4e-19])
 def test_small_boxes(gpu, oracle, box, k, path):
     n = 3000
     x, y, vx, vy, u = ics.uniform_blast(n, 8)
