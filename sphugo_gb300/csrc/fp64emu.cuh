@@ -386,6 +386,11 @@ __device__ __forceinline__ double emu_div_n(double x, const EmuDivisor &D) {
     return emu_double(((uint64_t)eh << 32) + Q);
 }
 
+// RN(x / 3), 3 a divisor prepared once: 2^115 / (3 2^51) = 2^64 / 3, rounded down
+__device__ __forceinline__ double emu_div3_n(double x) {
+    return emu_div_n(x, EmuDivisor{3ull << 51, 0x5555555555555555ull, 0x40080000u});
+}
+
 // RN(x / y): the unchecked quotient, or the hardware's when an operand lies
 // outside [2^-500, 2^500)
 __device__ __forceinline__ double emu_div(double x, const EmuDivisor &D, double y) {

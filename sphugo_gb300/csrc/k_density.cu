@@ -83,11 +83,11 @@ __device__ __noinline__ PairF pair_slow(double dx, double dy, double h, int kern
 }
 
 // F and dF of the Monahan kernel for q in [1/2, 1): (1 - q)^3 / 3 and
-// -(1 - q)^2, the difference exact; / 3 as a quotient with inv = 2^64 / 3
+// -(1 - q)^2, the difference exact
 __device__ __forceinline__ void monahan_far(double q, PairF &r) {
     const double z = emu_one_minus_n(q);
     const double z2 = emu_mul_n(z, z);
-    r.f = emu_div_n(emu_mul_n(z2, z), EmuDivisor{3ull << 51, 0x5555555555555555ull, 0x40080000u});
+    r.f = emu_div3_n(emu_mul_n(z2, z));
     r.df = emu_neg(z2);
 }
 

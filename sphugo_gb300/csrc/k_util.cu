@@ -385,8 +385,9 @@ __global__ void k_div_selftest(int64_t n, uint64_t seed, unsigned long long *bad
             a = __fma_rn(b, q, __dmul_rn(b, 0x1p-53));
         }
         const double ref = __ddiv_rn(a, b);
-        if (div_rn_recip(a, b, __drcp_rn(b)) != ref) nb++;
-        if (div3_rn(a) != __ddiv_rn(a, 3.0)) nb++;
+        if (emu_div_n(a, emu_divisor(b)) != ref) nb++;
+        const double third = __ddiv_rn(a, 3.0);
+        if (div3_rn(a) != third || emu_div3_n(a) != third) nb++;
     }
     if (nb) atomicAdd(bad, nb);
 }
@@ -485,6 +486,23 @@ __global__ void k_emu_selftest(int64_t n, uint64_t seed, unsigned long long *bad
         if (!emu_same(emu_one_minus(xh), __dsub_rn(1.0, xh))) nb++;
         if (!emu_same(emu_one_minus(x), __dsub_rn(1.0, x))) nb++;
         if (!emu_same(emu_one_minus(1.0), __dsub_rn(1.0, 1.0))) nb++;
+        // the unchecked forms, over the ranges that the kernels' range tests admit
+        // (products up to 2^+-1000, quotients of numerators up to 2^+-800, roots of
+        // every normal number, 1 - x for x in [1/2, 1), thirds of (1 - q)^3), and squares
+        const double ua = emu_operand(r1, cls, 523u + (uint32_t)(r3 % 1001u)), ub = emu_operand(r2, cls, 523u + (uint32_t)((r3 >> 10) % 1001u));
+        if (cls != 0) {
+            if (!emu_same(emu_mul_n(ua, ub), __dmul_rn(ua, ub))) nb++;
+            const double un = emu_operand(r1, cls, 223u + (uint32_t)((r3 >> 20) % 1601u)), ud = emu_operand(r2, cls, 823u + (uint32_t)((r3 >> 31) % 401u));
+            if (!emu_same(emu_div_n(un, emu_divisor(ud)), __ddiv_rn(un, ud))) nb++;
+            const double us = emu_double(((uint64_t)(1u + (uint32_t)((r3 >> 42) % 2046u)) << 52) | (emu_bits(ua) & kEmuFrac));
+            if (!emu_same(emu_sqrt_n(us), __dsqrt_rn(us))) nb++;
+            const double ut = emu_double(((uint64_t)(1022u - (uint32_t)((r3 >> 53) % 162u)) << 52) | (emu_bits(ua) & kEmuFrac));
+            if (!emu_same(emu_div3_n(ut), __ddiv_rn(ut, 3.0))) nb++;
+        }
+        if (!emu_same(emu_one_minus_n(xh), __dsub_rn(1.0, xh))) nb++;
+        if (!emu_same(emu_sq(x), __dmul_rn(x, x))) nb++;
+        // x as a float
+        if (__float_as_uint(emu_d2f(x)) != __float_as_uint(__double2float_rn(x)) && x == x) nb++;
         // float pairs of the operands and of the products
         float h1, l1;
         emu_split_df(x, h1, l1);

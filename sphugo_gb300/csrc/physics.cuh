@@ -25,19 +25,6 @@ __device__ __forceinline__ double div3_rn(double a) {
     return __fma_rn(r, y, q0);
 }
 
-// RN(a/b) given y = RN(1/b) (shared by many quotients with the same b):
-// q1 below is faithful (within one ulp of a/b), the residual a - b q1 is exact
-// in the FMA, and Markstein's theorem (y within half an ulp of 1/b, q1
-// faithful) makes RN(q1 + r1 y) the correctly rounded quotient. No
-// overflow/underflow for the operands used here (distances and their ratios).
-__device__ __forceinline__ double div_rn_recip(double a, double b, double y) {
-    const double q0 = emu_mul(a, y);
-    const double r0 = __fma_rn(-b, q0, a);
-    const double q1 = __fma_rn(r0, y, q0);
-    const double r1 = __fma_rn(-b, q1, a);
-    return __fma_rn(r1, y, q1);
-}
-
 // sim/sph.go:258-276 Monahan2D and :284-304 Wendtland2D, reference rounding.
 __device__ __forceinline__ double kf_exact(int kernel, double q) {
     if (kernel == SPH_KERNEL_WENDLAND) {
