@@ -587,10 +587,9 @@ __global__ void __launch_bounds__(256, 4) k_knn(KnnArgs a) {
 //   3. each lane scans the whole tile for its own query (broadcast reads) and
 //      keeps every record within R as a 32-bit key: the squared distance in
 //      units of R^2 / 2^23 (23 bits) above the tile slot (9 bits);
-//   4. each lane keeps its k+1 smallest keys in ascending order (a
-//      branch-free insertion chain in registers; an insertion sort in its
-//      shared-memory column for k > 80) and accepts the first k when the FP32
-//      values decide them:
+//   4. each lane sorts its keys (a network in registers; an insertion sort in
+//      its shared-memory column for k > 80) and accepts the first k when the
+//      FP32 values decide them:
 //      the k-th lies 3 eps inside R (the tile held every candidate), the
 //      (k+1)-th lies more than 2 eps beyond it (the set), and in the FP64
 //      forms every neighbour is more than 2 eps from the next (the order;
@@ -620,8 +619,6 @@ struct TileSmem {
     // (264, 610 or 2112 min/max for LCAP = 24, 40, 96); longer lists take a
     // shared-memory insertion sort
     static constexpr bool REG = NR <= 4;
-    static constexpr bool NET = NR <= 4;
-    static constexpr int A = NET ? LCAP : 81;
     float2 rec[kTileCap];             // candidate positions relative to the group origin
     uint32_t code[kTileCap];          // (slot << kCodeShift) | image
     int4 rect[32];                    // per query: cell rectangle at the tile level
@@ -888,29 +885,13 @@ __global__ void __launch_bounds__(kTileWarps * 32, (MODE == MODE_MIXED || NR > 2
         const float Dy = fmaxf(fabsf((float)(BY0 << sh) * sy0 - oy), fabsf((float)((BY1 + 1) << sh) * sy0 - oy));
         // (the last term also covers the float-pair residues of the records, 2^-48 |p - origin|)
         const float ea = kEpsRel * (R2 + 2.f * R * (Dx + Dy)) + 2.3e-13f * fmaxf(S.flmax, S.fmag) * R;
-        if (TS::REG) {
-            // the A smallest keys, ascending, by a branch-free insertion chain
-            // per list entry (registers only: no divergence, no smem latency chain)
-            constexpr int A = TS::A;
+        if constexpr (TS::REG) {
+            constexpr int A = LCAP;
             uint32_t arr[A];
             const int m = ok ? cnt : 0;
-            if constexpr (TS::NET) {
 #pragma unroll
-                for (int i = 0; i < A; i++) arr[i] = i < m ? sm.list[i][lane] : 0xffffffffu;
-                if (ok) OddEvenSort<A>{arr}.run();
-            } else {
-#pragma unroll
-                for (int i = 0; i < A; i++) arr[i] = 0xffffffffu;
-                for (int e = 0; e < m; e++) {
-                    uint32_t v = sm.list[e][lane];
-#pragma unroll
-                    for (int i = 0; i < A; i++) {
-                        const uint32_t lo = min(arr[i], v);
-                        v = max(arr[i], v);
-                        arr[i] = lo;
-                    }
-                }
-            }
+            for (int i = 0; i < A; i++) arr[i] = i < m ? sm.list[i][lane] : 0xffffffffu;
+            if (ok) OddEvenSort<A>{arr}.run();
             // arr is ascending: the k-th key is the largest of the first k, the
             // (k+1)-th the smallest of the rest (reductions rather than
             // selects at i == k - 1, which the compiler turns into an indexed
