@@ -7,6 +7,7 @@ import pytest
 from sphugo_gb300 import _lib as L
 from sphugo_gb300 import ics
 from sphugo_gb300 import sim as S
+import test_gpu_parity as parity
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +68,45 @@ def test_default_goes_on_after_a_checkpoint(gpu, tmp_path, path):
     sa, sb = a.state(), b.state()
     for key in sa:
         assert np.array_equal(sa[key], sb[key]), key
+
+
+def scene(name, seed=9):
+    """Small states whose default search is the per-query one, and whether tiles settle most of their queries."""
+    if name == "walls":  # open axes, gravity, reflections
+        n = 2000
+        x, y, vx, vy, u = ics.uniform_blast(n, seed)
+        conf = S.SphConfig(DeltaTHalf=5e-4, Gamma=5 / 3, ParticleMass=1.0 / n, Acceleration=S.Vec2(0.0, 0.5), Kernel="Wendtland",
+                           Reflections=S.Reflections(L=0.31, R=S.DBL_MAX, U=-S.DBL_MAX, D=0.69), ViscosityAlpha=1.0,
+                           ViscosityBeta=2.0)
+        return conf, (0.3 + 0.4 * x, 0.2 + 0.5 * y, vx, vy, u), 10, True
+    if name == "box":  # neither unit nor square
+        n = 1500
+        x, y, vx, vy, u = ics.uniform_blast(n, seed)
+        conf = S.SphConfig(DeltaTHalf=1e-4, Gamma=5 / 3, ParticleMass=1.0 / n, HorPeriodicity=(0.2, 0.8),
+                           VertPeriodicity=(-1.0, 1.0), ViscosityAlpha=1.0, ViscosityBeta=2.0)
+        return conf, (0.2 + 0.6 * x, -1.0 + 2.0 * y, vx, vy, u), 6, True
+    if name == "far":  # far from the origin
+        n = 2000
+        x, y, vx, vy, u = ics.uniform_blast(n, seed)
+        conf = S.SphConfig(DeltaTHalf=1e-4, Gamma=5 / 3, ParticleMass=1.0 / n, HorPeriodicity=(1000.0, 1001.0),
+                           VertPeriodicity=(-3000.0, -2998.0), ViscosityAlpha=1.0, ViscosityBeta=2.0)
+        return conf, (1000.0 + x, -3000.0 + 2.0 * y, vx, vy, u), 6, True
+    n, k = {"images": (64, 32), "few": (40, 16), "long": (200, 64), "blast": (10_000, 32), "k45": (3000, 45)}[name]
+    return ics.periodic_config(n, k, 1e-4), ics.uniform_blast(n, n), 3, n > 1000
+
+
+@pytest.mark.parametrize("path", [1, 2, 4, 8])
+@pytest.mark.parametrize("name", ["walls", "box", "far", "images", "few", "long", "blast", "k45"])
+def test_tiles_of_small_states(gpu, oracle, name, path):
+    conf, arrs, steps, most = scene(name)
+    k = conf.NeighbourCount
+    if path in (4, 8) and k > (37 if path == 8 else 80):
+        pytest.skip("no block tiles of that many warps for this k")
+    g, o = parity.pair(oracle, conf, arrs)
+    g.SetSearch(path)
+    g.Step(steps)
+    o.step(steps)
+    parity.assert_bitwise(g, o)
+    if most:
+        assert g.search_stats()[1] < len(arrs[0])
+    g.close()
