@@ -98,7 +98,7 @@ FP64_NOTE = ("the density and the force compute their multiplications, square ro
              "instructions beside the FP64 unit (bit-identical to the hardware instructions; "
              "sph_selftest_fp64emu), so frac can exceed 1 against the FP64 unit's issue ceiling; ncu on the "
              "clustered workload at N = 1,048,576: force FP64 pipe 73 %, ALU pipe 57 %, issue slots 67 % busy; "
-             "density 68 %, 67 %, 70 %")
+             "density 67 %, 67 %, 70 %")
 
 
 def algorithmic(k, div, sqrt, lo_frac, visc_frac):

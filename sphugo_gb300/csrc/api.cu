@@ -57,8 +57,11 @@ int default_block_warps(int k) {
 // Whether the default search is the per-query one. With few particles the
 // block tiles are few (40 of 256 queries at N = 10,000, on 152 SMs), and a
 // tile's chain of steps is longer than a warp per query, of which all are
-// resident at once. FP64 forms, kNN stage: N = 1000 26 us with tiles, 12
-// without, 3000 33 and 14, 10,000 34 and 23, 30,000 38 and 45. The mixed form
+// resident at once. FP64 forms, kNN stage at k = 32: N = 1000 26 us with tiles, 12
+// without, 3000 33 and 14, 10,000 34 and 23, 30,000 38 and 45. At k = 16 to 64 it
+// took 0.34 to 0.93 of the tiles' time, above k = 80 0.07 to 0.91 (uniform and
+// clustered states, N = 400 to 16,384, ensembles of 4 x 4000 to 200 x 80), but 1.06
+// at uniform N = 16,384, k = 48, and 1.4 on a perfect lattice of 16,384. The mixed form
 // keeps the tiles at every size: its sums follow the order of the lists they
 // leave, and a changed default would move its results in the last bits.
 constexpr int64_t kPerQueryMaxN = 16384;

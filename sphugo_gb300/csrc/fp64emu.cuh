@@ -4,14 +4,16 @@
 // integer instructions (and FP32 seeds and conversions).
 //
 // GB300 issues two FP64 lanes per SM per clock: one warp-wide FP64
-// instruction holds a sub-partition's FP64 unit for about 64 cycles, while
+// instruction holds a sub-partition's FP64 unit for 75 cycles (measured), while
 // the same sub-partition can issue one instruction of another kind every
-// cycle. The FP64-bound kernels leave about 90 % of the issue slots idle, so
-// some of their operations are computed here, on the integer and FP32
-// pipes, in parallel with the hardware FP64 instructions. Every result is
-// the hardware instruction's, bit for bit (sph_selftest_fp64emu checks each
-// against __dmul_rn, __dadd_rn, __dsub_rn, __ddiv_rn, __dsqrt_rn and the
-// double -> float conversion).
+// cycle. So the FP64 kernels compute products, quotients and roots here, on
+// the integer and FP32 pipes, beside the hardware's additions (their FP64 unit,
+// ALU and issue slots are then each about two thirds busy). Every result is the
+// hardware instruction's, bit for bit (sph_selftest_fp64emu checks each, and the
+// unchecked forms over the ranges that the kernels' tests admit, against
+// __dmul_rn, __dadd_rn, __dsub_rn, __ddiv_rn, __dsqrt_rn and the double -> float
+// conversion). The checked sum, difference and 1 - x are called by these checks
+// alone at present.
 //
 // Method for products and sums (the textbook guard digits and sticky bit,
 // e.g. D. Goldberg, "What every computer scientist should know about

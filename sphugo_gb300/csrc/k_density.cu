@@ -10,9 +10,9 @@
 // sums run in hardware (four per pair, three more where q < 1/2) and the
 // products, quotients and roots on the integer pipes (fp64emu.cuh), unchecked
 // behind one range test per pair; pair_slow computes a pair that fails it with
-// the hardware alone. ncu, uniform blast N = 1,048,576, k = 32: FP64 pipe 62 %,
-// ALU 61 %, issue 64 % busy, none of them alone the bound; the next round's
-// loads issued early changed nothing (542 us both).
+// the hardware alone. ncu, clustered N = 1,048,576, k = 32: FP64 pipe 67 %, ALU
+// 67 %, issue 70 % busy, none of them alone the bound; the next round's loads
+// issued early changed nothing.
 //
 // Measured against one thread per particle with three passes over its list
 // (density stage, us): N = 1000 49 -> 12, 10,000 61 -> 21, 100,000 107 -> 70,

@@ -20,7 +20,10 @@ constexpr int kMixedBlocks = 20;  // resident blocks (warps) per SM (8 KB each)
 // at 32 particles, 20 warps resident per SM, and with 72 and seven, 25 resident.
 // The second hides more latency, but each of its warps takes longer: it runs
 // beyond one pass of its own (121,600 particles), except where the first takes
-// just two (97,280 each; from one and a half of the second's on, up to 204,288).
+// just two (97,280 each; from one and a half of the second's on, up to 204,288):
+// there the first took 0.95 to 1.00 of the second's time at k = 16, 32 and 45,
+// 0.98 to 1.02 at 21, 0.98 to 1.04 at 64 (N = 183,000 to 204,000, uniform and
+// clustered).
 // Force stage, us, first and second: N = 50,000 81 and 86, 100,000 133 and 140,
 // 110,000 137 and 157; 130,000 173 and 167, 140,000 185 and 171, 170,000 212
 // and 205; 200,000 237 and 243; 250,000 303 and 290, 300,000 338 and 330,
@@ -324,14 +327,14 @@ __device__ __forceinline__ void pair_geom(const SimDev &S, const PArrays &B, uin
 // lost in the other component's, and is marked, and the marked components' terms
 // are set to 0 before phase C. Force stage, us, k = 28, with the hardware's
 // arithmetic for all of them and so: perfect lattice at rest, N = 250,000, 765 and
-// 273 (a jittered moving one 262 both ways), N = 1,048,576 2604 and 739 (949 and
+// 276 (a jittered moving one 262 both ways), N = 1,048,576 2604 and 749 (949 and
 // 953), cold gas moving 2957 and 1048, at rest 3135 and 667, alpha = 0 1602 and
 // 1009, viscosity off 1964 and 914. Zero components out of line too: 424 for the
 // first; in a form of phase B of its own, for chunks that have them: 0.5 to 2 % more
 // for every other state.
 //
-// Bound (ncu, uniform blast N = 1,048,576, k = 32): FP64 pipe 72 %, ALU 57 %,
-// issue 67 % busy; moving work either way between the two pipes (the sums
+// Bound (ncu, clustered N = 1,048,576, k = 32): FP64 pipe 73 %, ALU 57 %, issue
+// 67 % busy; moving work either way between the two pipes (the sums
 // cA + cB, hA + hB, rhoA + rhoB on the integer pipe, the dot product or r^2 on
 // the FP64 unit) changed nothing or cost up to 5 %. The loads are issued a
 // round early: 1335 -> 1231 us; one loop for both kinds of pairs instead of
